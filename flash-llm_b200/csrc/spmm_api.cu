@@ -11,6 +11,7 @@
 #include <new>
 
 #include "../../include/SpMM_API.cuh"
+#include "launch.h"
 #include "spmm_kernel_direct_sm100.cuh"
 #include "spmm_kernel_sm100.cuh"
 #include "tiled_csl_host.h"
@@ -349,34 +350,20 @@ template<int N_TILE>
 static cudaError_t launch_spmm(cudaStream_t stream, const CUtensorMap& tmap, const SpmmParams& params, int tile_rows,
                                int n_tiles)
 {
-    const SpmmPlan&     pl = params.plan;
-    cudaLaunchConfig_t  cfg{};
-    cudaLaunchAttribute attr[2];
-    cfg.gridDim          = dim3(pl.cluster_k, tile_rows, n_tiles * pl.workspace_k);
-    cfg.blockDim         = dim3((pl.path == kPathDirect ? 1 + kDirectIssuers + pl.scatter_warps * pl.producers
-                                                        : pl.producers + 2 + pl.scatter_warps) * 32, 1, 1);
-    cfg.dynamicSmemBytes = pl.smem_bytes;
-    cfg.stream           = stream;
-    attr[0].id               = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = pl.cluster_k;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs                = attr;
-    cfg.numAttrs             = 1;
-    if (g_launch_overlap.load(std::memory_order_relaxed)) {
-        attr[1].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.numAttrs                                       = 2;
-    }
-    count_launch();
+    const SpmmPlan& pl = params.plan;
+    const dim3      grid(pl.cluster_k, tile_rows, n_tiles * pl.workspace_k);
+    auto            launch = [&](auto kernel, int warps) {
+        return launch_in_stream_order(kernel, grid, dim3(warps * 32), pl.smem_bytes, stream, pl.cluster_k, tmap, params);
+    };
     if (pl.path == kPathDirect) {
+        const int warps = 1 + kDirectIssuers + pl.scatter_warps * pl.producers;
         if (pl.scatter_warps == 8)
-            return cudaLaunchKernelEx(&cfg, spmm_tcgen05_direct_kernel<N_TILE, kDirectCapWide, 8, 1>, tmap, params);
+            return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapWide, 8, 1>, warps);
         if (pl.producers == 2)
-            return cudaLaunchKernelEx(&cfg, spmm_tcgen05_direct_kernel<N_TILE, kDirectCapPair, 4, 2, 2>, tmap, params);
-        return cudaLaunchKernelEx(&cfg, spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks>, tmap, params);
+            return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapPair, 4, 2, 2>, warps);
+        return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks>, warps);
     }
-    return cudaLaunchKernelEx(&cfg, spmm_tcgen05_kernel<N_TILE>, tmap, params);
+    return launch(spmm_tcgen05_kernel<N_TILE>, pl.producers + 2 + pl.scatter_warps);
 }
 
 static cudaError_t reduce_partials(cudaStream_t stream, half* C, const float* ws, long long count, int parts,
@@ -385,19 +372,8 @@ static cudaError_t reduce_partials(cudaStream_t stream, half* C, const float* ws
     const int       threads = 256;
     const long long groups  = (count + 3) / 4;
     const unsigned  blocks  = static_cast<unsigned>((groups + threads - 1) / threads);
-    count_launch();
-    cudaLaunchConfig_t  cfg{};
-    cudaLaunchAttribute attr[1];
-    cfg.gridDim  = dim3(blocks, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.stream   = stream;
-    if (g_launch_overlap.load(std::memory_order_relaxed)) {
-        attr[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs                                          = attr;
-        cfg.numAttrs                                       = 1;
-    }
-    return cudaLaunchKernelEx(&cfg, splitk_reduce_f32_kernel, C, ws, count, parts, bias, M, activation, residual);
+    return launch_in_stream_order(splitk_reduce_f32_kernel, dim3(blocks), dim3(threads), 0, stream, 1, C, ws, count, parts, bias, M,
+                                  activation, residual);
 }
 
 static cudaError_t reduce_workspace(cudaStream_t stream, half* C, const half* ws, long long count, int parts)
@@ -405,9 +381,7 @@ static cudaError_t reduce_workspace(cudaStream_t stream, half* C, const half* ws
     const int       threads = 256;
     const long long groups  = (count + 7) / 8;
     const unsigned  blocks  = static_cast<unsigned>((groups + threads - 1) / threads);
-    count_launch();
-    splitk_reduce_kernel<<<blocks, threads, 0, stream>>>(C, ws, count, parts);
-    return cudaGetLastError();
+    return launch_in_stream_order(splitk_reduce_kernel, dim3(blocks), dim3(threads), 0, stream, 1, C, ws, count, parts);
 }
 
 static bool n_supported(int N)
@@ -516,6 +490,7 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
     params.status       = st->status;
     params.bias         = bias;
     params.activation   = activation;
+    params.early_weights = g_launch_overlap.load(std::memory_order_relaxed);
     params.residual     = residual;
     params.M            = M_Global;
     params.N            = N_Global;

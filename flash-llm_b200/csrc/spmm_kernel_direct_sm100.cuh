@@ -221,10 +221,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     int          n_in = 0;                  // vectors of the whole tile whose share is in nxt
     const uint4* src  = p.compressed;
     bool         bad  = false;
-    if (warp >= first_sw) {
-#pragma unroll
-        for (int q = 0; q < CAP; ++q)
-            nxt[q] = make_uint4(0u, 0u, 0u, 0u);
+    auto fetch_first_tile = [&]() {
         if (st < L) {
             const int vb = offs_global[st], ve = offs_global[st + 1];
             bad          = (ve < vb) || (ve - vb > kMaxTileVectors) || (vb < 0);
@@ -232,6 +229,13 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
             src          = p.compressed + (bad ? 0 : vb);
             load_batch<WPT, CAP>(nxt, src + first_vec, n_in, n_in - first_vec);
         }
+    };
+    if (warp >= first_sw) {
+#pragma unroll
+        for (int q = 0; q < CAP; ++q)
+            nxt[q] = make_uint4(0u, 0u, 0u, 0u);
+        if (p.early_weights)
+            fetch_first_tile();
     }
 
     // ---- set-up
@@ -253,6 +257,11 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     if (warp == mma_warp) {
         ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
         ptx::tmem_relinquish();
+    }
+    if (!p.early_weights) {
+        ptx::grid_dependency_wait();
+        if (warp >= first_sw)
+            fetch_first_tile();
     }
     if (staged) {
         // This CTA's slice of TileOffsets is read once, together, instead of one dependent load per tile.

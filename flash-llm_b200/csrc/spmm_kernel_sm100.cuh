@@ -39,6 +39,7 @@ struct SpmmParams {
     float*        partial;       // workspace_k fp32 partial matrices [N][M] (used when workspace_k > 1)
     unsigned int* status;        // per-device status word
     const half*   bias;          // [M] added to every output row before the activation, or nullptr
+    int           early_weights;  // weights may be read before the kernels enqueued earlier have completed (launch overlap)
     int           activation;    // kActNone or kActRelu, applied to the fp32 sum before the one fp16 rounding
     const half*   residual;      // [N][M] like C, added after the activation and before the rounding, or nullptr
     int           M, N, K;
@@ -260,8 +261,8 @@ __device__ __forceinline__ bool offsets_slice_is_bad(const int* offs_global, int
 
 // The B loader thread: `batches` 3-D TMA boxes of KB K tiles of [N_TILE x 64] each into a ring of b_stages buffers.
 // B (and, through the MMAs that consume it, every store of the kernel) must come after the kernels before this one in
-// the stream; the compressed weights and their offsets are streamed without waiting, which is what the caller promises
-// to be safe when it enables launch overlap.
+// the stream.  The compressed weights and their offsets are streamed without waiting only where the caller promises that
+// to be safe by enabling launch overlap; otherwise every thread has waited before it read them.
 __device__ __forceinline__ void load_b_batches(const CUtensorMap* tmap, int batches, int KB, int b_stages, uint32_t slab_bytes,
                                                uint32_t b_base, uint32_t b_full, uint32_t b_empty, int n_coord, int k_begin,
                                                volatile uint32_t* abort_flag, unsigned int* status)
@@ -669,6 +670,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
         ptx::tmem_relinquish();
     }
+    if (!p.early_weights)
+        ptx::grid_dependency_wait();
     if (staged) {
         // This CTA's slice of TileOffsets is read once, together, instead of one dependent load per tile.
         for (int i = threadIdx.x; i <= L; i += blockDim.x)
@@ -1040,6 +1043,8 @@ __global__ void splitk_reduce_f32_kernel(half* __restrict__ C, const float* __re
 // C[i] = fp16(sum_s float(ws[s*count + i])) over fp16 partial matrices; eight outputs per thread, 16-byte accesses.
 __global__ void splitk_reduce_kernel(half* __restrict__ C, const half* __restrict__ ws, long long count, int parts)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     const long long i8 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
     if (i8 >= count)
         return;

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/SpMM_API.cuh"
+#include "launch.h"
 #include "tiled_csl_device.cuh"
 #include "tiled_csl_host.h"
 #include "tiling.h"
@@ -74,12 +75,11 @@ int FlashLLM_EncodeOnDevice_TileOffsets(void* stream, const void* A_d, int M, in
         return rc;
     const int    k_tiles = K / kTileK, tiles = (M / kTileM) * k_tiles;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    count_launch();
-    csl_count_kernel<<<(tiles + kEncodeWarps - 1) / kEncodeWarps, kEncodeWarps * 32, 0, s>>>(
-        static_cast<const uint16_t*>(A_d), K, tiles, k_tiles, TileOffsets_d);
-    count_launch();
-    csl_scan_kernel<<<1, 1024, 0, s>>>(TileOffsets_d, tiles, status);
-    return static_cast<int>(cudaGetLastError());
+    cudaError_t  e = launch_in_stream_order(csl_count_kernel, dim3((tiles + kEncodeWarps - 1) / kEncodeWarps), dim3(kEncodeWarps * 32),
+                                           0, s, 1, static_cast<const uint16_t*>(A_d), K, tiles, k_tiles, TileOffsets_d);
+    if (e == cudaSuccess)
+        e = launch_in_stream_order(csl_scan_kernel, dim3(1), dim3(1024), 0, s, 1, TileOffsets_d, tiles, status);
+    return static_cast<int>(e);
 }
 
 int FlashLLM_EncodeOnDevice_Pack(void* stream, const void* A_d, int M, int K, const int* TileOffsets_d,
@@ -94,14 +94,9 @@ int FlashLLM_EncodeOnDevice_Pack(void* stream, const void* A_d, int M, int K, co
     const int    k_tiles = K / kTileK, tiles = (M / kTileM) * k_tiles;
     const int    blocks  = (tiles + kEncodeWarps - 1) / kEncodeWarps;
     cudaStream_t s       = static_cast<cudaStream_t>(stream);
-    count_launch();
-    if (reorder)
-        csl_pack_reorder_kernel<<<blocks, kEncodeWarps * 32, 0, s>>>(static_cast<const uint16_t*>(A_d), K, tiles, k_tiles,
-                                                                      TileOffsets_d, Compressed_A_d, status);
-    else
-        csl_pack_scan_kernel<<<blocks, kEncodeWarps * 32, 0, s>>>(static_cast<const uint16_t*>(A_d), K, tiles, k_tiles,
-                                                                   TileOffsets_d, Compressed_A_d, status);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_in_stream_order(reorder ? csl_pack_reorder_kernel : csl_pack_scan_kernel, dim3(blocks),
+                                                   dim3(kEncodeWarps * 32), 0, s, 1, static_cast<const uint16_t*>(A_d), K, tiles,
+                                                   k_tiles, TileOffsets_d, Compressed_A_d, status));
 }
 
 void FlashLLM_Free(void* p)

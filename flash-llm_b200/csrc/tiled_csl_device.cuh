@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx_sm100.cuh"
 #include "tiling.h"
 
 namespace flashllm {
@@ -53,6 +54,8 @@ __device__ __forceinline__ int slot_of_pick(int q, int vectors)
 __global__ void __launch_bounds__(kEncodeWarps * 32)
     csl_count_kernel(const uint16_t* __restrict__ A, int K, int tiles, int k_tiles, int* __restrict__ offs)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     const int t    = blockIdx.x * kEncodeWarps + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (t >= tiles)
@@ -72,6 +75,8 @@ __global__ void __launch_bounds__(kEncodeWarps * 32)
 // Step 1b: in-place inclusive scan of offs[1..tiles], offs[0] = 0, offs[tiles + 1] = offs[tiles].  One CTA.
 __global__ void __launch_bounds__(1024) csl_scan_kernel(int* __restrict__ offs, int tiles, unsigned int* status)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     __shared__ long long part[1024];
     const int            tid   = threadIdx.x;
     const int            chunk = (tiles + 1023) / 1024;
@@ -112,6 +117,8 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_reorder_kernel(con
                                                                              uint32_t* __restrict__ out,
                                                                              unsigned int* status)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     __shared__ uint32_t s_mask[kEncodeWarps][kHeightEntries];   // buckets at least this high
     __shared__ uint16_t s_above[kEncodeWarps][kHeightEntries];  // words lying above this height (< 8192 + 3)
     const int w    = threadIdx.x >> 5;
@@ -201,6 +208,8 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_scan_kernel(const 
                                                                           uint32_t* __restrict__ out,
                                                                           unsigned int* status)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31;
     const int t    = blockIdx.x * kEncodeWarps + (threadIdx.x >> 5);
     if (t >= tiles)

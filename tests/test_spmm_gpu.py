@@ -225,3 +225,37 @@ def test_launch_overlap_keeps_stream_order(lib, oracle):
     assert lib.consume_status() == 0
     for i, out in enumerate(outs):
         assert_close(out.cpu().numpy(), want[i % 4], f"chained call {i}")
+
+
+@pytest.mark.parametrize("split_k", [1, 8])
+@pytest.mark.parametrize("N", [16, 128])
+def test_weights_written_earlier_in_the_stream_are_seen(lib, oracle, N, split_k):
+    """Without launch overlap a call may follow, on its stream, the work that produces its weights and offsets: kernels are
+    launched before their predecessor has drained, so they must not read either early.  The copies sit behind a long
+    kernel, and the buffers hold another matrix until they run."""
+    M, K = 1024, 2048
+    dev = torch.device("cuda:0")
+    B = lib.synthetic.dense_uniform_matrix(N, K, 5).numpy()
+    problems = []
+    for seed, sparsity in ((81, 0.8), (82, 0.9)):
+        A = lib.synthetic.sparse_uniform_matrix(M, K, sparsity, seed).numpy()
+        comp, offs, _ = lib.InitSparseMatrixA_API(A)
+        problems.append((torch.from_numpy(comp.view(np.int32)).to(dev), torch.from_numpy(offs).to(dev), oracle.gemm_f32(A, B)))
+    words = torch.zeros(max(c.numel() for c, _, _ in problems), dtype=torch.int32, device=dev)
+    offsets = torch.zeros_like(problems[0][1])
+    B_d = torch.from_numpy(B).to(dev)
+    ws = torch.empty((split_k, N, M), dtype=torch.float16, device=dev)
+    outs = [torch.empty((N, M), dtype=torch.float16, device=dev) for _ in range(6)]
+    slow = torch.zeros((1 << 26,), dtype=torch.float32, device=dev)
+    stream = torch.cuda.current_stream().cuda_stream
+    for i, out in enumerate(outs):
+        comp_d, offs_d, _ = problems[i % 2]
+        slow.add_(1.0)
+        words[:comp_d.numel()].copy_(comp_d)
+        offsets.copy_(offs_d)
+        lib.SpMM_SplitK_API(stream, None, words.data_ptr(), offsets.data_ptr(), B_d.data_ptr(), out.data_ptr(), M, N, K,
+                            ws.data_ptr(), split_k)
+    torch.cuda.synchronize()
+    assert lib.consume_status() == 0
+    for i, out in enumerate(outs):
+        assert_close(out.cpu().numpy(), problems[i % 2][2], f"call {i}")
