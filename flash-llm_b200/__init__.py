@@ -31,6 +31,7 @@ from .api import (  # noqa: F401
     read_output_sizes,
     read_rank_lists,
     read_sparse_matrix_bin_files,
+    release_scratch,
     set_launch_overlap,
     set_plan,
     splitk_reduction,

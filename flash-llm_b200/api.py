@@ -95,6 +95,8 @@ def library() -> C.CDLL:
     L.FlashLLM_SpMM_SplitK_AllReduce.argtypes = [C.c_void_p] * 6 + [C.c_int] * 3 + [C.c_void_p, C.c_int, C.c_void_p, C.c_int]
     L.FlashLLM_SplitK_Reduction.restype = C.c_int
     L.FlashLLM_SplitK_Reduction.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int]
+    L.FlashLLM_ReleaseScratch.restype = C.c_int
+    L.FlashLLM_ReleaseScratch.argtypes = []
     L.FlashLLM_SetLaunchOverlap.argtypes = [C.c_int]
     L.FlashLLM_SetPlan.argtypes = [_i32p, C.c_int]
     L.FlashLLM_GetPlan.restype = C.c_int
@@ -352,9 +354,14 @@ def set_launch_overlap(enable: bool) -> None:
     library().FlashLLM_SetLaunchOverlap(1 if enable else 0)
 
 
+def release_scratch() -> None:
+    """Free the current device's scratch of the streaming kernel (allocated per stream on first use); synchronises."""
+    _check(library().FlashLLM_ReleaseScratch(), "ReleaseScratch")
+
+
 PLAN_FIELDS = ("cluster_k", "workspace_k", "a_stages", "b_stages", "b_batch", "ring_slots", "chunk_vectors",
                "scatter_warps", "producers", "path", "reduce")
-PATH_RING, PATH_DIRECT = 1, 2
+PATH_RING, PATH_DIRECT, PATH_STREAM = 1, 2, 3
 REDUCE_SECOND_KERNEL, REDUCE_LAST_CTA = 1, 2
 
 

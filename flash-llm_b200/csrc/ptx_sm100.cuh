@@ -31,6 +31,15 @@ __device__ __forceinline__ uint32_t ld_relaxed_sys_u32(const unsigned int* ptr)
     return v;
 }
 
+// Counts in on a counter in global memory; what this thread, and the threads it has synchronised with, stored before is
+// visible to whoever observes the new count, and what the others stored before theirs is visible afterwards.
+__device__ __forceinline__ uint32_t atom_add_acq_rel_gpu(unsigned int* ptr, uint32_t v)
+{
+    uint32_t before;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(before) : "l"(ptr), "r"(v) : "memory");
+    return before;
+}
+
 __device__ __forceinline__ uint64_t globaltimer_ns()
 {
     uint64_t t;
@@ -234,6 +243,49 @@ __device__ __forceinline__ bool umma_tile_commit_probe(uint32_t d_tmem, uint64_t
           "r"(probe_b)
         : "memory");
     return ready != 0;
+}
+
+// One 128x64 tile of A times one [N x 64] slab of B, executed by a CONVERGED warp: the four K=16 MMAs, the commit that
+// hands the A stage back, and (do_commit_b != 0) the commit that hands the B batch back, all by one elected lane.
+__device__ __forceinline__ void umma_tile_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                uint32_t accumulate_first, uint32_t commit_a_bar, uint32_t commit_b_bar,
+                                                uint32_t do_commit_b)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred pacc, ptrue, pe, pcb;\n"
+        ".reg .b64 da, db;\n"
+        "setp.ne.b32 pacc, %4, 0;\n"
+        "setp.eq.b32 ptrue, 0, 0;\n"
+        "elect.sync _|pe, 0xffffffff;\n"
+        "setp.ne.and.b32 pcb, %7, 0, pe;\n"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pacc;\n"
+        "add.s64 da, %1, 2;\n"
+        "add.s64 db, %2, 2;\n"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, ptrue;\n"
+        "add.s64 da, %1, 4;\n"
+        "add.s64 db, %2, 4;\n"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, ptrue;\n"
+        "add.s64 da, %1, 6;\n"
+        "add.s64 db, %2, 6;\n"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, ptrue;\n"
+        "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n"
+        "@pcb tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n"
+        "}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(commit_a_bar), "r"(commit_b_bar), "r"(do_commit_b)
+        : "memory");
+}
+
+// umma_commit by one elected lane of a converged warp (the lane umma_tile_elect elects).
+__device__ __forceinline__ void umma_commit_elect(uint32_t bar)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred pe;\n"
+        "elect.sync _|pe, 0xffffffff;\n"
+        "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+        "}\n" ::"r"(bar)
+        : "memory");
 }
 
 // Arrives once on the mbarrier when every tcgen05 operation issued so far by this thread has completed.

@@ -14,6 +14,7 @@
 #include "launch.h"
 #include "spmm_kernel_direct_sm100.cuh"
 #include "spmm_kernel_sm100.cuh"
+#include "spmm_kernel_stream_sm100.cuh"
 #include "tiled_csl_host.h"
 #include "tiling.h"
 
@@ -46,6 +47,19 @@ void count_launch()
 
 constexpr int kMaxDevices = 64;
 
+// Scratch of the streaming form: one counter per tile row and two fp32 [N][128] parts per CTA of the largest grid at the
+// largest N it takes.  Launches on one stream follow one another, so a scratch belongs to a stream (by its unique id: a
+// handle may be reused while its old stream's work still runs).  It is allocated at the stream's first such call and kept;
+// at most kScratchStreams per device, further streams run the other forms.  FlashLLM_ReleaseScratch gives it back.
+constexpr int    kScratchStreams = 8, kScratchRows = 4096, kScratchCtas = 2 * 160, kScratchMaxN = 64;
+constexpr size_t kScratchBytes   = kScratchRows * sizeof(unsigned int)
+                                 + size_t(2) * kScratchCtas * kScratchMaxN * kTileM * sizeof(float);
+
+struct StreamScratch {
+    unsigned long long stream_id = 0;
+    unsigned char*     memory    = nullptr;
+};
+
 struct DeviceState {
     std::mutex     mutex;
     bool           ready      = false;  // set once every step of the set-up has succeeded; a failed set-up is retried
@@ -56,7 +70,37 @@ struct DeviceState {
     unsigned int*  tile_counters   = nullptr;  // device address of g_tile_counters on this device
     int            counter_streams = 0;        // streams that own a counter set so far
     cudaStream_t   counter_stream[kCounterSets] = {nullptr};
+    int            scratch_streams = 0;
+    StreamScratch  scratch[kScratchStreams];
 };
+
+// The scratch of `stream` on this device, allocated on first use; nullptr while the stream is being captured (a graph may
+// be replayed on any stream), when all places are taken, or when memory is short.
+static unsigned char* scratch_of_stream(DeviceState* st, cudaStream_t stream)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    unsigned long long      id      = 0;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone
+        || cudaStreamGetId(stream, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(st->mutex);
+    for (int i = 0; i < st->scratch_streams; ++i)
+        if (st->scratch[i].stream_id == id)
+            return st->scratch[i].memory;
+    if (st->scratch_streams >= kScratchStreams)
+        return nullptr;
+    unsigned char* memory = nullptr;
+    if (cudaMalloc(reinterpret_cast<void**>(&memory), kScratchBytes) != cudaSuccess
+        || cudaMemset(memory, 0, kScratchRows * sizeof(unsigned int)) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(memory);
+        return nullptr;
+    }
+    st->scratch[st->scratch_streams++] = {id, memory};
+    return memory;
+}
 
 // The counter set of `stream` on this device, or nullptr when all sets are taken by other streams.
 static unsigned int* counters_of_stream(DeviceState* st, cudaStream_t stream)
@@ -107,6 +151,9 @@ static cudaError_t raise_smem_limit_of(Kernel kernel, int optin)
                                 optin - static_cast<int>(attr.sharedSizeBytes));
 }
 
+// Vectors per lane the streaming form keeps in registers: what 96 registers (two CTAs of 10 warps per SM) have room for.
+constexpr int kStreamCap = 14;
+
 template<int N_TILE>
 static cudaError_t raise_smem_limit(int optin)
 {
@@ -117,6 +164,9 @@ static cudaError_t raise_smem_limit(int optin)
         e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks>, optin);
     if (e == cudaSuccess)
         e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapPair, 4, 2, 2>, optin);
+    if constexpr (N_TILE <= kScratchMaxN)
+        if (e == cudaSuccess)
+            e = raise_smem_limit_of(spmm_tcgen05_stream_kernel<N_TILE, kStreamCap>, optin);
     return e;
 }
 
@@ -213,6 +263,58 @@ static bool is_pow2(int v)
     return v > 0 && (v & (v - 1)) == 0;
 }
 
+static int stream_smem_bytes(const SpmmPlan& pl)
+{
+    return kStreamStages * kDenseTileBytes + pl.b_stages * pl.b_batch * pl.n_tile * kTileK * 2
+           + 8 * (2 * kStreamStages + 4 + 2 * pl.b_stages) + 16 + 4 * pl.offsets_staged;
+}
+
+// The streaming form: as many CTAs as the GPU holds, fewer only when there are fewer tiles.
+static cudaError_t make_stream_plan(const DeviceState* st, SpmmPlan pl, int tile_rows, int k_tiles, SpmmPlan* out)
+{
+    const long long tiles = static_cast<long long>(tile_rows) * k_tiles;
+    long long       ctas  = static_cast<long long>(kStreamCtasPerSm) * st->sm_count;
+    ctas                  = ctas < kScratchCtas ? ctas : kScratchCtas;
+    ctas                  = ctas < tiles ? ctas : tiles;
+    if (pl.n_tile > kScratchMaxN || tile_rows > kScratchRows || tiles > 0x7FFFFFFFll)
+        return cudaErrorInvalidConfiguration;
+    pl.ctas           = static_cast<int>(ctas);
+    pl.cluster_k      = 1;
+    pl.workspace_k    = 1;
+    pl.scatter_warps  = kStreamStages;
+    pl.a_stages       = kStreamStages;
+    pl.producers      = 1;
+    pl.reduce         = kReduceLastCta;
+    pl.b_batch        = 8192 / (pl.n_tile * kTileK * 2);  // 8 KB per TMA instruction ...
+    pl.b_stages       = pl.n_tile <= 32 ? 2 : 3;          // ... and four to eight tiles' worth of B ahead of the MMAs
+    const int longest = static_cast<int>((tiles + ctas - 1) / ctas);
+    pl.offsets_staged = longest + 1 <= 2048 ? ((longest + 1 + 3) / 4) * 4 : 0;
+    pl.smem_bytes     = stream_smem_bytes(pl);
+    *out              = pl;
+    return cudaSuccess;
+}
+
+// What a launch costs, in tiles of one CTA while two share an SM (0.49 us at N = 16, 80 % sparsity; 0.54 us at N = 64).
+// Fitted to launches of 8..288 tile rows by 16..512 K tiles, B200, back to back on one stream:
+//   one CTA (cluster) per tile row  10.5 + 2.3 with a cluster sum + the tiles of a CTA per wave, two thirds of that while
+//                                   no SM holds two CTAs; + 4 for a second kernel
+//   streaming form                  0.93 of the tiles of a CTA + 15 + 0.45 per part of a row at N <= 16, more for wider
+//                                   parts (the last part's CTA sums the row while everybody else has finished)
+static double one_row_cost(const DeviceState* st, long long capacity, int ctas_flat, int k_tiles, int s, int g, int n_tile)
+{
+    const long long clusters = static_cast<long long>(ctas_flat) * g;
+    const double    waves    = static_cast<double>((clusters + capacity - 1) / capacity);
+    const double    tiles    = static_cast<double>((k_tiles + s * g - 1) / (s * g)) * (clusters * s <= st->sm_count ? 0.66 : 1.0);
+    return waves * (tiles + 10.5 + (n_tile - 16) * 0.15 + (s > 1 ? 2.3 : 0.0)) + (g > 1 ? 4.0 : 0.0);
+}
+
+static double stream_cost(const SpmmPlan& pl, int tile_rows, int k_tiles)
+{
+    const double tiles = static_cast<double>(tile_rows) * k_tiles / pl.ctas;
+    const double parts = 1.0 + static_cast<double>(pl.ctas) / tile_rows;
+    return 0.93 * tiles + 15.0 + (pl.n_tile - 16) * 0.15 + 0.45 * parts * (0.5 + pl.n_tile / 32.0);
+}
+
 // Chooses how to cut K and how deep to pipeline.  Takes the place of the reference's per-N switch over
 // TilingConfig instances (csrc/SpMM_API.cu:79-118) and of its hand-tuned Split_K tables
 // (kernel_benchmark/benchmark.sh:13-15).
@@ -220,7 +322,9 @@ static bool is_pow2(int v)
 // fp16 matrices hold half as many fp32 ones).
 // `sends`: the call is the sending half of a fused all-reduce, where workspace parts are always summed by the last
 // CTA of a tile, which then also stores the sum to every GPU.
-static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max_parts, SpmmPlan* out, bool sends = false)
+// `may_stream`: the call may use the streaming form (the stream's scratch is at hand).
+static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max_parts, SpmmPlan* out, bool sends = false,
+                             bool may_stream = true)
 {
     PlanOverride ov;
     {
@@ -238,6 +342,11 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // Two pipelines per SM (4 scatter warps, 4 stages each) where they fit; wide-N tiles need the shared memory for
     // their B batches, so they run one deeper pipeline per SM instead.
     pl.path               = ov.v[kPlanPath] ? ov.v[kPlanPath] : kDefaultPath;
+    bool pinned           = false;
+    for (int v : ov.v)
+        pinned |= v != 0;
+    if (pl.path == kPathStream)  // pinned: other fields do not apply to it
+        return may_stream && !sends ? make_stream_plan(st, pl, tile_rows, k_tiles, out) : cudaErrorInvalidConfiguration;
     const bool direct     = pl.path == kPathDirect;
     pl.scatter_warps      = ov.v[kPlanScatterWarps] ? ov.v[kPlanScatterWarps]
                                                     : (direct ? (pl.n_tile <= 64 ? 4 : 8) : (pl.n_tile <= 32 ? 4 : 8));
@@ -307,6 +416,15 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
             }
         }
     }
+    if (may_stream && !pinned && !sends) {
+        SpmmPlan sp = pl;
+        sp.path     = kPathStream;
+        if (make_stream_plan(st, sp, tile_rows, k_tiles, &sp) == cudaSuccess
+            && stream_cost(sp, tile_rows, k_tiles) < one_row_cost(st, capacity(best_s), ctas_flat, k_tiles, best_s, best_g, pl.n_tile)) {
+            *out = sp;
+            return cudaSuccess;
+        }
+    }
     pl.cluster_k = ov.v[kPlanClusterK] ? ov.v[kPlanClusterK] : best_s;
     if (pl.cluster_k > k_tiles)
         pl.cluster_k = k_tiles;
@@ -355,6 +473,12 @@ static cudaError_t launch_spmm(cudaStream_t stream, const CUtensorMap& tmap, con
     auto            launch = [&](auto kernel, int warps) {
         return launch_in_stream_order(kernel, grid, dim3(warps * 32), pl.smem_bytes, stream, pl.cluster_k, tmap, params);
     };
+    if (pl.path == kPathStream) {
+        if constexpr (N_TILE <= kScratchMaxN)
+            return launch_in_stream_order(spmm_tcgen05_stream_kernel<N_TILE, kStreamCap>, dim3(pl.ctas), dim3(kStreamWarps * 32),
+                                          pl.smem_bytes, stream, 1, tmap, params);
+        return cudaErrorInvalidConfiguration;
+    }
     if (pl.path == kPathDirect) {
         const int warps = 1 + kDirectIssuers + pl.scatter_warps * pl.producers;
         if (pl.scatter_warps == 8)
@@ -448,7 +572,8 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
                                    int          activation,
                                    const half*  residual = nullptr,
                                    FlashLLMComm* comm = nullptr,
-                                   int           phases = 3)
+                                   int           phases = 3,
+                                   bool          may_allocate = true)
 {
     if (!n_supported(N_Global)) {
         printf("MM_Sparse_API Error: Unsupported N dimension %d!\n", N_Global);
@@ -468,11 +593,20 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
         return err;
 
     SpmmParams params{};
-    if ((err = make_plan(st, M_Global, N_Global, K_Global, comm ? kCommLocalParts : Split_K / 2, &params.plan,
-                         comm != nullptr))
-        != cudaSuccess)
+    SpmmPlan&  pl        = params.plan;
+    const int  max_parts = comm ? kCommLocalParts : Split_K / 2;
+    const bool sends     = comm != nullptr;
+    if ((err = make_plan(st, M_Global, N_Global, K_Global, max_parts, &pl, sends, may_allocate)) != cudaSuccess)
         return err;
-    SpmmPlan& pl = params.plan;
+    if (pl.path == kPathStream) {
+        unsigned char* scratch = scratch_of_stream(st, stream);
+        if (scratch != nullptr) {
+            params.tile_counters = reinterpret_cast<unsigned int*>(scratch);
+            params.partial       = reinterpret_cast<float*>(scratch + kScratchRows * sizeof(unsigned int));
+        }
+        else if ((err = make_plan(st, M_Global, N_Global, K_Global, max_parts, &pl, sends, false)) != cudaSuccess)
+            return err;
+    }
     // The sum over workspace parts reads 16-byte groups of the workspace and writes 8-byte groups of C.
     if (!comm && pl.workspace_k > 1
         && ((reinterpret_cast<uintptr_t>(Reduction_Workspace) & 15u) != 0 || (reinterpret_cast<uintptr_t>(C) & 7u) != 0))
@@ -481,7 +615,8 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
     params.compressed   = Compressed_A;
     params.tile_offsets = TileOffsets;
     params.out          = C;
-    params.partial      = pl.workspace_k > 1 ? reinterpret_cast<float*>(Reduction_Workspace) : nullptr;
+    if (pl.workspace_k > 1)
+        params.partial = reinterpret_cast<float*>(Reduction_Workspace);
     if (!comm && pl.workspace_k > 1 && pl.reduce == kReduceLastCta) {
         params.tile_counters = counters_of_stream(st, stream);
         if (params.tile_counters == nullptr)
@@ -699,10 +834,10 @@ int FlashLLM_SpMM_SplitK_NoAlloc(void*       stream,
     DeviceState* st  = device_state(&err);  // first call on a device: looks the scratch address up, allocates nothing
     if (!st)
         return static_cast<int>(err);
-    return static_cast<int>(SpMM_SplitK_API(static_cast<cudaStream_t>(stream), nullptr,
-                                            static_cast<const uint4*>(Compressed_A), TileOffsets,
-                                            static_cast<const half*>(B), static_cast<half*>(C), M, N, K,
-                                            reinterpret_cast<half*>(st->noalloc_scratch), Split_K));
+    return static_cast<int>(spmm_launch_all(static_cast<cudaStream_t>(stream), static_cast<const uint4*>(Compressed_A),
+                                            TileOffsets, static_cast<const half*>(B), static_cast<half*>(C), M, N, K,
+                                            reinterpret_cast<half*>(st->noalloc_scratch), Split_K, nullptr, kActNone, nullptr,
+                                            nullptr, 3, false));
 }
 
 unsigned long long FlashLLM_Comm_BufferBytes(int world, long long max_elems)
@@ -810,6 +945,21 @@ int FlashLLM_SplitK_Reduction(void* stream, void* C, const void* Reduction_Works
         return static_cast<int>(cudaErrorInvalidValue);
     return static_cast<int>(reduce_workspace(static_cast<cudaStream_t>(stream), static_cast<half*>(C),
                                              static_cast<const half*>(Reduction_Workspace), count, Split_K));
+}
+
+int FlashLLM_ReleaseScratch(void)
+{
+    cudaError_t  err = cudaSuccess;
+    DeviceState* st  = device_state(&err);
+    if (!st)
+        return static_cast<int>(err);
+    if ((err = cudaDeviceSynchronize()) != cudaSuccess)
+        return static_cast<int>(err);
+    std::lock_guard<std::mutex> lock(st->mutex);
+    for (int i = 0; i < st->scratch_streams; ++i)
+        cudaFree(st->scratch[i].memory);
+    st->scratch_streams = 0;
+    return 0;
 }
 
 void FlashLLM_SetLaunchOverlap(int enable)

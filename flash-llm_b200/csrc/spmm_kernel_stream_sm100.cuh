@@ -1,0 +1,466 @@
+// Load-as-Sparse / Compute-as-Dense SpMM for sm_100a, streaming form: a persistent grid over the linear tile sequence.
+//
+// The tiles of A in the order of TileOffsets (tile row by tile row, K tile by K tile) are ONE sequence, and so are their
+// words in Compressed_A.  CTA c of P takes tiles [T*c/P, T*(c+1)/P) of it, whatever rows they belong to, so every SM gets
+// the same share of the matrix for any number of tile rows.  (One CTA per tile row leaves SMs idle whenever the rows do
+// not fill the last wave: 216 rows on 296 CTA slots, 384 rows on 296.)  A maximal run of a CTA's tiles inside one tile row
+// is a segment:
+//
+//   * scatter warps decompress tile after tile as in the register-streaming form and know nothing of rows;
+//   * the MMA-issuing warp accumulates a segment in one of two tensor-memory accumulators and changes over at a row's
+//     end without draining anything;
+//   * four epilogue warps read a finished accumulator while the next segment is being multiplied.  A segment that is a
+//     whole row becomes output at once; a part of a row is parked as an fp32 tile in the stream's scratch and counted in
+//     on the row's counter, and whoever completes the count adds the parts up in CTA order (the same bits whoever comes
+//     last) and finishes the output.  No CTA waits for another.
+//
+// The MMA-issuing warp runs converged and elects one lane inside the instruction block: operands then stay in uniform
+// registers.  Issued from a branch taken by one lane, the four MMAs and the commit of a tile cost 271 cycles instead of
+// the 170 the tensor core needs for them (M128 N16 K16), which took two issuing warps to hide.
+//
+// Measured (B200, back to back on one stream, against one CTA or cluster per tile row): 27648x9216 N=8 90 % 62.8 -> 46.4 us,
+// 25600x9216 N=16 80 % 75.9 -> 53.0, 9216x36864 N=32 70 % 106 -> 103, 49152x12288 N=64 80 % 184 -> 166, 36864x9216 N=16
+// 80 % (288 rows: hardly any quantisation to begin with) 76.8 -> 72.0.  A CTA's share is bound by the shared-memory work of
+// its tiles: of ~3300 cycles from one tile of a stage to the next at 80 %, 570 go to clearing the stage, 1140 to the 16-bit
+// scatter stores (they wait for the tensor core's operand reads), 1070 to getting the next tile's loads issued behind the
+// other warps' stores, 430 to the stage's hand-back.  Six stages per CTA, or one CTA of 8 or 12 warps per SM, are slower.
+#pragma once
+#include "spmm_kernel_direct_sm100.cuh"
+
+namespace flashllm {
+
+constexpr int kStreamStages       = 4;  // decompressed tiles in flight per CTA, one scatter warp each
+constexpr int kStreamCtasPerSm    = 2;
+constexpr int kStreamFirstScatter = 2;  // warp 0 loads B, warp 1 issues MMAs
+constexpr int kStreamFirstEpi     = kStreamFirstScatter + kStreamStages;
+constexpr int kStreamWarps        = kStreamFirstEpi + 4;
+
+// First tile of CTA c's share, and the CTA whose share holds tile t.
+__device__ __forceinline__ int stream_begin(long long tiles, int ctas, int c)
+{
+    return static_cast<int>(tiles * c / ctas);
+}
+__device__ __forceinline__ int stream_owner(long long tiles, int ctas, long long t)
+{
+    return static_cast<int>(((t + 1) * ctas - 1) / tiles);
+}
+
+// Warp-collective bounded wait: every lane probes (the probe parks the warp for a while), one answer for all lanes.
+__device__ __forceinline__ bool
+wait_bounded_converged(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int* status)
+{
+    if (ptx::mbar_try_wait(bar, parity))
+        return true;
+    uint64_t t0 = 0;
+    bool     ok = true;
+    for (uint32_t it = 1; ok && !ptx::mbar_try_wait(bar, parity); ++it) {
+        if ((it & 255u) == 0u) {
+            if (*abort_flag)
+                ok = false;
+            else if (abort_flag[kDepsResolved] == 0u)  // still behind the previous kernel of the stream: no clock yet
+                t0 = 0;
+            else {
+                const uint64_t now = ptx::globaltimer_ns();
+                if (t0 == 0)
+                    t0 = now;
+                else if (now - t0 > kWaitLimitNs) {
+                    *abort_flag = 1u;
+                    atomicOr(status, kStatusWaitExpired);
+                    ok = false;
+                }
+            }
+        }
+    }
+    return ok;
+}
+
+// Adds the parked parts of tile row `row` up in CTA order and finishes the output (the 128 epilogue threads).
+template<int N_TILE>
+__device__ __forceinline__ void
+sum_row_parts(const SpmmParams& p, long long tiles, int ctas, int row, int c_first, int c_last, int tid)
+{
+    const long long row_begin = static_cast<long long>(row) * p.k_tiles;
+    const size_t    slot      = static_cast<size_t>(N_TILE) * kTileM;
+    const bool      wide_out  = (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
+    // only the row's first CTA may have begun before the row: this is then its last segment, in its second slot
+    const float* const first = p.partial + slot * (2 * c_first + (stream_begin(tiles, ctas, c_first) < row_begin ? 1 : 0));
+    // Four groups of four outputs per thread and three parts at a time: twelve 16-byte loads in flight (a part is an L2
+    // round trip away, and a row of a narrow matrix may have twenty of them); added in CTA order.
+    constexpr int Q = 4, P = 3;
+    const int     quads = p.N * (kTileM / 4);
+    for (int q0 = tid; q0 < quads; q0 += Q * 128) {
+        float4 acc[Q];
+#pragma unroll
+        for (int i = 0; i < Q; ++i)
+            if (q0 + i * 128 < quads)
+                acc[i] = __ldcg(reinterpret_cast<const float4*>(first) + q0 + i * 128);
+        for (int c = c_first + 1; c <= c_last; c += P) {
+            float4 v[P][Q];
+#pragma unroll
+            for (int j = 0; j < P; ++j)
+#pragma unroll
+                for (int i = 0; i < Q; ++i)
+                    if (c + j <= c_last && q0 + i * 128 < quads)
+                        v[j][i] = __ldcg(reinterpret_cast<const float4*>(p.partial + slot * (2 * (c + j))) + q0 + i * 128);
+#pragma unroll
+            for (int j = 0; j < P; ++j)
+#pragma unroll
+                for (int i = 0; i < Q; ++i)
+                    if (c + j <= c_last) {
+                        acc[i].x += v[j][i].x;
+                        acc[i].y += v[j][i].y;
+                        acc[i].z += v[j][i].z;
+                        acc[i].w += v[j][i].w;
+                    }
+        }
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            const int q = q0 + i * 128;
+            if (q >= quads)
+                break;
+            const int    n = q / (kTileM / 4), out_row = row * kTileM + (q % (kTileM / 4)) * 4;
+            const size_t at = static_cast<size_t>(n) * p.M + out_row;
+            uint2        o;
+            half*        oh = reinterpret_cast<half*>(&o);
+            oh[0]           = finish_output(acc[i].x, p.bias, out_row, p.activation, p.residual, at);
+            oh[1]           = finish_output(acc[i].y, p.bias, out_row + 1, p.activation, p.residual, at + 1);
+            oh[2]           = finish_output(acc[i].z, p.bias, out_row + 2, p.activation, p.residual, at + 2);
+            oh[3]           = finish_output(acc[i].w, p.bias, out_row + 3, p.activation, p.residual, at + 3);
+            if (wide_out)
+                *reinterpret_cast<uint2*>(p.out + at) = o;
+            else
+                for (int e = 0; e < 4; ++e)
+                    p.out[at + e] = oh[e];
+        }
+    }
+}
+
+template<int N_TILE, int CAP>
+__global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
+    spmm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap tmap_b, const SpmmParams p)
+{
+    static_assert(N_TILE == 16 || N_TILE == 32 || N_TILE == 64, "unsupported MMA N");
+    constexpr uint32_t kBSlab    = N_TILE * kTileK * 2;              // one K tile of B in shared memory
+    constexpr uint32_t kTmemCols = 2 * N_TILE < 32 ? 32 : 2 * N_TILE;  // two accumulators
+
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    const uint32_t raw_addr = ptx::smem_u32(smem_raw);
+    const uint32_t base     = (raw_addr + 1023u) & ~1023u;  // swizzled operands need 1024-byte alignment
+    uint8_t* const smem     = smem_raw + (base - raw_addr);
+
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);  // uniform: the issuing warp stays converged
+    const int lane = threadIdx.x & 31;
+
+    const int       b_stages = p.plan.b_stages;
+    const int       KB       = p.plan.b_batch;
+    const int       ctas     = gridDim.x;
+    const int       cta      = blockIdx.x;
+    const long long tiles    = static_cast<long long>(p.M / kTileM) * p.k_tiles;
+    const int       t_begin  = stream_begin(tiles, ctas, cta);
+    const int       L        = stream_begin(tiles, ctas, cta + 1) - t_begin;  // >= 1: the grid has at most `tiles` CTAs
+    const int       row0     = t_begin / p.k_tiles;
+    const int       k0       = t_begin - row0 * p.k_tiles;  // K tile the CTA starts at
+
+    // ---- shared memory carve-up
+    const uint32_t a_base    = base;
+    const uint32_t b_base    = a_base + kStreamStages * kDenseTileBytes;
+    const uint32_t a_full    = b_base + b_stages * KB * kBSlab;
+    const uint32_t a_empty   = a_full + 8u * kStreamStages;
+    const uint32_t acc_full  = a_empty + 8u * kStreamStages;  // two of each: the accumulators take turns
+    const uint32_t acc_empty = acc_full + 16u;
+    const uint32_t b_full    = acc_empty + 16u;
+    const uint32_t b_empty   = b_full + 8u * b_stages;
+    const uint32_t misc_off  = (b_empty + 8u * b_stages) - base;
+    volatile uint32_t* const tmem_slot  = reinterpret_cast<volatile uint32_t*>(smem + misc_off);
+    volatile uint32_t* const abort_flag = reinterpret_cast<volatile uint32_t*>(smem + misc_off + 4);
+    int* const               offs_stage = reinterpret_cast<int*>(smem + misc_off + 16);  // plan.offsets_staged ints
+
+    const int* const offs_global = p.tile_offsets + t_begin;
+    const bool       staged      = (L + 1 <= p.plan.offsets_staged);
+    const int* const offs        = staged ? offs_stage : offs_global;  // valid after the set-up barrier
+
+    if (raw_addr != base) {  // the launch did not honour the 1024-byte alignment: nothing below would be valid
+        if (threadIdx.x == 0)
+            atomicOr(p.status, kStatusSmemMisaligned);
+        return;
+    }
+
+    // ---- scatter warps request their first tile before anything else (see the register-streaming form)
+    const bool   scatters = warp >= kStreamFirstScatter && warp < kStreamFirstEpi;
+    const int    sw       = warp - kStreamFirstScatter;  // the stage, and the tile stream sw, sw + kStreamStages, ...
+    uint4        nxt[CAP];
+    int          n_in = 0;
+    const uint4* src  = p.compressed;
+    bool         bad  = false;
+    auto fetch_first_tile = [&]() {
+        if (sw < L) {
+            const int vb = offs_global[sw], ve = offs_global[sw + 1];
+            bad          = (ve < vb) || (ve - vb > kMaxTileVectors) || (vb < 0);
+            n_in         = bad ? 0 : ve - vb;
+            src          = p.compressed + (bad ? 0 : vb);
+            load_batch<1, CAP>(nxt, src + lane, n_in, n_in - lane);
+        }
+    };
+    if (scatters) {
+#pragma unroll
+        for (int q = 0; q < CAP; ++q)
+            nxt[q] = make_uint4(0u, 0u, 0u, 0u);
+        if (p.early_weights)
+            fetch_first_tile();
+    }
+
+    // ---- set-up
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStreamStages; ++i) {
+            ptx::mbar_init(a_full + 8u * i, 1);
+            ptx::mbar_init(a_empty + 8u * i, 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            ptx::mbar_init(acc_full + 8u * i, 1);
+            ptx::mbar_init(acc_empty + 8u * i, 4);  // every epilogue warp hands its quarter back
+        }
+        for (int i = 0; i < b_stages; ++i) {
+            ptx::mbar_init(b_full + 8u * i, 1);
+            ptx::mbar_init(b_empty + 8u * i, 1);
+        }
+        abort_flag[0]             = 0u;
+        abort_flag[kDepsResolved] = 0u;
+        ptx::fence_mbar_init();
+        ptx::prefetch_tensormap(&tmap_b);
+    }
+    if (warp == 1) {
+        ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
+        ptx::tmem_relinquish();
+    }
+    if (!p.early_weights) {
+        ptx::grid_dependency_wait();
+        if (scatters)
+            fetch_first_tile();
+    }
+    if (staged) {
+        for (int i = threadIdx.x; i <= L; i += blockDim.x)
+            offs_stage[i] = offs_global[i];
+    }
+    bool bad_slice = offsets_slice_is_bad(offs_global, L);
+    ptx::tc_fence_before_sync();
+    bad_slice = __syncthreads_or(bad_slice ? 1 : 0) != 0;
+    ptx::tc_fence_after_sync();
+    const bool go = !bad_slice;  // false: every role skips its work and nothing is stored
+    if (bad_slice && threadIdx.x == 0) {
+        atomicOr(p.status, kStatusBadTileOffsets);
+        *abort_flag = 1u;
+    }
+    const uint32_t tmem_acc = *tmem_slot;
+    if (threadIdx.x == 0)
+        ptx::grid_launch_dependents();
+
+    if (warp == 0) {
+        // ================================================================ B loader: KB K tiles per TMA instruction
+        if (lane == 0 && go) {
+            ptx::grid_dependency_wait();
+            abort_flag[kDepsResolved] = 1u;
+            int      bs = 0, issued = 0;
+            uint32_t use = 0;
+            bool     ok  = true;
+            for (int j = 0, k = k0; ok && j < L; k = 0) {
+                const int len = L - j < p.k_tiles - k ? L - j : p.k_tiles - k;  // this segment
+                for (int b = 0; b < len; b += KB) {
+                    if (!wait_bounded_relaxed(b_empty + 8u * bs, (use & 1u) ^ 1u, abort_flag, p.status)) {
+                        ok = false;
+                        break;
+                    }
+                    ptx::mbar_arrive_expect_tx(b_full + 8u * bs, KB * kBSlab);
+                    ptx::tma_load_3d(b_base + bs * KB * kBSlab, &tmap_b, 0, 0, k + b, b_full + 8u * bs);
+                    ++issued;
+                    if (++bs == b_stages) {
+                        bs = 0;
+                        ++use;
+                    }
+                }
+                j += len;
+            }
+            if (*abort_flag) {  // give copies already issued a bounded chance to land before the CTA may exit
+                const uint64_t t_leave = ptx::globaltimer_ns();
+                for (int back = 1; back <= b_stages && back <= issued; ++back) {
+                    const int bb = issued - back;
+                    while (!ptx::mbar_test_wait(b_full + 8u * (bb % b_stages), (bb / b_stages) & 1u)
+                           && ptx::globaltimer_ns() - t_leave < 2000000ull) {}
+                }
+            }
+        }
+    }
+    else if (warp == 1) {
+        // ================================================================ MMA issuer (converged warp)
+        if (go) {
+            const uint32_t idesc   = ptx::umma_idesc_f16_f32(kTileM, N_TILE);
+            const uint64_t a_desc0 = ptx::umma_desc_kmajor_sw128(a_base);
+            const uint64_t b_desc0 = ptx::umma_desc_kmajor_sw128(b_base);
+            int            s = 0, bs = 0, seg = 0;
+            uint32_t       a_par = 0, b_par = 0;
+            bool           ok = true;
+            for (int j = 0, k = k0; ok && j < L; k = 0, ++seg) {
+                const int      len = L - j < p.k_tiles - k ? L - j : p.k_tiles - k;
+                const uint32_t acc = tmem_acc + static_cast<uint32_t>((seg & 1) * N_TILE);
+                ok = __all_sync(0xFFFFFFFFu, wait_bounded_converged(acc_empty + 8u * (seg & 1), ((seg >> 1) & 1u) ^ 1u, abort_flag,
+                                                                    p.status));
+                for (int i = 0, kb = 0; ok && i < len; ++i) {
+                    ok = wait_bounded_converged(a_full + 8u * s, a_par, abort_flag, p.status);
+                    if (kb == 0)
+                        ok = wait_bounded_converged(b_full + 8u * bs, b_par, abort_flag, p.status) && ok;
+                    ok = __all_sync(0xFFFFFFFFu, ok);
+                    if (!ok)
+                        break;
+                    const bool batch_done = kb + 1 == KB || i + 1 == len;
+                    ptx::tc_fence_after_sync();
+                    ptx::umma_tile_elect(acc, a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
+                                         b_desc0 + static_cast<uint32_t>((bs * KB + kb) * (kBSlab >> 4)), idesc, i != 0 ? 1u : 0u,
+                                         a_empty + 8u * s, b_empty + 8u * bs, batch_done ? 1u : 0u);
+                    if (++s == kStreamStages) {
+                        s = 0;
+                        a_par ^= 1u;
+                    }
+                    ++kb;
+                    if (batch_done) {
+                        kb = 0;
+                        if (++bs == b_stages) {
+                            bs = 0;
+                            b_par ^= 1u;
+                        }
+                    }
+                }
+                if (ok)
+                    ptx::umma_commit_elect(acc_full + 8u * (seg & 1));
+                j += len;
+            }
+        }
+    }
+    else if (warp < kStreamFirstEpi) {
+        // ================================================================ scatter warps: one whole tile at a time
+        if (go) {
+            const uint32_t stage     = a_base + sw * kDenseTileBytes;
+            const uint32_t full_bar  = a_full + 8u * sw;
+            const uint32_t empty_bar = a_empty + 8u * sw;
+            if (lane == 0) {
+                for (int a = 1; a < kPrefetchAhead; ++a) {
+                    const int t = sw + a * kStreamStages;
+                    if (t < L && offs[t + 1] > offs[t])
+                        ptx::prefetch_l2_bulk(p.compressed + offs[t], static_cast<uint32_t>(offs[t + 1] - offs[t]) * 16u);
+                }
+            }
+            uint32_t use = 0;
+            for (int j = sw; j < L; j += kStreamStages, ++use) {
+                bool ok = !bad;
+                if (use > 0)
+                    ok = wait_bounded_converged(empty_bar, (use & 1u) ^ 1u, abort_flag, p.status) && ok;
+                if (!__all_sync(0xFFFFFFFFu, ok))
+                    break;
+                // offsets of this warp's following tile: read here, where the load/store unit is idle (see the
+                // register-streaming form)
+                const bool has_next = j + kStreamStages < L;
+                int        vb2 = 0, ve2 = 0;
+                if (has_next) {
+                    vb2 = offs[j + kStreamStages];
+                    ve2 = offs[j + kStreamStages + 1];
+                }
+                zero_fill_stage(stage, lane);
+                __syncwarp();  // another lane's zero must not land on top of a new value
+                const int rem = n_in - lane;
+                scatter_batch<1, CAP>(stage, nxt, n_in, rem);
+                for (int v0 = CAP * 32; v0 < n_in; v0 += CAP * 32) {  // tiles denser than the register budget
+                    load_batch<1, CAP>(nxt, src + v0 + lane, n_in - v0, rem - v0);
+                    scatter_batch<1, CAP>(stage, nxt, n_in - v0, rem - v0);
+                }
+                ptx::fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0)
+                    ptx::mbar_arrive(full_bar);
+                if (has_next) {  // start fetching the following tile, and pull the one after it into L2
+                    bad  = (ve2 < vb2) || (ve2 - vb2 > kMaxTileVectors) || (vb2 < 0);
+                    n_in = bad ? 0 : ve2 - vb2;
+                    src  = p.compressed + (bad ? 0 : vb2);
+                    load_batch<1, CAP>(nxt, src + lane, n_in, n_in - lane);
+                    if (lane == 0 && j + kPrefetchAhead * kStreamStages < L) {
+                        const int pb = offs[j + kPrefetchAhead * kStreamStages], pe = offs[j + kPrefetchAhead * kStreamStages + 1];
+                        if (pe > pb)
+                            ptx::prefetch_l2_bulk(p.compressed + pb, static_cast<uint32_t>(pe - pb) * 16u);
+                    }
+                }
+            }
+        }
+    }
+    else {
+        // ================================================================ epilogue warps
+        const int tid     = threadIdx.x - kStreamFirstEpi * 32;
+        const int quarter = warp & 3;  // the tensor-memory lanes this warp may read
+        const int r       = quarter * 32 + lane;
+        int       seg     = 0;
+        for (int j = 0, k = k0, row = row0; j < L; k = 0, ++row, ++seg) {
+            const int      len   = L - j < p.k_tiles - k ? L - j : p.k_tiles - k;
+            const bool     whole = len == p.k_tiles;
+            const uint32_t acc   = tmem_acc + static_cast<uint32_t>((seg & 1) * N_TILE) + (static_cast<uint32_t>(quarter * 32) << 16);
+            bool           ok    = go && wait_bounded_converged(acc_full + 8u * (seg & 1), (seg >> 1) & 1u, abort_flag, p.status);
+            ok                   = __all_sync(0xFFFFFFFFu, ok);
+            ptx::tc_fence_after_sync();
+            float* const park = whole ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (seg == 0 ? 0 : 1)) + r;
+            if (ok) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < N_TILE; c0 += 16) {
+                    uint32_t t0[8], t1[8];
+                    ptx::tmem_ld_x8(acc + c0, t0);
+                    ptx::tmem_ld_x8(acc + c0 + 8, t1);
+                    ptx::tmem_wait_ld();
+                    if (c0 + 16 == N_TILE) {  // the accumulator has been read: the issuer may start a segment in it
+                        ptx::tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0)
+                            ptx::mbar_arrive(acc_empty + 8u * (seg & 1));
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const int   n = c0 + i;
+                        const float v = __uint_as_float(i < 8 ? t0[i & 7] : t1[i & 7]);
+                        if (n < p.N) {
+                            if (park != nullptr)
+                                __stcg(park + n * kTileM, v);
+                            else {
+                                const size_t at = static_cast<size_t>(n) * p.M + row * kTileM + r;
+                                p.out[at]       = finish_output(v, p.bias, row * kTileM + r, p.activation, p.residual, at);
+                            }
+                        }
+                    }
+                }
+            }
+            if (!whole) {
+                const long long row_begin = static_cast<long long>(row) * p.k_tiles;
+                const int       c_first   = stream_owner(tiles, ctas, row_begin);
+                const int       c_last    = stream_owner(tiles, ctas, row_begin + p.k_tiles - 1);
+                const bool gave_up = barrier_any(1u, 128u, !ok);
+                if (tid == 0) {
+                    // arrivals in the low half of the counter; a CTA that gave up also marks the high half, so that the
+                    // last one knows the row's sum is not to be trusted
+                    const unsigned int mine = gave_up ? 0x10001u : 1u;
+                    ptx::grid_dependency_wait();  // counters may be in use by the stream's previous launch until it is over
+                    const unsigned int before = ptx::atom_add_acq_rel_gpu(p.tile_counters + row, mine);
+                    const bool         last   = (before & 0xFFFFu) + 1u == static_cast<unsigned int>(c_last - c_first + 1);
+                    if (last)
+                        p.tile_counters[row] = 0u;  // nobody else touches it again in this launch
+                    abort_flag[kLastOfTile] = last ? (((before + mine) >> 16) != 0u ? 2u : 1u) : 0u;
+                }
+                ptx::named_barrier_sync(1u, 128u);
+                if (abort_flag[kLastOfTile] == 1u) {
+                    sum_row_parts<N_TILE>(p, tiles, ctas, row, c_first, c_last, tid);
+                }
+                ptx::named_barrier_sync(1u, 128u);  // kLastOfTile is free again
+            }
+            j += len;
+        }
+    }
+
+    // ================================================================ tear-down
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 1)
+        ptx::tmem_dealloc(tmem_acc, kTmemCols);
+}
+
+}  // namespace flashllm

@@ -49,9 +49,11 @@ constexpr int kReduceLastCta      = 2;  // inside the SpMM kernel, by the last C
 
 constexpr int kPathRing   = 1;  // bulk copies into a shared-memory ring (spmm_tcgen05_kernel)
 constexpr int kPathDirect = 2;  // global loads into the scatter warps' registers (spmm_tcgen05_direct_kernel)
+constexpr int kPathStream = 3;  // the same, as a persistent grid over the linear tile sequence (spmm_tcgen05_stream_kernel)
 
 struct SpmmPlan {
-    int path;    // kPathRing or kPathDirect
+    int path;    // kPathRing, kPathDirect or kPathStream
+    int ctas;    // kPathStream: CTAs of the persistent grid
     int n_tile;  // MMA N: 16, 32, 64 or 128
     int cluster_k;
     int workspace_k;

@@ -291,6 +291,13 @@ int FlashLLM_SplitK_Reduction(void* stream, void* C, const void* Reduction_Works
  * case).  Off by default.  Process-wide. */
 void FlashLLM_SetLaunchOverlap(int enable);
 
+/* Gives back the current device's scratch memory (about 20 MB for each of at most 8 streams).  An SpMM that runs as a
+ * persistent grid over all tiles of the matrix parks the parts of tile rows shared between CTAs there; it is allocated at
+ * a stream's first such call (never while the stream is being captured, nor by FlashLLM_SpMM_SplitK_NoAlloc: those calls
+ * run the forms that need none).  Synchronises the device; no call may be made concurrently from another thread; the next
+ * call allocates again. */
+int FlashLLM_ReleaseScratch(void);
+
 /* Tuning hook replacing the reference's compile-time TilingConfig<...> choice (csrc/TilingConfig.h:36-52,
  * csrc/SpMM_API.cu:79-118): fixes launch-plan fields for subsequent calls from this process.  `fields` holds up to
  * eleven ints, 0 = choose automatically, in this order:
@@ -306,7 +313,9 @@ void FlashLLM_SetLaunchOverlap(int enable);
  *                     with 4 scatter_warps: 2 = two warps share every tile (8 scatter warps on 4 stages)
  *   9 path            1 = ring form: the compressed stream is copied into a shared-memory ring by bulk copies;
  *                     2 = register-streaming form (the default): scatter warps load their tiles' words from global
- *                     memory into registers, tiles alternate between two MMA-issuing threads
+ *                     memory into registers, tiles alternate between two MMA-issuing threads;
+ *                     3 = streaming form: the same work dealt out as one linear sequence of tiles over a persistent grid
+ *                     (N <= 64; chosen where one CTA per tile row would leave SMs idle; the other fields do not apply)
  *  10 reduce          who adds the workspace parts up: 1 = a second kernel (the default; with launch overlap it
  *                     hides behind the neighbouring SpMMs); 2 = the SpMM kernel itself: every CTA parks its fp32
  *                     partial tile and counts itself in on a counter of the output tile, the CTA that completes the

@@ -1,0 +1,107 @@
+"""The streaming form of the SpMM kernel (a persistent grid over the linear tile sequence) where its shares of the
+sequence can go wrong: fewer tiles than CTAs, shares inside one tile row, shares that end exactly at a row's end, rows cut
+into two and into many parts, tiles above the register budget; with every output epilogue, on several streams, and with
+malformed offsets."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import DeviceProblem, assert_close, random_problem
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def streaming(lib):
+    lib.set_plan(path=lib.api.PATH_STREAM)
+    yield
+    lib.set_plan()
+
+
+@pytest.mark.parametrize("M,K,N,sparsity", [
+    (128, 64, 16, 0.8),          # one tile, one CTA
+    (128, 64 * 37, 8, 0.8),      # one row in 37 single-tile parts
+    (384, 64 * 5, 32, 0.7),      # fewer tiles than CTAs, three rows
+    (128 * 37, 64 * 8, 16, 0.9), # 296 tiles: one per CTA on 148 SMs, eight parts to a row
+    (128 * 37, 64 * 16, 64, 0.8),# two tiles per CTA, shares ending at row ends
+    (128 * 41, 64 * 13, 16, 0.8),# nothing divides anything
+    (128 * 74, 64 * 9, 32, 0.75),# rows cut into two or three parts
+    (128 * 300, 64 * 3, 16, 0.8),# more rows than CTAs: whole rows inside a share
+    (256, 64 * 700, 16, 0.5),    # long shares, tiles above the register budget
+    (256, 64 * 400, 64, 0.99),   # many parts of a wide output, nearly empty tiles
+])
+def test_shares_of_the_tile_sequence(lib, oracle, streaming, M, K, N, sparsity):
+    A, B = random_problem(lib, M, K, N, sparsity, M + K + N)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    prob = DeviceProblem(lib, comp, offs, B, M, N, K, 1)
+    first = prob.run().copy()
+    assert_close(first, oracle.gemm_f32(A, B), f"M={M} K={K} N={N} s={sparsity}")
+    for _ in range(5):  # parts are added in CTA order, whichever CTA finishes the row
+        assert np.array_equal(prob.run(), first)
+
+
+@pytest.mark.parametrize("bias,relu,residual", [(True, False, False), (True, True, False), (True, False, True), (False, True, True)])
+def test_output_epilogues(lib, oracle, streaming, bias, relu, residual):
+    """Whole rows leave through one epilogue and summed rows through another; C only two-byte aligned takes narrow stores."""
+    M, K, N = 128 * 41, 64 * 13, 16
+    A, B = random_problem(lib, M, K, N, 0.8, 17)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    rng = np.random.default_rng(18)
+    b = (rng.standard_normal(M) * 2).astype(np.float16)
+    r = (rng.standard_normal((N, M)) * 4).astype(np.float16)
+    want = oracle.gemm_f32(A, B) + (b.astype(np.float32)[None, :] if bias else 0)
+    want = (np.maximum(want, 0) if relu else want) + (r.astype(np.float32) if residual else 0)
+    to_dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    comp_d, offs_d, B_d, b_d, r_d = to_dev(comp.view(np.int32)), to_dev(offs), to_dev(B), to_dev(b), to_dev(r)
+    for shift in (0, 1):
+        C = torch.full((N * M + 8,), float("nan"), dtype=torch.float16, device="cuda")[shift:shift + N * M]
+        lib.spmm_splitk_epilogue(torch.cuda.current_stream().cuda_stream, comp_d.data_ptr(), offs_d.data_ptr(), B_d.data_ptr(),
+                                 C.data_ptr(), M, N, K, None, 1, b_d.data_ptr() if bias else None,
+                                 lib.ACT_RELU if relu else lib.ACT_NONE, r_d.data_ptr() if residual else None)
+        torch.cuda.synchronize()
+        assert lib.consume_status() == 0
+        assert_close(C.view(N, M).cpu().numpy(), want, f"bias={bias} relu={relu} residual={residual} shift={shift}")
+
+
+def test_streams_without_a_scratch_of_their_own_run_another_form(lib, oracle):
+    """At most eight streams hold scratch; calls on further streams, and after the scratch was given back, are still right."""
+    M, K, N = 128 * 100, 64 * 40, 16
+    A, B = random_problem(lib, M, K, N, 0.8, 23)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    want = oracle.gemm_f32(A, B)
+    assert lib.get_plan(M, N, K, 1)["path"] == lib.api.PATH_STREAM, "this case is meant to be streamed"
+    prob = DeviceProblem(lib, comp, offs, B, M, N, K, 1)
+    for s in [torch.cuda.current_stream()] + [torch.cuda.Stream() for _ in range(12)]:
+        with torch.cuda.stream(s):
+            assert_close(prob.run(), want, "one of many streams")
+    lib.release_scratch()
+    assert_close(prob.run(), want, "after the scratch was released")
+
+
+def test_a_captured_call_needs_no_scratch(lib, oracle):
+    M, K, N = 128 * 100, 64 * 40, 16
+    A, B = random_problem(lib, M, K, N, 0.8, 29)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    prob = DeviceProblem(lib, comp, offs, B, M, N, K, 1)
+    prob.run()
+    prob.C.fill_(float("nan"))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        lib.SpMM_SplitK_API(torch.cuda.current_stream().cuda_stream, None, prob.comp.data_ptr(), prob.offs.data_ptr(),
+                            prob.B.data_ptr(), prob.C.data_ptr(), M, N, K, None, 1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert lib.consume_status() == 0
+    assert_close(prob.C.cpu().numpy(), oracle.gemm_f32(A, B), "replayed")
+
+
+def test_malformed_offsets_are_reported_not_followed(lib, oracle, streaming):
+    """The CTA that meets them gives up, its rows are not stored, the counters are left clean for the next call."""
+    M, K, N = 128 * 37, 64 * 16, 16
+    A, B = random_problem(lib, M, K, N, 0.8, 31)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    broken = offs.copy()
+    broken[5] = broken[4] - 3
+    DeviceProblem(lib, comp, broken, B, M, N, K, 1).run(check_status=False)
+    assert lib.consume_status() & 2
+    assert_close(DeviceProblem(lib, comp, offs, B, M, N, K, 1).run(), oracle.gemm_f32(A, B), "call after a malformed one")
