@@ -230,7 +230,8 @@ def SpMM_SplitK_API(stream: int, A: int | None, Compressed_A: int, TileOffsets: 
     All buffer arguments are integer device pointers; ``A`` is unused and may be ``None``."""
     code = library().FlashLLM_SpMM_SplitK(stream, A, Compressed_A, TileOffsets, B, C_out, M, N, K,
                                           Reduction_Workspace, Split_K)
-    _check(code, f"SpMM_SplitK_API(M={M}, N={N}, K={K}, Split_K={Split_K})")
+    if code:  # the message is only put together for an error: it costs as much as the call
+        _check(code, f"SpMM_SplitK_API(M={M}, N={N}, K={K}, Split_K={Split_K})")
 
 
 ACT_NONE, ACT_RELU = 0, 1
@@ -243,7 +244,8 @@ def spmm_splitk_bias_act(stream: int, Compressed_A: int, TileOffsets: int, B: in
     rounding; ``bias`` is a device pointer to M halves or ``None``, ``activation`` ``ACT_NONE`` or ``ACT_RELU``."""
     code = library().FlashLLM_SpMM_SplitK_BiasAct(stream, Compressed_A, TileOffsets, B, C_out, M, N, K,
                                                   Reduction_Workspace, Split_K, bias, activation)
-    _check(code, f"SpMM_SplitK_BiasAct(M={M}, N={N}, K={K}, Split_K={Split_K})")
+    if code:
+        _check(code, f"SpMM_SplitK_BiasAct(M={M}, N={N}, K={K}, Split_K={Split_K})")
 
 
 def spmm_splitk_epilogue(stream: int, Compressed_A: int, TileOffsets: int, B: int, C_out: int, M: int, N: int, K: int,
@@ -254,7 +256,8 @@ def spmm_splitk_epilogue(stream: int, Compressed_A: int, TileOffsets: int, B: in
     matmul).  ``residual`` is a device matrix laid out like C that does not overlap it, or ``None``."""
     code = library().FlashLLM_SpMM_SplitK_Epilogue(stream, Compressed_A, TileOffsets, B, C_out, M, N, K,
                                                    Reduction_Workspace, Split_K, bias, activation, residual)
-    _check(code, f"SpMM_SplitK_Epilogue(M={M}, N={N}, K={K}, Split_K={Split_K})")
+    if code:
+        _check(code, f"SpMM_SplitK_Epilogue(M={M}, N={N}, K={K}, Split_K={Split_K})")
 
 
 def spmm_splitk_no_alloc(stream: int, Compressed_A: int, TileOffsets: int, B: int, C_out: int, M: int, N: int, K: int,
@@ -264,7 +267,8 @@ def spmm_splitk_no_alloc(stream: int, Compressed_A: int, TileOffsets: int, B: in
     library instead of a caller workspace.  ``Split_K*M*N*2`` must fit in it.  Calls that overlap on the GPU share
     that array and race; the first call on a device should precede any stream capture."""
     code = library().FlashLLM_SpMM_SplitK_NoAlloc(stream, Compressed_A, TileOffsets, B, C_out, M, N, K, Split_K)
-    _check(code, f"SpMM_SplitK_NoAlloc(M={M}, N={N}, K={K}, Split_K={Split_K})")
+    if code:
+        _check(code, f"SpMM_SplitK_NoAlloc(M={M}, N={N}, K={K}, Split_K={Split_K})")
 
 
 # ----------------------------------------------------------------------------- fused row-parallel SpMM + all-reduce
@@ -327,7 +331,8 @@ def spmm_splitk_allreduce(comm, stream: int, Compressed_A: int, TileOffsets: int
     2 = the summing kernel only (for driving several ranks from one stream: all ranks' phase 1, then their phase 2)."""
     code = library().FlashLLM_SpMM_SplitK_AllReduce(comm, stream, Compressed_A, TileOffsets, B, C_out, M, N, K, bias,
                                                     activation, residual, phases)
-    _check(code, f"SpMM_SplitK_AllReduce(M={M}, N={N}, K={K})")
+    if code:
+        _check(code, f"SpMM_SplitK_AllReduce(M={M}, N={N}, K={K})")
 
 
 def splitk_reduction(stream: int, C_out: int, workspace: int, M: int, N: int, split_k: int) -> None:

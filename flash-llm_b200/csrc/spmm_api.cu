@@ -241,6 +241,7 @@ struct PlanOverride {
 };
 static PlanOverride g_override;
 static std::mutex   g_override_mutex;
+static std::atomic<unsigned> g_override_version{0};  // counts FlashLLM_SetPlan calls
 static std::atomic<int> g_launch_overlap{0};
 
 
@@ -464,6 +465,61 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     return cudaSuccess;
 }
 
+// B as a 3-D tensor {64 K-elements (inner), N, K/64}: one box = b_batch K tiles of [n_tile x 64], each stored as a
+// 128-byte-swizzled slab; rows past N and K tiles past K/64 read as 0.
+static cudaError_t encode_b_map(const half* B, int N, int K, const SpmmPlan& pl, CUtensorMap* map)
+{
+    const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(kTileK), static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(K / kTileK)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K) * 2, static_cast<cuuint64_t>(kTileK) * 2};
+    const cuuint32_t box[3]     = {static_cast<cuuint32_t>(kTileK), static_cast<cuuint32_t>(pl.n_tile),
+                                   static_cast<cuuint32_t>(pl.b_batch)};
+    const cuuint32_t estr[3]    = {1, 1, 1};
+    const CUresult   r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<half*>(B), dims, strides, box, estr,
+                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// What a call derives from its sizes and B's address alone, kept per thread: a decode loop repeats a few dozen calls, and
+// the search over K cuts and the tensor map's encoding are 2 us of each, a third of a small call.
+struct CallKey {
+    const DeviceState* device;
+    int                M, N, K, max_parts;
+    bool               sends, may_stream, overlap;
+    unsigned           override_version;
+    bool operator==(const CallKey& o) const
+    {
+        return device == o.device && M == o.M && N == o.N && K == o.K && max_parts == o.max_parts && sends == o.sends
+               && may_stream == o.may_stream && overlap == o.overlap && override_version == o.override_version;
+    }
+};
+struct CallMemo {
+    CallKey     key{};
+    SpmmPlan    plan{};
+    const half* B = nullptr;  // what `map` was encoded for
+    CUtensorMap map{};
+};
+
+static cudaError_t plan_call(const CallKey& key, CallMemo** out)
+{
+    constexpr unsigned kEntries = 64;
+    static thread_local CallMemo memo[kEntries];
+    const unsigned hash = (static_cast<unsigned>(key.M) / kTileM * 2654435761u) ^ (static_cast<unsigned>(key.K) / kTileK * 40503u)
+                          ^ (static_cast<unsigned>(key.N) * 97u) ^ static_cast<unsigned>(key.max_parts + key.may_stream);
+    CallMemo& m = memo[(hash ^ (hash >> 16)) % kEntries];
+    if (!(m.key == key)) {
+        SpmmPlan          plan{};
+        const cudaError_t err = make_plan(key.device, key.M, key.N, key.K, key.max_parts, &plan, key.sends, key.may_stream);
+        if (err != cudaSuccess)
+            return err;
+        m.key  = key;
+        m.plan = plan;
+        m.B    = nullptr;
+    }
+    *out = &m;
+    return cudaSuccess;
+}
+
 template<int N_TILE>
 static cudaError_t launch_spmm(cudaStream_t stream, const CUtensorMap& tmap, const SpmmParams& params, int tile_rows,
                                int n_tiles)
@@ -593,20 +649,26 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
         return err;
 
     SpmmParams params{};
-    SpmmPlan&  pl        = params.plan;
-    const int  max_parts = comm ? kCommLocalParts : Split_K / 2;
-    const bool sends     = comm != nullptr;
-    if ((err = make_plan(st, M_Global, N_Global, K_Global, max_parts, &pl, sends, may_allocate)) != cudaSuccess)
+    SpmmPlan&  pl = params.plan;
+    CallKey    key{st,           M_Global,     N_Global, K_Global, comm ? kCommLocalParts : Split_K / 2,
+                comm != nullptr, may_allocate, g_launch_overlap.load(std::memory_order_relaxed) != 0,
+                g_override_version.load(std::memory_order_relaxed)};
+    CallMemo*  memo = nullptr;
+    if ((err = plan_call(key, &memo)) != cudaSuccess)
         return err;
-    if (pl.path == kPathStream) {
+    if (memo->plan.path == kPathStream) {
         unsigned char* scratch = scratch_of_stream(st, stream);
         if (scratch != nullptr) {
             params.tile_counters = reinterpret_cast<unsigned int*>(scratch);
             params.partial       = reinterpret_cast<float*>(scratch + kScratchRows * sizeof(unsigned int));
         }
-        else if ((err = make_plan(st, M_Global, N_Global, K_Global, max_parts, &pl, sends, false)) != cudaSuccess)
-            return err;
+        else {
+            key.may_stream = false;
+            if ((err = plan_call(key, &memo)) != cudaSuccess)
+                return err;
+        }
     }
+    pl = memo->plan;
     // The sum over workspace parts reads 16-byte groups of the workspace and writes 8-byte groups of C.
     if (!comm && pl.workspace_k > 1
         && ((reinterpret_cast<uintptr_t>(Reduction_Workspace) & 15u) != 0 || (reinterpret_cast<uintptr_t>(C) & 7u) != 0))
@@ -632,20 +694,13 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
     params.K            = K_Global;
     params.k_tiles      = K_Global / kTileK;
 
-    // B as a 3-D tensor {64 K-elements (inner), N, K/64}: one box = b_batch K tiles of [n_tile x 64], each stored as
-    // a 128-byte-swizzled slab; rows past N and K tiles past K/64 read as 0.
-    CUtensorMap      tmap;
-    const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(kTileK), static_cast<cuuint64_t>(N_Global),
-                                   static_cast<cuuint64_t>(K_Global / kTileK)};
-    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K_Global) * 2, static_cast<cuuint64_t>(kTileK) * 2};
-    const cuuint32_t box[3]     = {static_cast<cuuint32_t>(kTileK), static_cast<cuuint32_t>(pl.n_tile),
-                                   static_cast<cuuint32_t>(pl.b_batch)};
-    const cuuint32_t estr[3]    = {1, 1, 1};
-    const CUresult   cres       = g_encode_tiled(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<half*>(B), dims,
-                                       strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cres != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
+    if (memo->B != B) {
+        memo->B = nullptr;
+        if ((err = encode_b_map(B, N_Global, K_Global, pl, &memo->map)) != cudaSuccess)
+            return err;
+        memo->B = B;
+    }
+    const CUtensorMap& tmap = memo->map;
 
     const int tile_rows = M_Global / kTileM;
     const int n_tiles   = (N_Global + pl.n_tile - 1) / pl.n_tile;
@@ -972,6 +1027,7 @@ void FlashLLM_SetPlan(const int* fields, int count)
     std::lock_guard<std::mutex> lock(g_override_mutex);
     for (int i = 0; i < kPlanFieldCount; ++i)
         g_override.v[i] = (fields != nullptr && i < count) ? fields[i] : 0;
+    g_override_version.fetch_add(1, std::memory_order_relaxed);
 }
 
 int FlashLLM_GetPlan(int M, int N, int K, int Split_K, int* out, int count)
