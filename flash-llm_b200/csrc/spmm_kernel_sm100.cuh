@@ -83,6 +83,38 @@ __device__ __forceinline__ half finish_output(float acc, const half* bias, int m
     return __float2half_rn(acc);
 }
 
+// C consecutive columns of output row m as finish_output finishes them; the first is element `at` of the output, and all
+// C or none of them lie inside it (`columns` left: N is 8 or a multiple of C wherever this is called).  Nothing is decided
+// per element: with a chain of branches on p's pointers for every element the 128 columns of one tile took 10 us of a
+// 13.0 us launch (128x64, N = 128), this way the launch takes 7.2 us.  Adding -0.0 leaves every value as it is.
+template<int C>
+__device__ __forceinline__ void finish_columns(const SpmmParams& p, float (&v)[C], size_t at, int columns, int m)
+{
+    if (columns < C)
+        return;
+    const float  bias = p.bias != nullptr ? __half2float(p.bias[m]) : -0.0f;
+    const bool   relu = p.activation == kActRelu;
+    const size_t step = static_cast<size_t>(p.M);
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        v[i] += bias;
+        v[i] = relu ? fmaxf(v[i], 0.0f) : v[i];
+    }
+    if (p.residual != nullptr) {
+        half res[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i)
+            res[i] = p.residual[at + i * step];
+#pragma unroll
+        for (int i = 0; i < C; ++i)
+            v[i] += __half2float(res[i]);
+    }
+    half* out = p.out + at;
+#pragma unroll
+    for (int i = 0; i < C; ++i, out += step)
+        *out = __float2half_rn(v[i]);
+}
+
 // Pipeline-analysis builds (never the shipped one) drop one stage of the kernel to see what it costs, as the
 // reference does with its own stubs (csrc/SpMM_Kernel.cuh:64-111).  Bits: 1 no zero-fill, 2 no scatter stores,
 // 8 no ring reads.  Results are wrong with any bit set.
@@ -300,65 +332,67 @@ __device__ __forceinline__ void load_b_batches(const CUtensorMap* tmap, int batc
 // accumulators that hold tiles (they lie `acc_stride` columns apart; 0 of them = an empty K range, output 0), then
 // stored as fp16 C, as an fp32 partial tile in the workspace, or parked in shared memory (`red`, [N_TILE][128] fp32
 // over the idle A stages) for the cluster sum.
-template<int N_TILE>
+template<int N_TILE, int BATCH = 8>
 __device__ __forceinline__ void accumulators_to_output(const SpmmParams& p, uint32_t tmem_acc, int accumulators, int acc_stride,
                                                        int quarter, int lane, int sw, int per_quarter, int S, int G, int g,
                                                        int n_idx, int tile_row, bool acc_ok, float* red)
 {
-    const int col_share   = (N_TILE / per_quarter) < 8 ? 8 : (N_TILE / per_quarter);
+    const int col_share   = (N_TILE / per_quarter) < BATCH ? BATCH : (N_TILE / per_quarter);
     const int col_begin   = sw < 4 * per_quarter ? (sw / 4) * col_share : N_TILE;
     const int col_end     = (col_begin + col_share) < N_TILE ? (col_begin + col_share) : N_TILE;
     const int n_valid     = (p.N - n_idx * N_TILE) < N_TILE ? (p.N - n_idx * N_TILE) : N_TILE;
     const int row_in_tile = quarter * 32 + lane;
     const size_t tile_off = static_cast<size_t>(n_idx) * N_TILE * p.M + static_cast<size_t>(tile_row) * kTileM;
-    half* const  out_tile  = p.out + tile_off;
     float* const part_tile = G > 1 ? p.partial + static_cast<size_t>(g) * p.M * p.N + tile_off : nullptr;
-    for (int c0 = col_begin; c0 < col_end; c0 += 8) {
-        float r[8];
+    const uint32_t acc     = tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16);
+    auto           load    = [&](uint32_t from, float (&v)[BATCH]) {
+        uint32_t t[BATCH / 8][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            r[i] = 0.0f;
-        if (accumulators == 2) {  // the two loads go out together and are waited for once
-            uint32_t t0[8], t1[8];
-            ptx::tmem_ld_x8(tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16) + c0, t0);
-            ptx::tmem_ld_x8(tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16) + acc_stride + c0, t1);
-            ptx::tmem_wait_ld();
+        for (int i = 0; i < BATCH / 8; ++i)
+            ptx::tmem_ld_x8(from + i * 8, t[i]);
+        ptx::tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                r[i] = __uint_as_float(t0[i]) + __uint_as_float(t1[i]);
+        for (int i = 0; i < BATCH; ++i)
+            v[i] = __uint_as_float(t[i / 8][i % 8]);
+    };
+    for (int c0 = col_begin; c0 < col_end; c0 += BATCH) {
+        float r[BATCH];
+        if (accumulators == 0) {
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i)
+                r[i] = 0.0f;
         }
-        else {
-            for (int a = 0; a < accumulators; ++a) {
-                uint32_t t[8];
-                ptx::tmem_ld_x8(tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16) + a * acc_stride + c0, t);
-                ptx::tmem_wait_ld();
+        else
+            load(acc + c0, r);
+        if (accumulators == 2) {
+            float more[BATCH];
+            load(acc + acc_stride + c0, more);
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    r[i] += __uint_as_float(t[i]);
-            }
+            for (int i = 0; i < BATCH; ++i)
+                r[i] += more[i];
         }
-        if (S == 1) {
-            if (acc_ok) {
+        if (S > 1) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (c0 + i < n_valid) {
-                        const size_t at = static_cast<size_t>(c0 + i) * p.M + row_in_tile;
-                        if (part_tile)
-                            part_tile[at] = r[i];
-                        else if (p.push_world > 0) {
-                            for (int w = 0; w < p.push_world; ++w)
-                                p.push_slot[w][tile_off + at] = r[i];
-                        }
-                        else
-                            out_tile[at] = finish_output(r[i], p.bias, tile_row * kTileM + row_in_tile, p.activation, p.residual,
-                                                         tile_off + at);
-                    }
-            }
-        }
-        else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < BATCH; ++i)
                 red[(c0 + i) * kTileM + row_in_tile] = r[i];
+        }
+        else if (acc_ok) {
+            const size_t at = static_cast<size_t>(c0) * p.M + row_in_tile;
+            if (part_tile != nullptr) {
+#pragma unroll
+                for (int i = 0; i < BATCH; ++i)
+                    if (c0 + i < n_valid)
+                        part_tile[at + static_cast<size_t>(i) * p.M] = r[i];
+            }
+            else if (p.push_world > 0) {
+                for (int w = 0; w < p.push_world; ++w)
+#pragma unroll
+                    for (int i = 0; i < BATCH; ++i)
+                        if (c0 + i < n_valid)
+                            p.push_slot[w][tile_off + at + static_cast<size_t>(i) * p.M] = r[i];
+            }
+            else
+                finish_columns<BATCH>(p, r, tile_off + at, n_valid - c0, tile_row * kTileM + row_in_tile);
         }
     }
     if (S == 1 && part_tile != nullptr && p.tile_counters != nullptr)

@@ -404,30 +404,28 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
             float* const park = whole ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (seg == 0 ? 0 : 1)) + r;
             if (ok) {
 #pragma unroll 1
-                for (int c0 = 0; c0 < N_TILE; c0 += 16) {
-                    uint32_t t0[8], t1[8];
-                    ptx::tmem_ld_x8(acc + c0, t0);
-                    ptx::tmem_ld_x8(acc + c0 + 8, t1);
+                for (int c0 = 0; c0 < N_TILE; c0 += 8) {
+                    uint32_t t[8];
+                    ptx::tmem_ld_x8(acc + c0, t);
                     ptx::tmem_wait_ld();
-                    if (c0 + 16 == N_TILE) {  // the accumulator has been read: the issuer may start a segment in it
+                    if (c0 + 8 == N_TILE) {  // the accumulator has been read: the issuer may start a segment in it
                         ptx::tc_fence_before_sync();
                         __syncwarp();
                         if (lane == 0)
                             ptx::mbar_arrive(acc_empty + 8u * (seg & 1));
                     }
+                    float v[8];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int   n = c0 + i;
-                        const float v = __uint_as_float(i < 8 ? t0[i & 7] : t1[i & 7]);
-                        if (n < p.N) {
-                            if (park != nullptr)
-                                __stcg(park + n * kTileM, v);
-                            else {
-                                const size_t at = static_cast<size_t>(n) * p.M + row * kTileM + r;
-                                p.out[at]       = finish_output(v, p.bias, row * kTileM + r, p.activation, p.residual, at);
-                            }
-                        }
+                    for (int i = 0; i < 8; ++i)
+                        v[i] = __uint_as_float(t[i]);
+                    if (park != nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (c0 + i < p.N)
+                                __stcg(park + (c0 + i) * kTileM, v[i]);
                     }
+                    else
+                        finish_columns<8>(p, v, static_cast<size_t>(c0) * p.M + row * kTileM + r, p.N - c0, row * kTileM + r);
                 }
             }
             if (!whole) {
