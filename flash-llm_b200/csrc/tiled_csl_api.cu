@@ -75,7 +75,7 @@ int FlashLLM_EncodeOnDevice_TileOffsets(void* stream, const void* A_d, int M, in
         return rc;
     const int    k_tiles = K / kTileK, tiles = (M / kTileM) * k_tiles;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaError_t  e = launch_in_stream_order(csl_count_kernel, dim3((tiles + kEncodeWarps - 1) / kEncodeWarps), dim3(kEncodeWarps * 32),
+    cudaError_t  e = launch_in_stream_order(csl_count_kernel, dim3((tiles + kCountTiles - 1) / kCountTiles), dim3(kEncodeWarps * 32),
                                            0, s, 1, static_cast<const uint16_t*>(A_d), K, tiles, k_tiles, TileOffsets_d);
     if (e == cudaSuccess)
         e = launch_in_stream_order(csl_scan_kernel, dim3(1), dim3(1024), 0, s, 1, TileOffsets_d, tiles, status);
@@ -92,11 +92,25 @@ int FlashLLM_EncodeOnDevice_Pack(void* stream, const void* A_d, int M, int K, co
     if (int rc = device_status_pointer(&status))
         return rc;
     const int    k_tiles = K / kTileK, tiles = (M / kTileM) * k_tiles;
-    const int    blocks  = (tiles + kEncodeWarps - 1) / kEncodeWarps;
     cudaStream_t s       = static_cast<cudaStream_t>(stream);
-    return static_cast<int>(launch_in_stream_order(reorder ? csl_pack_reorder_kernel : csl_pack_scan_kernel, dim3(blocks),
-                                                   dim3(kEncodeWarps * 32), 0, s, 1, static_cast<const uint16_t*>(A_d), K, tiles,
-                                                   k_tiles, TileOffsets_d, Compressed_A_d, status));
+    const auto   launch  = [&](auto kernel, int blocks, int warps) {
+        return static_cast<int>(launch_in_stream_order(kernel, dim3(blocks), dim3(warps * 32), 0, s, 1,
+                                                       static_cast<const uint16_t*>(A_d), K, tiles, k_tiles, TileOffsets_d,
+                                                       Compressed_A_d, status));
+    };
+    if (!reorder)
+        return launch(csl_pack_scan_kernel, (tiles + kEncodeWarps - 1) / kEncodeWarps, kEncodeWarps);
+    // A persistent grid; L1 keeps what kPackCtasPerSm CTAs' shared memory leaves of 228 KB (it holds the loads in flight).
+    int         device = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(csl_pack_reorder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kPackCarveoutPercent);
+    if (e != cudaSuccess)
+        return static_cast<int>(e);
+    const int blocks = (tiles + kPackWarps - 1) / kPackWarps;
+    return launch(csl_pack_reorder_kernel, blocks < kPackCtasPerSm * sms ? blocks : kPackCtasPerSm * sms, kPackWarps);
 }
 
 void FlashLLM_Free(void* p)

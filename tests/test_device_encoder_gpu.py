@@ -64,3 +64,50 @@ def test_device_encoded_buffers_feed_the_kernel(lib, oracle):
     torch.cuda.synchronize()
     assert lib.consume_status() == 0
     assert_close(C.cpu().numpy(), oracle.gemm_f32(A.numpy(), B.numpy()), "device-encoded SpMM")
+
+
+@pytest.mark.parametrize("shift", [0, 2])
+def test_tiles_of_every_density_and_special_values(lib, shift):
+    """Buckets from empty to all 256 cells, around the height a warp's lists hold (136 words), with zeros, NaN, infinities
+    and subnormals among them; groups of 32 tiles that end in the middle of a row; A only 4-byte aligned."""
+    M, K = 128 * 5, 64 * 27
+    rng = np.random.default_rng(5)
+    A = rng.uniform(-1, 1, (M, K)).astype(np.float16)
+    density = rng.choice([0.0, 0.05, 0.2, 0.4, 0.5, 0.53, 0.6, 0.9, 1.0], size=(M // 128, K // 64))
+    A[rng.random((M, K)) >= np.kron(density, np.ones((128, 64)))] = 0
+    bits = A.view(np.uint16)
+    special = rng.random((M, K))
+    for i, b in enumerate((0x8000, 0x7C00, 0xFC00, 0x7E00, 0xFFFF, 0x0001, 0x83FF)):
+        bits[(special > i * 0.004) & (special <= (i + 1) * 0.004)] = b
+    comp_h, offs_h, _ = lib.InitSparseMatrixA_API(A)
+    flat = torch.zeros(M * K + 8, dtype=torch.float16, device="cuda")
+    A_d = flat[shift:shift + M * K]
+    A_d.copy_(torch.from_numpy(A).view(-1))
+    assert (A_d.data_ptr() % 16 == 0) == (shift == 0)
+    T = offs_h.size - 2
+    offs = torch.full((T + 2,), -7, dtype=torch.int32, device="cuda")
+    comp = torch.full((comp_h.size + 4,), -1, dtype=torch.int32, device="cuda")
+    L, stream = lib.library(), torch.cuda.current_stream().cuda_stream
+    assert L.FlashLLM_EncodeOnDevice_TileOffsets(stream, A_d.data_ptr(), M, K, offs.data_ptr()) == 0
+    for start in (0, 1):  # words to a 16-byte aligned place, and to a 4-byte aligned one
+        comp.fill_(-1)
+        assert L.FlashLLM_EncodeOnDevice_Pack(stream, A_d.data_ptr(), M, K, offs.data_ptr(), comp.data_ptr() + 4 * start, 1) == 0
+        torch.cuda.synchronize()
+        assert lib.consume_status() == 0
+        assert np.array_equal(offs.cpu().numpy(), offs_h)
+        got = comp.cpu().numpy().view(np.uint32)
+        assert np.array_equal(got[start:start + comp_h.size], comp_h)
+        assert (got[:start] == 0xFFFFFFFF).all() and (got[start + comp_h.size:] == 0xFFFFFFFF).all()
+
+
+@pytest.mark.parametrize("tiles", [31, 33, 32 * 1024, 32 * 1024 + 1])
+def test_offsets_over_many_groups(lib, tiles):
+    """The offsets' two levels at the edges of a group (32 tiles) and of a round (1024 groups), against a plain cumulative sum."""
+    A = torch.zeros((128, 64 * tiles), dtype=torch.float16, device="cuda")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(tiles)
+    A[:3] = (torch.rand((3, 64 * tiles), generator=gen, device="cuda") < 0.3).half()
+    vectors = ((A[:3] != 0).view(3, tiles, 64).sum((0, 2)) + 3) // 4
+    _, offs = torch.ops.flashllm.encode(A)
+    want = torch.cat([torch.zeros(1, dtype=torch.int64, device="cuda"), vectors.cumsum(0), vectors.sum().view(1)])
+    assert torch.equal(offs.long(), want)
