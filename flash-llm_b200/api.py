@@ -366,7 +366,7 @@ def release_scratch() -> None:
 
 PLAN_FIELDS = ("cluster_k", "workspace_k", "a_stages", "b_stages", "b_batch", "ring_slots", "chunk_vectors",
                "scatter_warps", "producers", "path", "reduce")
-PATH_RING, PATH_DIRECT, PATH_STREAM = 1, 2, 3
+PATH_RING, PATH_DIRECT, PATH_STREAM, PATH_WIDE = 1, 2, 3, 4
 REDUCE_SECOND_KERNEL, REDUCE_LAST_CTA = 1, 2
 
 

@@ -15,6 +15,7 @@
 #include "spmm_kernel_direct_sm100.cuh"
 #include "spmm_kernel_sm100.cuh"
 #include "spmm_kernel_stream_sm100.cuh"
+#include "spmm_kernel_wide_sm100.cuh"
 #include "tiled_csl_host.h"
 #include "tiling.h"
 
@@ -207,6 +208,12 @@ static DeviceState* device_state(cudaError_t* err)
         e = raise_smem_limit<64>(st->smem_optin);
     if (e == cudaSuccess)
         e = raise_smem_limit<128>(st->smem_optin);
+    if (e == cudaSuccess)
+        e = raise_smem_limit_of(spmm_tcgen05_wide_kernel<256, kWideCap>, st->smem_optin);
+    if (e == cudaSuccess)
+        e = raise_smem_limit_of(spmm_tcgen05_wide_kernel<384, kWideCap>, st->smem_optin);
+    if (e == cudaSuccess)
+        e = raise_smem_limit_of(spmm_tcgen05_wide_kernel<512, kWideCap>, st->smem_optin);
     st->ready = (e == cudaSuccess);
     *err      = e;
     return st->ready ? st : nullptr;
@@ -316,6 +323,67 @@ static double stream_cost(const SpmmPlan& pl, int tile_rows, int k_tiles)
     return 0.93 * tiles + 15.0 + (pl.n_tile - 16) * 0.15 + 0.45 * parts * (0.5 + pl.n_tile / 32.0);
 }
 
+// Clusters of S CTAs resident at a time on 148 SMs (measured), two CTAs or one per SM.
+constexpr int kClustersResident2[kMaxClusterK + 1] = {0, 296, 148, 92, 71, 56, 45, 37, 33};
+constexpr int kClustersResident1[kMaxClusterK + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+
+// N >= 256: output columns per CTA, cluster parts S and workspace parts G by the cheapest estimate, in SM cycles; what the
+// caller pinned is kept.  A CTA of the wide form takes kTileCycles per tile (by hundreds of columns; 128 columns are the
+// register-streaming form, whose own choice follows when that is the cheapest: then cudaErrorInvalidConfiguration), 8000 to
+// 14000 around them, 2000 per 128 columns more for a cluster sum; a second kernel costs 5000 and its bytes.  From 36864x9216
+// (288 rows), 9216x9216 and 4736x7232 at N = 256, 384, 512 with every width and S: the choice is the fastest or within 4 %.
+static cudaError_t make_wide_plan(const DeviceState* st, SpmmPlan pl, const PlanOverride& ov, int tile_rows, int k_tiles, int N,
+                                  int max_extra, SpmmPlan* out)
+{
+    static const int kTileCycles[5] = {0, 600, 780, 1080, 1300};
+    double           best = 0.0;
+    int              width = 0;  // in 128 columns
+    for (int w = 1; w <= 4 && (w - 1) * 128 < N; ++w) {
+        if (ov.v[kPlanProducers] && ov.v[kPlanProducers] != w)
+            continue;
+        const int n_tiles = (N + w * 128 - 1) / (w * 128);
+        for (int s = 1; s <= kMaxClusterK && s <= k_tiles; ++s) {
+            // the cluster sum parks fp32 [columns][128] over the pipeline buffers
+            if ((w == 4 && s > 1) || (ov.v[kPlanClusterK] && ov.v[kPlanClusterK] != s))
+                continue;
+            const int capacity = kClustersResident1[s] * st->sm_count / 148;
+            for (int g = 1; g <= max_extra && g <= 32 && s * g <= k_tiles; ++g) {
+                if (ov.v[kPlanWorkspaceK] && ov.v[kPlanWorkspaceK] != g)
+                    continue;
+                const long long clusters = static_cast<long long>(tile_rows) * n_tiles * g;
+                const double    waves    = static_cast<double>((clusters + capacity - 1) / (capacity < 1 ? 1 : capacity));
+                const double    per_cta  = static_cast<double>((k_tiles + s * g - 1) / (s * g)) * kTileCycles[w] + 6000.0 + w * 2000.0
+                                       + (s > 1 ? w * 2000.0 : 0.0);
+                const double cost = waves * per_cta + (g > 1 ? 5000.0 + 0.03 * g * tile_rows * N : 0.0);
+                if (width == 0 || cost < best) {
+                    width          = w;
+                    best           = cost;
+                    pl.cluster_k   = s;
+                    pl.workspace_k = g;
+                }
+            }
+        }
+    }
+    if (width < 2)
+        return cudaErrorInvalidConfiguration;
+    pl.path          = kPathWide;
+    pl.reduce        = kReduceSecondKernel;
+    pl.n_tile        = width * 128;
+    pl.producers     = width;
+    pl.a_stages      = wide_a_stages(pl.n_tile);
+    pl.scatter_warps = pl.a_stages;
+    pl.b_stages      = wide_b_stages(pl.n_tile);
+    pl.b_batch       = 1;
+    const int buffers = pl.a_stages * kDenseTileBytes + pl.b_stages * wide_mma_n(pl.n_tile) * kTileK * 2;
+    const int bars    = 8 * (2 * pl.a_stages + 2 * pl.b_stages + 1) + 16;
+    const int longest = (k_tiles + pl.cluster_k * pl.workspace_k - 1) / (pl.cluster_k * pl.workspace_k) + 1;
+    const int staged  = ((longest + 1 + 3) / 4) * 4;
+    pl.offsets_staged = buffers + bars + 4 * staged <= st->smem_optin ? staged : 0;
+    pl.smem_bytes     = buffers + bars + 4 * pl.offsets_staged;
+    *out              = pl;
+    return cudaSuccess;
+}
+
 // Chooses how to cut K and how deep to pipeline.  Takes the place of the reference's per-N switch over
 // TilingConfig instances (csrc/SpMM_API.cu:79-118) and of its hand-tuned Split_K tables
 // (kernel_benchmark/benchmark.sh:13-15).
@@ -348,6 +416,13 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
         pinned |= v != 0;
     if (pl.path == kPathStream)  // pinned: other fields do not apply to it
         return may_stream && !sends ? make_stream_plan(st, pl, tile_rows, k_tiles, out) : cudaErrorInvalidConfiguration;
+    if (pl.path == kPathWide || (N >= 256 && !pinned && !sends)) {
+        if (N < 256 || N % 128 != 0 || sends)
+            return cudaErrorInvalidConfiguration;
+        const cudaError_t e = make_wide_plan(st, pl, ov, tile_rows, k_tiles, N, max_parts > 1 ? max_parts : 1, out);
+        if (e == cudaSuccess || pl.path == kPathWide)
+            return e;
+    }
     const bool direct     = pl.path == kPathDirect;
     pl.scatter_warps      = ov.v[kPlanScatterWarps] ? ov.v[kPlanScatterWarps]
                                                     : (direct ? (pl.n_tile <= 64 ? 4 : 8) : (pl.n_tile <= 32 ? 4 : 8));
@@ -380,8 +455,6 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // the sum by the last CTA 2 + 0.1 per part (8 + 0.1 per part in a fused all-reduce, where the peers wait for that
     // CTA: measured on 2 GPUs, 9216x1152 ... 9216x18432), a second kernel half a tile per part.  The cheapest (S, G) wins,
     // fewer parts on a tie.  Replaces the reference's hand-tuned Split_K tables (kernel_benchmark/benchmark.sh:13-15).
-    static const int kClustersResident2[kMaxClusterK + 1] = {0, 296, 148, 92, 71, 56, 45, 37, 33};  // two CTAs per SM
-    static const int kClustersResident1[kMaxClusterK + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};   // one CTA per SM
     const bool two_resident = two_per_sm && ((direct && pl.producers == 1) ? kDirectBlocks : 2) == 2;
     const int* resident     = two_resident ? kClustersResident2 : kClustersResident1;
     auto capacity = [&](int S_) {  // the table is for 148 SMs
@@ -465,13 +538,14 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     return cudaSuccess;
 }
 
-// B as a 3-D tensor {64 K-elements (inner), N, K/64}: one box = b_batch K tiles of [n_tile x 64], each stored as a
+// B as a 3-D tensor {64 K-elements (inner), N, K/64}: one box = b_batch K tiles of [n_tile x 64] (wide form: of one MMA's columns), each stored as a
 // 128-byte-swizzled slab; rows past N and K tiles past K/64 read as 0.
 static cudaError_t encode_b_map(const half* B, int N, int K, const SpmmPlan& pl, CUtensorMap* map)
 {
     const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(kTileK), static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(K / kTileK)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K) * 2, static_cast<cuuint64_t>(kTileK) * 2};
-    const cuuint32_t box[3]     = {static_cast<cuuint32_t>(kTileK), static_cast<cuuint32_t>(pl.n_tile),
+    const int        columns    = pl.path == kPathWide ? wide_mma_n(pl.n_tile) : pl.n_tile;
+    const cuuint32_t box[3]     = {static_cast<cuuint32_t>(kTileK), static_cast<cuuint32_t>(columns),
                                    static_cast<cuuint32_t>(pl.b_batch)};
     const cuuint32_t estr[3]    = {1, 1, 1};
     const CUresult   r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<half*>(B), dims, strides, box, estr,
@@ -544,6 +618,17 @@ static cudaError_t launch_spmm(cudaStream_t stream, const CUtensorMap& tmap, con
         return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks>, warps);
     }
     return launch(spmm_tcgen05_kernel<N_TILE>, pl.producers + 2 + pl.scatter_warps);
+}
+
+template<int N_TILE>
+static cudaError_t launch_wide(cudaStream_t stream, const CUtensorMap& tmap, const SpmmParams& params, int tile_rows,
+                               int n_tiles)
+{
+    const SpmmPlan& pl = params.plan;
+    return launch_in_stream_order(spmm_tcgen05_wide_kernel<N_TILE, kWideCap>,
+                                  dim3(pl.cluster_k, tile_rows, n_tiles * pl.workspace_k),
+                                  dim3((kWideFirstScatter + wide_a_stages(N_TILE)) * 32), pl.smem_bytes, stream, pl.cluster_k, tmap,
+                                  params);
 }
 
 static cudaError_t reduce_partials(cudaStream_t stream, half* C, const float* ws, long long count, int parts,
@@ -739,6 +824,9 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
             case 16: err = launch_spmm<16>(stream, tmap, params, tile_rows, n_tiles); break;
             case 32: err = launch_spmm<32>(stream, tmap, params, tile_rows, n_tiles); break;
             case 64: err = launch_spmm<64>(stream, tmap, params, tile_rows, n_tiles); break;
+            case 256: err = launch_wide<256>(stream, tmap, params, tile_rows, n_tiles); break;
+            case 384: err = launch_wide<384>(stream, tmap, params, tile_rows, n_tiles); break;
+            case 512: err = launch_wide<512>(stream, tmap, params, tile_rows, n_tiles); break;
             default: err = launch_spmm<128>(stream, tmap, params, tile_rows, n_tiles); break;
         }
         if (err != cudaSuccess)

@@ -74,6 +74,89 @@ wait_bounded_converged(uint32_t bar, uint32_t parity, volatile uint32_t* abort_f
     return ok;
 }
 
+// A scatter warp's tiles sw, sw + STAGES, ... of a CTA's L tiles: the words of the next one wait in registers (up to CAP
+// 16-byte vectors per lane) while the warp's stage is still being multiplied.
+template<int CAP, int STAGES>
+struct TileStream {
+    uint4        nxt[CAP];
+    int          n_in;  // vectors of the tile in nxt
+    const uint4* src;
+    bool         bad;
+
+    __device__ __forceinline__ void clear()
+    {
+        n_in = 0;
+        src  = nullptr;
+        bad  = false;
+#pragma unroll
+        for (int q = 0; q < CAP; ++q)
+            nxt[q] = make_uint4(0u, 0u, 0u, 0u);
+    }
+
+    __device__ __forceinline__ void fetch(const SpmmParams& p, int vb, int ve, int lane)
+    {
+        bad  = (ve < vb) || (ve - vb > kMaxTileVectors) || (vb < 0);
+        n_in = bad ? 0 : ve - vb;
+        src  = p.compressed + (bad ? 0 : vb);
+        load_batch<1, CAP>(nxt, src + lane, n_in, n_in - lane);
+    }
+
+    // The first tile, by offsets straight from global memory, before the CTA's set-up.
+    __device__ __forceinline__ void fetch_first(const SpmmParams& p, const int* offs_global, int sw, int L, int lane)
+    {
+        if (sw < L)
+            fetch(p, offs_global[sw], offs_global[sw + 1], lane);
+    }
+
+    __device__ __forceinline__ void run(const SpmmParams& p, const int* offs, int sw, int L, int lane, uint32_t stage,
+                                        uint32_t full_bar, uint32_t empty_bar, volatile uint32_t* abort_flag)
+    {
+        if (lane == 0) {
+            for (int a = 1; a < kPrefetchAhead; ++a) {
+                const int t = sw + a * STAGES;
+                if (t < L && offs[t + 1] > offs[t])
+                    ptx::prefetch_l2_bulk(p.compressed + offs[t], static_cast<uint32_t>(offs[t + 1] - offs[t]) * 16u);
+            }
+        }
+        uint32_t use = 0;
+        for (int j = sw; j < L; j += STAGES, ++use) {
+            bool ok = !bad;
+            if (use > 0)
+                ok = wait_bounded_converged(empty_bar, (use & 1u) ^ 1u, abort_flag, p.status) && ok;
+            if (!__all_sync(0xFFFFFFFFu, ok))
+                break;
+            // offsets of this warp's following tile: read here, where the load/store unit is idle (see the
+            // register-streaming form)
+            const bool has_next = j + STAGES < L;
+            int        vb2 = 0, ve2 = 0;
+            if (has_next) {
+                vb2 = offs[j + STAGES];
+                ve2 = offs[j + STAGES + 1];
+            }
+            zero_fill_stage(stage, lane);
+            __syncwarp();  // another lane's zero must not land on top of a new value
+            const int rem = n_in - lane;
+            scatter_batch<1, CAP>(stage, nxt, n_in, rem);
+            for (int v0 = CAP * 32; v0 < n_in; v0 += CAP * 32) {  // tiles denser than the register budget
+                load_batch<1, CAP>(nxt, src + v0 + lane, n_in - v0, rem - v0);
+                scatter_batch<1, CAP>(stage, nxt, n_in - v0, rem - v0);
+            }
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0)
+                ptx::mbar_arrive(full_bar);
+            if (has_next) {  // start fetching the following tile, and pull the one after it into L2
+                fetch(p, vb2, ve2, lane);
+                if (lane == 0 && j + kPrefetchAhead * STAGES < L) {
+                    const int pb = offs[j + kPrefetchAhead * STAGES], pe = offs[j + kPrefetchAhead * STAGES + 1];
+                    if (pe > pb)
+                        ptx::prefetch_l2_bulk(p.compressed + pb, static_cast<uint32_t>(pe - pb) * 16u);
+                }
+            }
+        }
+    }
+};
+
 // Adds the parked parts of tile row `row` up in CTA order and finishes the output (the 128 epilogue threads).
 template<int N_TILE>
 __device__ __forceinline__ void
@@ -186,27 +269,13 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
     }
 
     // ---- scatter warps request their first tile before anything else (see the register-streaming form)
-    const bool   scatters = warp >= kStreamFirstScatter && warp < kStreamFirstEpi;
-    const int    sw       = warp - kStreamFirstScatter;  // the stage, and the tile stream sw, sw + kStreamStages, ...
-    uint4        nxt[CAP];
-    int          n_in = 0;
-    const uint4* src  = p.compressed;
-    bool         bad  = false;
-    auto fetch_first_tile = [&]() {
-        if (sw < L) {
-            const int vb = offs_global[sw], ve = offs_global[sw + 1];
-            bad          = (ve < vb) || (ve - vb > kMaxTileVectors) || (vb < 0);
-            n_in         = bad ? 0 : ve - vb;
-            src          = p.compressed + (bad ? 0 : vb);
-            load_batch<1, CAP>(nxt, src + lane, n_in, n_in - lane);
-        }
-    };
+    const bool scatters = warp >= kStreamFirstScatter && warp < kStreamFirstEpi;
+    const int  sw       = warp - kStreamFirstScatter;  // the stage, and the tile stream sw, sw + kStreamStages, ...
+    TileStream<CAP, kStreamStages> stream;
     if (scatters) {
-#pragma unroll
-        for (int q = 0; q < CAP; ++q)
-            nxt[q] = make_uint4(0u, 0u, 0u, 0u);
+        stream.clear();
         if (p.early_weights)
-            fetch_first_tile();
+            stream.fetch_first(p, offs_global, sw, L, lane);
     }
 
     // ---- set-up
@@ -235,7 +304,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
     if (!p.early_weights) {
         ptx::grid_dependency_wait();
         if (scatters)
-            fetch_first_tile();
+            stream.fetch_first(p, offs_global, sw, L, lane);
     }
     if (staged) {
         for (int i = threadIdx.x; i <= L; i += blockDim.x)
@@ -336,57 +405,8 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
     }
     else if (warp < kStreamFirstEpi) {
         // ================================================================ scatter warps: one whole tile at a time
-        if (go) {
-            const uint32_t stage     = a_base + sw * kDenseTileBytes;
-            const uint32_t full_bar  = a_full + 8u * sw;
-            const uint32_t empty_bar = a_empty + 8u * sw;
-            if (lane == 0) {
-                for (int a = 1; a < kPrefetchAhead; ++a) {
-                    const int t = sw + a * kStreamStages;
-                    if (t < L && offs[t + 1] > offs[t])
-                        ptx::prefetch_l2_bulk(p.compressed + offs[t], static_cast<uint32_t>(offs[t + 1] - offs[t]) * 16u);
-                }
-            }
-            uint32_t use = 0;
-            for (int j = sw; j < L; j += kStreamStages, ++use) {
-                bool ok = !bad;
-                if (use > 0)
-                    ok = wait_bounded_converged(empty_bar, (use & 1u) ^ 1u, abort_flag, p.status) && ok;
-                if (!__all_sync(0xFFFFFFFFu, ok))
-                    break;
-                // offsets of this warp's following tile: read here, where the load/store unit is idle (see the
-                // register-streaming form)
-                const bool has_next = j + kStreamStages < L;
-                int        vb2 = 0, ve2 = 0;
-                if (has_next) {
-                    vb2 = offs[j + kStreamStages];
-                    ve2 = offs[j + kStreamStages + 1];
-                }
-                zero_fill_stage(stage, lane);
-                __syncwarp();  // another lane's zero must not land on top of a new value
-                const int rem = n_in - lane;
-                scatter_batch<1, CAP>(stage, nxt, n_in, rem);
-                for (int v0 = CAP * 32; v0 < n_in; v0 += CAP * 32) {  // tiles denser than the register budget
-                    load_batch<1, CAP>(nxt, src + v0 + lane, n_in - v0, rem - v0);
-                    scatter_batch<1, CAP>(stage, nxt, n_in - v0, rem - v0);
-                }
-                ptx::fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0)
-                    ptx::mbar_arrive(full_bar);
-                if (has_next) {  // start fetching the following tile, and pull the one after it into L2
-                    bad  = (ve2 < vb2) || (ve2 - vb2 > kMaxTileVectors) || (vb2 < 0);
-                    n_in = bad ? 0 : ve2 - vb2;
-                    src  = p.compressed + (bad ? 0 : vb2);
-                    load_batch<1, CAP>(nxt, src + lane, n_in, n_in - lane);
-                    if (lane == 0 && j + kPrefetchAhead * kStreamStages < L) {
-                        const int pb = offs[j + kPrefetchAhead * kStreamStages], pe = offs[j + kPrefetchAhead * kStreamStages + 1];
-                        if (pe > pb)
-                            ptx::prefetch_l2_bulk(p.compressed + pb, static_cast<uint32_t>(pe - pb) * 16u);
-                    }
-                }
-            }
-        }
+        if (go)
+            stream.run(p, offs, sw, L, lane, a_base + sw * kDenseTileBytes, a_full + 8u * sw, a_empty + 8u * sw, abort_flag);
     }
     else {
         // ================================================================ epilogue warps

@@ -50,11 +50,12 @@ constexpr int kReduceLastCta      = 2;  // inside the SpMM kernel, by the last C
 constexpr int kPathRing   = 1;  // bulk copies into a shared-memory ring (spmm_tcgen05_kernel)
 constexpr int kPathDirect = 2;  // global loads into the scatter warps' registers (spmm_tcgen05_direct_kernel)
 constexpr int kPathStream = 3;  // the same, as a persistent grid over the linear tile sequence (spmm_tcgen05_stream_kernel)
+constexpr int kPathWide   = 4;  // one CTA per tile row and 256..512 output columns (spmm_tcgen05_wide_kernel)
 
 struct SpmmPlan {
-    int path;    // kPathRing, kPathDirect or kPathStream
+    int path;    // kPathRing, kPathDirect, kPathStream or kPathWide
     int ctas;    // kPathStream: CTAs of the persistent grid
-    int n_tile;  // MMA N: 16, 32, 64 or 128
+    int n_tile;  // output columns of a CTA: 16, 32, 64 or 128; kPathWide: 256, 384 or 512
     int cluster_k;
     int workspace_k;
     int a_stages;

@@ -315,7 +315,9 @@ int FlashLLM_ReleaseScratch(void);
  *                     2 = register-streaming form (the default): scatter warps load their tiles' words from global
  *                     memory into registers, tiles alternate between two MMA-issuing threads;
  *                     3 = streaming form: the same work dealt out as one linear sequence of tiles over a persistent grid
- *                     (N <= 64; chosen where one CTA per tile row would leave SMs idle; the other fields do not apply)
+ *                     (N <= 64; chosen where one CTA per tile row would leave SMs idle; the other fields do not apply);
+ *                     4 = wide form (N >= 256: a CTA multiplies a tile by 256, 384 or 512 output columns; `producers` = 2,
+ *                     3 or 4 pins the width in 128 columns, cluster_k and workspace_k apply, 512 columns take cluster_k 1)
  *  10 reduce          who adds the workspace parts up: 1 = a second kernel (the default; with launch overlap it
  *                     hides behind the neighbouring SpMMs); 2 = the SpMM kernel itself: every CTA parks its fp32
  *                     partial tile and counts itself in on a counter of the output tile, the CTA that completes the
