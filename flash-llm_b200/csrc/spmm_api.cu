@@ -92,11 +92,18 @@ static unsigned char* scratch_of_stream(DeviceState* st, cudaStream_t stream)
             return st->scratch[i].memory;
     if (st->scratch_streams >= kScratchStreams)
         return nullptr;
-    unsigned char* memory = nullptr;
-    if (cudaMalloc(reinterpret_cast<void**>(&memory), kScratchBytes) != cudaSuccess
-        || cudaMemset(memory, 0, kScratchRows * sizeof(unsigned int)) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
-        cudaGetLastError();
+    // Another thread may be capturing: allocate in relaxed mode, and clear the counters in this stream's own order.
+    unsigned char*        memory = nullptr;
+    cudaStreamCaptureMode mode   = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    bool ok = cudaMalloc(reinterpret_cast<void**>(&memory), kScratchBytes) == cudaSuccess;
+    if (ok && cudaMemsetAsync(memory, 0, kScratchRows * sizeof(unsigned int), stream) != cudaSuccess) {
         cudaFree(memory);
+        ok = false;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) {
+        cudaGetLastError();
         return nullptr;
     }
     st->scratch[st->scratch_streams++] = {id, memory};
@@ -121,7 +128,9 @@ static DeviceState g_devices[kMaxDevices];
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn  g_encode_tiled = nullptr;
+using ReplaceAddressFn = CUresult (*)(CUtensorMap*, void*);
+static EncodeTiledFn    g_encode_tiled    = nullptr;
+static ReplaceAddressFn g_replace_address = nullptr;
 static std::once_flag g_encode_once;
 
 // Register budget of the register-streaming kernel: vectors per lane kept in registers (tiles of up to 768 vectors,
@@ -237,8 +246,11 @@ static cudaError_t load_encode_tiled()
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) == cudaSuccess
             && qres == cudaDriverEntryPointSuccess)
             g_encode_tiled = reinterpret_cast<EncodeTiledFn>(fn);
+        if (cudaGetDriverEntryPoint("cuTensorMapReplaceAddress", &fn, cudaEnableDefault, &qres) == cudaSuccess
+            && qres == cudaDriverEntryPointSuccess)
+            g_replace_address = reinterpret_cast<ReplaceAddressFn>(fn);
     });
-    return g_encode_tiled ? cudaSuccess : cudaErrorNotSupported;
+    return g_encode_tiled && g_replace_address ? cudaSuccess : cudaErrorNotSupported;
 }
 
 // ---------------------------------------------------------------- launch plan
@@ -554,8 +566,8 @@ static cudaError_t encode_b_map(const half* B, int N, int K, const SpmmPlan& pl,
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// What a call derives from its sizes and B's address alone, kept per thread: a decode loop repeats a few dozen calls, and
-// the search over K cuts and the tensor map's encoding are 2 us of each, a third of a small call.
+// What a call derives from its sizes alone, kept per thread: a decode loop repeats a few dozen calls, and the search over
+// K cuts and the tensor map's encoding are 2 us of each, a third of a small call.  The map's address is set on every call.
 struct CallKey {
     const DeviceState* device;
     int                M, N, K, max_parts;
@@ -570,7 +582,7 @@ struct CallKey {
 struct CallMemo {
     CallKey     key{};
     SpmmPlan    plan{};
-    const half* B = nullptr;  // what `map` was encoded for
+    bool        has_map = false;
     CUtensorMap map{};
 };
 
@@ -586,9 +598,9 @@ static cudaError_t plan_call(const CallKey& key, CallMemo** out)
         const cudaError_t err = make_plan(key.device, key.M, key.N, key.K, key.max_parts, &plan, key.sends, key.may_stream);
         if (err != cudaSuccess)
             return err;
-        m.key  = key;
-        m.plan = plan;
-        m.B    = nullptr;
+        m.key     = key;
+        m.plan    = plan;
+        m.has_map = false;
     }
     *out = &m;
     return cudaSuccess;
@@ -779,11 +791,14 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
     params.K            = K_Global;
     params.k_tiles      = K_Global / kTileK;
 
-    if (memo->B != B) {
-        memo->B = nullptr;
+    if (memo->has_map) {
+        if (g_replace_address(&memo->map, const_cast<half*>(B)) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    else {
         if ((err = encode_b_map(B, N_Global, K_Global, pl, &memo->map)) != cudaSuccess)
             return err;
-        memo->B = B;
+        memo->has_map = true;
     }
     const CUtensorMap& tmap = memo->map;
 

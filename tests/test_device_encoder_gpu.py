@@ -3,6 +3,8 @@ import numpy as np
 import pytest
 import torch
 
+from flash_llm_b200 import torch_op  # noqa: F401  (registers torch.ops.flashllm)
+
 pytestmark = pytest.mark.gpu
 
 

@@ -18,13 +18,13 @@ def pinned(lib):
 
 @pytest.mark.parametrize("width", [2, 3, 4])
 @pytest.mark.parametrize("M,K,N,sparsity", [
-    (128, 64, 256, 0.8),         # one tile; at widths 384 and 512 columns beyond N
-    (384, 64 * 5, 384, 0.9),     # fewer K tiles than stages
-    (256, 64 * 9, 512, 0.8),     # one K tile more than eight stages
-    (256, 64 * 31, 640, 0.7),    # two column groups, the second one partly beyond N
+    (128, 64, 512, 0.8),         # one tile; at width 384 columns beyond N
+    (384, 64 * 5, 512, 0.9),     # fewer K tiles than stages
+    (256, 64 * 9, 640, 0.8),     # one K tile more than eight stages; groups of columns partly and wholly beyond N
+    (256, 64 * 31, 896, 0.7),
     (128, 64 * 13, 1024, 0.4),   # tiles above the register budget
-    (128, 64 * 7, 256, 0.0),     # dense tiles
-    (128, 64 * 900, 256, 0.995), # more offsets than shared memory stages at 384 and 512 columns
+    (128, 64 * 7, 512, 0.0),     # dense tiles
+    (128, 64 * 900, 512, 0.995), # more offsets than shared memory stages
 ])
 def test_widths(lib, oracle, pinned, width, M, K, N, sparsity):
     A, B = random_problem(lib, M, K, N, sparsity, M + K + N)
@@ -84,7 +84,7 @@ def test_malformed_offsets_are_reported_not_followed(lib, oracle, pinned):
     comp, offs, _ = lib.InitSparseMatrixA_API(A)
     broken = offs.copy()
     broken[25] = broken[24] - 3
-    pinned(producers=2)
+    pinned(producers=2, cluster_k=1)
     got = DeviceProblem(lib, comp, broken, B, M, N, K, 1).run(check_status=False)
     assert lib.consume_status() & 2
     want = oracle.gemm_f32(A, B)
