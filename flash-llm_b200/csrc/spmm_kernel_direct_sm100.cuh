@@ -118,6 +118,31 @@ __device__ __forceinline__ void scatter_batch(uint32_t stage, const uint4 (&buf)
         scatter_rows<CAP / 2, CAP, WPT, CAP>(stage, buf, rem);
 }
 
+// Scatters a warp's share of a tile of n_in vectors whose first CAP rows are in buf.  Rows beyond them are fetched half a
+// batch at a time into the registers just emptied, so that their latency hides behind the other half's stores
+// (DENSE_MEASURED).
+template<int WPT, int CAP>
+__device__ __forceinline__ void scatter_tile(uint32_t stage, uint4 (&buf)[CAP], const uint4* lane_base, int n_in, int rem)
+{
+    constexpr int H = CAP / 2, V = H * WPT * 32;  // rows and vectors of half a batch
+    if (n_in <= 2 * V) {
+        scatter_batch<WPT, CAP>(stage, buf, n_in, rem);
+        return;
+    }
+    for (int v0 = 0;; v0 += 2 * V) {
+        scatter_rows<0, H, WPT, CAP>(stage, buf, rem - v0);
+        if (n_in > v0 + 2 * V)
+            load_rows<0, H, WPT, CAP>(buf, lane_base + v0 + 2 * V, rem - v0 - 2 * V);
+        if (n_in <= v0 + V)
+            break;
+        scatter_rows<H, CAP, WPT, CAP>(stage, buf, rem - v0);
+        if (n_in > v0 + 3 * V)
+            load_rows<H, CAP, WPT, CAP>(buf, lane_base + v0 + 2 * V, rem - v0 - 2 * V);
+        if (n_in <= v0 + 2 * V)
+            break;
+    }
+}
+
 // How many of its own tiles ahead a scatter warp asks the memory system to bring into L2 (its register loads run one
 // tile ahead).
 #ifndef FLASHLLM_PREFETCH_AHEAD
@@ -421,13 +446,8 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
                         if ((nxt[q].x ^ nxt[q].y ^ nxt[q].z ^ nxt[q].w) == 0x9E3779B9u)  // keeps the loads alive
                             scatter_word(stage, nxt[q].x);
 #else
-                    scatter_batch<WPT, CAP>(stage, nxt, n_in, rem);
+                    scatter_tile<WPT, CAP>(stage, nxt, src + first_vec, n_in, rem);
 #endif
-                    // tiles denser than the register budget: the rest in further batches, fetched only now
-                    for (int v0 = CAP * WPT * 32; v0 < n_in; v0 += CAP * WPT * 32) {
-                        load_batch<WPT, CAP>(nxt, src + v0 + first_vec, n_in - v0, rem - v0);
-                        scatter_batch<WPT, CAP>(stage, nxt, n_in - v0, rem - v0);
-                    }
                 }
                 if (lane == 0)
                     FL_TRACE(5, j);

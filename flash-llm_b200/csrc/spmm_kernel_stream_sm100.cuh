@@ -135,12 +135,7 @@ struct TileStream {
             }
             zero_fill_stage(stage, lane);
             __syncwarp();  // another lane's zero must not land on top of a new value
-            const int rem = n_in - lane;
-            scatter_batch<1, CAP>(stage, nxt, n_in, rem);
-            for (int v0 = CAP * 32; v0 < n_in; v0 += CAP * 32) {  // tiles denser than the register budget
-                load_batch<1, CAP>(nxt, src + v0 + lane, n_in - v0, rem - v0);
-                scatter_batch<1, CAP>(stage, nxt, n_in - v0, rem - v0);
-            }
+            scatter_tile<1, CAP>(stage, nxt, src + lane, n_in, n_in - lane);
             ptx::fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0)
