@@ -109,6 +109,9 @@ int FlashLLM_EncodeOnDevice_Pack(void* stream, const void* A_d, int M, int K, co
         e = cudaFuncSetAttribute(csl_pack_reorder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kPackCarveoutPercent);
     if (e != cudaSuccess)
         return static_cast<int>(e);
+    const int groups = (tiles + kEncodeWarps - 1) / kEncodeWarps;
+    if (int rc = launch(csl_pack_dense_kernel, groups < 8 * sms ? groups : 8 * sms, kEncodeWarps))
+        return rc;
     const int blocks = (tiles + kPackWarps - 1) / kPackWarps;
     return launch(csl_pack_reorder_kernel, blocks < kPackCtasPerSm * sms ? blocks : kPackCtasPerSm * sms, kPackWarps);
 }

@@ -176,13 +176,13 @@ __global__ void __launch_bounds__(1024) csl_scan_kernel(int* __restrict__ offs, 
 // Step 2, reordered format, tiles with buckets of any height: counts, tabulates the per-height terms of q in shared
 // memory (s_mask: buckets at least this high; s_above: words lying above this height), reads the tile again and places
 // every word on its own.
-__device__ __noinline__ void pack_tall_tile(const uint16_t* __restrict__ tile, int K, int vectors, uint32_t* __restrict__ dst,
-                                            uint32_t* s_mask, uint16_t* s_above, int lane, unsigned int* status)
+__device__ __forceinline__ void pack_any_tile(const uint16_t* __restrict__ tile, int K, int vectors, uint32_t* __restrict__ dst,
+                                              uint32_t* s_mask, uint16_t* s_above, int lane, unsigned int* status)
 {
     const int words = vectors * kVectorWords;
     // pass 1: bucket sizes and each bucket's first zero cell
     int count = 0, zero_loc = -1;
-#pragma unroll 4
+#pragma unroll 8
     for (int r = 0; r < kTileM; ++r) {
         const int      x    = (r & 7) << 3;
         const int      c0   = (2 * lane) ^ x;  // the bucket's two cells sit at columns c0, c0 + 1
@@ -222,7 +222,7 @@ __device__ __noinline__ void pack_tall_tile(const uint16_t* __restrict__ tile, i
 
     // pass 2: place every word
     int h = 0;
-#pragma unroll 4
+#pragma unroll 8
     for (int r = 0; r < kTileM; ++r) {
         const int      x    = (r & 7) << 3;
         const int      c0   = (2 * lane) ^ x;
@@ -246,6 +246,39 @@ __device__ __noinline__ void pack_tall_tile(const uint16_t* __restrict__ tile, i
     }
 }
 
+__device__ __noinline__ void pack_tall_tile(const uint16_t* tile, int K, int vectors, uint32_t* dst, uint32_t* s_mask,
+                                            uint16_t* s_above, int lane, unsigned int* status)
+{
+    pack_any_tile(tile, K, vectors, dst, s_mask, s_above, lane, status);
+}
+
+// The tiles of more than kListVectors vectors, which csl_pack_reorder_kernel leaves out: a matrix of such tiles wants
+// more warps per SM than that kernel's shared memory allows.  Persistent, so that it costs 3 us where there are none.
+constexpr int kListVectors = 1088;  // 136 words to a bucket: hardly ever one above 164
+
+__global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_dense_kernel(const uint16_t* __restrict__ A,
+                                                                           int K,
+                                                                           int tiles,
+                                                                           int k_tiles,
+                                                                           const int* __restrict__ offs,
+                                                                           uint32_t* __restrict__ out,
+                                                                           unsigned int* status)
+{
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    __shared__ uint32_t s_mask[kEncodeWarps][kHeightEntries];
+    __shared__ uint16_t s_above[kEncodeWarps][kHeightEntries];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int t = blockIdx.x * kEncodeWarps + w; t < tiles; t += gridDim.x * kEncodeWarps) {
+        const int first = offs[t], vectors = offs[t + 1] - first;
+        if (vectors > kListVectors) {
+            pack_any_tile(tile_start(A, K, k_tiles, t), K, vectors, out + static_cast<size_t>(first) * kVectorWords, s_mask[w],
+                          s_above[w], lane, status);
+            __syncwarp();
+        }
+    }
+}
+
 // Step 2, reordered format.
 //
 // A lane appends its bucket's words to a column of shared memory, the newest on top (height h in row kListRows - h: bank =
@@ -257,8 +290,8 @@ __device__ __noinline__ void pack_tall_tile(const uint16_t* __restrict__ tile, i
 // one after it into L2.  Bound by a tile's latency and by the loads L1 can keep in flight beside the CTAs' shared memory;
 // us per 36864x9216 pack at 80 %: six CTAs per SM 244, five 224, four 210, four with the L2 prefetch 195, three 241.
 constexpr int kPackWarps = 2, kPackCtasPerSm = 4;
-constexpr int kListRows = 140, kSpareRows = 8;  // 38 KB of shared memory per CTA: buckets of tiles of 60 % sparsity and more
-constexpr int kPackCarveoutPercent = 68;  // of 228 KB: kPackCtasPerSm CTAs and 1 KB for each
+constexpr int kListRows = 168, kSpareRows = 8;  // 44 KB of shared memory per CTA: the buckets of tiles of 50 % sparsity and more
+constexpr int kPackCarveoutPercent = 82;        // of 228 KB: kPackCtasPerSm CTAs and 1 KB for each
 
 // This lane's pair of cells of every row: bucket `lane` owns columns c0, c0 + 1 with c0 = 2 * lane ^ ((r & 7) << 3).
 __device__ __forceinline__ void load_bucket(uint32_t (&pair)[kTileM], const uint16_t* tile, int K, int lane)
@@ -303,13 +336,20 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
     uint32_t        pair[kTileM];
     // last tiles first: the counting pass has just read them and L2 still holds the end of the matrix
     int t = tiles - 1 - (static_cast<int>(blockIdx.x) * kPackWarps + w);
-    if (t >= 0)
+    auto vectors_of = [&](int tile) { return tile >= 0 ? offs[tile + 1] - offs[tile] : kListVectors + 1; };
+    int  vectors = vectors_of(t), vectors1 = vectors_of(t - stride);  // of this tile and the next one
+    if (vectors <= kListVectors)
         load_bucket(pair, tile_start(A, K, k_tiles, t), K, lane);
-    for (; t >= 0; t -= stride) {
-        const int       first   = offs[t];
-        const int       vectors = offs[t + 1] - first;
-        const int       words   = vectors * kVectorWords;
-        uint32_t* const dst     = out + static_cast<size_t>(first) * kVectorWords;
+    for (int vectors2; t >= 0; t -= stride, vectors = vectors1, vectors1 = vectors2) {
+        vectors2 = vectors_of(t - 2 * stride);
+        if (vectors > kListVectors) {  // csl_pack_dense_kernel's
+            if (vectors1 <= kListVectors)
+                load_bucket(pair, tile_start(A, K, k_tiles, t - stride), K, lane);
+            continue;
+        }
+        const int       first = offs[t];
+        const int       words = vectors * kVectorWords;
+        uint32_t* const dst   = out + static_cast<size_t>(first) * kVectorWords;
 
         // ---- the bucket's words, oldest in the last row
         __syncwarp();  // the previous tile's words have been read
@@ -340,9 +380,9 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
             at = at2;
             loc += kTileK;
         }
-        if (t >= stride)
+        if (vectors1 <= kListVectors)
             load_bucket(pair, tile_start(A, K, k_tiles, t - stride), K, lane);
-        if (t >= 2 * stride)
+        if (vectors2 <= kListVectors)
             prefetch_tile(tile_start(A, K, k_tiles, t - 2 * stride), K, lane);
         const int count = static_cast<int>(bottom - at) >> 7;
         if (__any_sync(0xFFFFFFFFu, count > kListRows - kVectorWords)) {  // (a column that overflowed counts at least kListRows)

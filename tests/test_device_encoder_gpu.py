@@ -70,17 +70,22 @@ def test_device_encoded_buffers_feed_the_kernel(lib, oracle):
 
 @pytest.mark.parametrize("shift", [0, 2])
 def test_tiles_of_every_density_and_special_values(lib, shift):
-    """Buckets from empty to all 256 cells, around the height a warp's lists hold (136 words), with zeros, NaN, infinities
-    and subnormals among them; groups of 32 tiles that end in the middle of a row; A only 4-byte aligned."""
+    """Tiles on both sides of the density that has a kernel of its own (1088 vectors), sparse ones with a full bucket (a warp's
+    lists hold 164 words), zeros, NaN, infinities and subnormals among them; groups of 32 tiles that end in the middle of a row; A only 4-byte aligned."""
     M, K = 128 * 5, 64 * 27
     rng = np.random.default_rng(5)
     A = rng.uniform(-1, 1, (M, K)).astype(np.float16)
-    density = rng.choice([0.0, 0.05, 0.2, 0.4, 0.5, 0.53, 0.6, 0.9, 1.0], size=(M // 128, K // 64))
+    density = rng.choice([0.0, 0.05, 0.2, 0.4, 0.5, 0.53, 0.54, 0.6, 0.9, 1.0], size=(M // 128, K // 64))
     A[rng.random((M, K)) >= np.kron(density, np.ones((128, 64)))] = 0
     bits = A.view(np.uint16)
     special = rng.random((M, K))
     for i, b in enumerate((0x8000, 0x7C00, 0xFC00, 0x7E00, 0xFFFF, 0x0001, 0x83FF)):
         bits[(special > i * 0.004) & (special <= (i + 1) * 0.004)] = b
+    for r in range(128):  # bucket 3 of the first tile full, bucket 31 of the last one but for its last cells
+        for tile_row, tile_col, bucket in ((0, 0, 3), (4, 26, 31)):
+            c = tile_col * 64 + ((2 * bucket) ^ ((r & 7) << 3))
+            A[tile_row * 128 + r, tile_col * 64:tile_col * 64 + 64] *= np.float16(0 if r % 3 else 1)
+            A[tile_row * 128 + r, c:c + 2] = 0.5 if r < 126 or tile_row == 0 else 0
     comp_h, offs_h, _ = lib.InitSparseMatrixA_API(A)
     flat = torch.zeros(M * K + 8, dtype=torch.float16, device="cuda")
     A_d = flat[shift:shift + M * K]
