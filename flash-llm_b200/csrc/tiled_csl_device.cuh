@@ -253,7 +253,7 @@ __device__ __noinline__ void pack_tall_tile(const uint16_t* tile, int K, int vec
 }
 
 // The tiles of more than kListVectors vectors, which csl_pack_reorder_kernel leaves out: a matrix of such tiles wants
-// more warps per SM than that kernel's shared memory allows.  Persistent, so that it costs 3 us where there are none.
+// more warps per SM than that kernel's shared memory allows.  Persistent, so that it costs 4 to 9 us where there are none.
 constexpr int kListVectors = 1088;  // 136 words to a bucket: hardly ever one above 164
 
 __global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_dense_kernel(const uint16_t* __restrict__ A,
@@ -287,8 +287,9 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_dense_kernel(const
 // is read before anything can be written over it).  The words then leave as whole 16-byte vectors.
 //
 // The grid is persistent: while the words of a tile are dealt and stored, the next one is on its way into registers and the
-// one after it into L2.  Bound by a tile's latency and by the loads L1 can keep in flight beside the CTAs' shared memory;
-// us per 36864x9216 pack at 80 %: six CTAs per SM 244, five 224, four 210, four with the L2 prefetch 195, three 241.
+// one after it into L2.  Bound by its own instructions (0.59 of the issue slots, hardly a stall on memory): the lists take
+// the shared memory that more warps would need, and L1 needs what they leave for the loads in flight.  us per 36864x9216
+// pack at 80 %: six CTAs per SM 244, five 224, four 210, four with the L2 prefetch 195, three 241 (lists of 140 rows).
 constexpr int kPackWarps = 2, kPackCtasPerSm = 4;
 constexpr int kListRows = 168, kSpareRows = 8;  // 44 KB of shared memory per CTA: the buckets of tiles of 50 % sparsity and more
 constexpr int kPackCarveoutPercent = 82;        // of 228 KB: kPackCtasPerSm CTAs and 1 KB for each
