@@ -355,10 +355,10 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
         // ---- the bucket's words, oldest in the last row
         __syncwarp();  // the previous tile's words have been read
         uint32_t at  = bottom;                           // where the next word goes
-        uint32_t loc = static_cast<uint32_t>(2 * lane);  // of the row's first cell
+        uint32_t loc = static_cast<uint32_t>(2 * lane) * 0x10001u + 0x10000u;  // of the row's two cells, low half first
 #pragma unroll
         for (int r = 0; r < kTileM; ++r) {
-            const uint32_t w0 = __byte_perm(pair[r], loc, 0x5410), w1 = __byte_perm(pair[r], loc + 1, 0x5432);
+            const uint32_t w0 = __byte_perm(pair[r], loc, 0x5410), w1 = __byte_perm(pair[r], loc, 0x7632);
             if (r % (kSpareRows / 2) == 0)  // at most kSpareRows words until the next look
                 at = static_cast<int>(at) > static_cast<int>(limit) ? at : limit;
             // (a position that a store has yet to read cannot be overwritten: it moves on through fresh registers)
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
                 : "r"(at), "r"(pair[r]), "r"(w0), "r"(w1), "r"(0u)
                 : "memory");
             at = at2;
-            loc += kTileK;
+            loc += kTileK * 0x10001u;
         }
         if (vectors1 <= kListVectors)
             load_bucket(pair, tile_start(A, K, k_tiles, t - stride), K, lane);
