@@ -318,8 +318,11 @@ static cudaError_t make_stream_plan(const DeviceState* st, SpmmPlan pl, int tile
 // Fitted to launches of 8..288 tile rows by 16..512 K tiles, B200, back to back on one stream:
 //   one CTA (cluster) per tile row  10.5 + 2.3 with a cluster sum + the tiles of a CTA per wave, two thirds of that while
 //                                   no SM holds two CTAs; + 4 for a second kernel
-//   streaming form                  0.93 of the tiles of a CTA + 15 + 0.45 per part of a row at N <= 16, more for wider
-//                                   parts (the last part's CTA sums the row while everybody else has finished)
+//   streaming form                  0.93 of the tiles of a CTA + 15 + 0.32 per part of a row at N <= 16, more for wider
+//                                   parts (the last part's CTA sums the row while everybody else has finished).  At 0.45
+//                                   for N <= 16 some forty shapes of 4..56 rows went by rows, 2..43 % slower: 2048x16384
+//                                   70 % 23.5 us against 16.4, 512x32768 30.4 / 22.8, 2048x32768 26.5 / 24.5; below 0.3
+//                                   512x22400 90 % (17.9 / 21.5) and 32000x1536 (18.2 / 19.4) would change too
 static double one_row_cost(const DeviceState* st, long long capacity, int ctas_flat, int k_tiles, int s, int g, int n_tile)
 {
     const long long clusters = static_cast<long long>(ctas_flat) * g;
@@ -332,7 +335,7 @@ static double stream_cost(const SpmmPlan& pl, int tile_rows, int k_tiles)
 {
     const double tiles = static_cast<double>(tile_rows) * k_tiles / pl.ctas;
     const double parts = 1.0 + static_cast<double>(pl.ctas) / tile_rows;
-    return 0.93 * tiles + 15.0 + (pl.n_tile - 16) * 0.15 + 0.45 * parts * (0.5 + pl.n_tile / 32.0);
+    return 0.93 * tiles + 15.0 + (pl.n_tile - 16) * 0.15 + parts * (pl.n_tile <= 16 ? 0.32 : 0.225 + pl.n_tile * 0.45 / 32.0);
 }
 
 // Clusters of S CTAs resident at a time on 148 SMs (measured), two CTAs or one per SM.
