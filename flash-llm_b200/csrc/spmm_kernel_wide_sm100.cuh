@@ -12,7 +12,7 @@
 //
 // Measured (B200, 80 %, us per call, 128 columns per CTA -> this form): 36864x9216 N = 256 / 384 / 512: 211 / 312 / 414 ->
 // 139 / 186 / 228 (1.53 PFLOP/s of dense contraction); 9216x9216: 51 / 100 / 99 -> 42 / 59 / 66; 4736x7232: 29 / 42 / 42 ->
-// 27 / 36 / 35.  512 columns are bound by the MMAs (1024 cycles of the 1300 per tile), 256 by the shared-memory path.  Tried
+// 27 / 36 / 35 (384 columns with 6 + 5 stages, before 8 + 4).  512 columns are bound by the MMAs (1024 cycles of the 1300 per tile), 256 by the shared-memory path.  Tried
 // and not kept: CTA pairs (cta_group::2, M = 256, half of B each), 1..6 % faster where the rows come out even and up to
 // 40 % slower where K has to be cut (33 clusters of four fit the GPU, 74 of two).
 #pragma once
@@ -21,11 +21,13 @@
 namespace flashllm {
 
 // Columns of one MMA, number of them per tile, A stages (= scatter warps) and B stages for `n_tile` output columns a CTA:
-// what fits the 227 KB of one CTA per SM.
+// 224 of the 227 KB of one CTA per SM.  Measured both ways (18944x9216 / 9472x4096 / 2048x8192 at 62..95 %): 384 columns with
+// 8 + 4 stages instead of 6 + 5 1..8 % faster (all eight warps share the epilogue), 512 columns with 8 + 3 or 7 + 3 4..15 %
+// slower (a slab of B is 512 MMA cycles, three of them less than its way from L2), 256 with 6 + 4 or 4 + 5 up to 20 % slower.
 __host__ __device__ constexpr int wide_mma_n(int n_tile) { return n_tile <= 256 ? n_tile : n_tile / 2; }
 __host__ __device__ constexpr int wide_slabs(int n_tile) { return n_tile / wide_mma_n(n_tile); }
-__host__ __device__ constexpr int wide_a_stages(int n_tile) { return n_tile <= 256 ? 8 : 6; }
-__host__ __device__ constexpr int wide_b_stages(int n_tile) { return n_tile == 256 ? 3 : n_tile == 384 ? 5 : 4; }
+__host__ __device__ constexpr int wide_a_stages(int n_tile) { return n_tile <= 384 ? 8 : 6; }
+__host__ __device__ constexpr int wide_b_stages(int n_tile) { return n_tile == 256 ? 3 : 4; }
 constexpr int kWideFirstScatter = 2;
 constexpr int kWideCap          = 24;  // vectors per lane kept in registers: tiles of up to 62.5 % sparsity
 
