@@ -308,6 +308,20 @@ __device__ __forceinline__ void tmem_wait_ld()
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Writes 8 columns of this warp's tensor-memory lanes, one row per lane (the layout tmem_ld_x8 reads).
+__device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const float (&v)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+                 "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_wait_st()
+{
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major operand whose rows are 128 bytes (64 fp16), stored with the
 // 128-byte swizzle in groups of 8 rows (1024 bytes per group); `addr` is the 1024-byte-aligned tile base
 // plus 32 bytes per 16-wide K step.

@@ -289,8 +289,16 @@ static int stream_smem_bytes(const SpmmPlan& pl)
            + 8 * (2 * kStreamStages + 4 + 2 * pl.b_stages) + 16 + 4 * pl.offsets_staged;
 }
 
+// K tiles that the tensor core adds up in one accumulator when K is cut into `parts` and every CTA alternates between two.
+// The tensor core truncates each of its additions, so the error of a sum grows with their number (measured: 7e-8 of the sum
+// per tile of four); the streaming form keeps to what the plan of one CTA or cluster per tile row comes to at the same sizes.
+static int tiles_per_accumulator(int k_tiles, int parts)
+{
+    return ((k_tiles + parts - 1) / parts + 1) / 2;
+}
+
 // The streaming form: as many CTAs as the GPU holds, fewer only when there are fewer tiles.
-static cudaError_t make_stream_plan(const DeviceState* st, SpmmPlan pl, int tile_rows, int k_tiles, SpmmPlan* out)
+static cudaError_t make_stream_plan(const DeviceState* st, SpmmPlan pl, int tile_rows, int k_tiles, int chunk_tiles, SpmmPlan* out)
 {
     const long long tiles = static_cast<long long>(tile_rows) * k_tiles;
     long long       ctas  = static_cast<long long>(kStreamCtasPerSm) * st->sm_count;
@@ -299,6 +307,7 @@ static cudaError_t make_stream_plan(const DeviceState* st, SpmmPlan pl, int tile
     if (pl.n_tile > kScratchMaxN || tile_rows > kScratchRows || tiles > 0x7FFFFFFFll)
         return cudaErrorInvalidConfiguration;
     pl.ctas           = static_cast<int>(ctas);
+    pl.chunk_tiles    = chunk_tiles;
     pl.cluster_k      = 1;
     pl.workspace_k    = 1;
     pl.scatter_warps  = kStreamStages;
@@ -430,7 +439,7 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     for (int v : ov.v)
         pinned |= v != 0;
     if (pl.path == kPathStream)  // pinned: other fields do not apply to it
-        return may_stream && !sends ? make_stream_plan(st, pl, tile_rows, k_tiles, out) : cudaErrorInvalidConfiguration;
+        return may_stream && !sends ? make_stream_plan(st, pl, tile_rows, k_tiles, (k_tiles + 1) / 2, out) : cudaErrorInvalidConfiguration;
     if (pl.path == kPathWide || (N >= 256 && !pinned && !sends)) {
         if (N < 256 || N % 128 != 0 || sends)
             return cudaErrorInvalidConfiguration;
@@ -508,7 +517,7 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     if (may_stream && !pinned && !sends) {
         SpmmPlan sp = pl;
         sp.path     = kPathStream;
-        if (make_stream_plan(st, sp, tile_rows, k_tiles, &sp) == cudaSuccess
+        if (make_stream_plan(st, sp, tile_rows, k_tiles, tiles_per_accumulator(k_tiles, best_s * best_g), &sp) == cudaSuccess
             && stream_cost(sp, tile_rows, k_tiles) < one_row_cost(st, capacity(best_s), ctas_flat, k_tiles, best_s, best_g, pl.n_tile)) {
             *out = sp;
             return cudaSuccess;

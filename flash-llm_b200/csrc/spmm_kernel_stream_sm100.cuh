@@ -7,9 +7,12 @@
 // is a segment:
 //
 //   * scatter warps decompress tile after tile as in the register-streaming form and know nothing of rows;
-//   * the MMA-issuing warp accumulates a segment in one of two tensor-memory accumulators and changes over at a row's
-//     end without draining anything;
-//   * four epilogue warps read a finished accumulator while the next segment is being multiplied.  A segment that is a
+//   * the MMA-issuing warp multiplies a segment in chunks of at most plan.chunk_tiles tiles, each in the other one of two
+//     tensor-memory accumulators than the chunk before, and changes over without draining anything;
+//   * four epilogue warps read a finished accumulator while the next chunk is being multiplied and add a segment's chunks
+//     up in fp32, in tensor memory.  The tensor core truncates every one of its additions: with a segment in one accumulator
+//     36864x9216 N = 16 at 80 % was 2.07501e-4 off its exact values in the 2-norm, in chunks it is 2.07427e-4 (rounding to
+//     fp16 alone: 2.07382e-4), and a layer of four such matmuls 3.03e-4 instead of 3.49e-4.  A segment that is a
 //     whole row becomes output at once; a part of a row is parked as an fp32 tile in the stream's scratch and counted in
 //     on the row's counter, and whoever completes the count adds the parts up in CTA order (the same bits whoever comes
 //     last) and finishes the output.  No CTA waits for another.
@@ -18,12 +21,13 @@
 // registers.  Issued from a branch taken by one lane, the four MMAs and the commit of a tile cost 271 cycles instead of
 // the 170 the tensor core needs for them (M128 N16 K16), which took two issuing warps to hide.
 //
-// Measured (B200, back to back on one stream, against one CTA or cluster per tile row): 27648x9216 N=8 90 % 62.8 -> 46.4 us,
-// 25600x9216 N=16 80 % 75.9 -> 53.0, 9216x36864 N=32 70 % 106 -> 103, 49152x12288 N=64 80 % 184 -> 166, 36864x9216 N=16
-// 80 % (288 rows: hardly any quantisation to begin with) 76.8 -> 72.0.  A CTA's share is bound by the shared-memory work of
-// its tiles: of ~3300 cycles from one tile of a stage to the next at 80 %, 570 go to clearing the stage, 1140 to the 16-bit
-// scatter stores (they wait for the tensor core's operand reads), 1070 to getting the next tile's loads issued behind the
-// other warps' stores, 430 to the stage's hand-back.  Six stages per CTA, or one CTA of 8 or 12 warps per SM, are slower.
+// Measured (B200, back to back on one stream, against one CTA or cluster per tile row): 27648x9216 N=8 90 % 62.8 -> 45.3 us,
+// 25600x9216 N=16 80 % 75.9 -> 53.0, 9216x36864 N=32 70 % 106.5 -> 106.2, 49152x12288 N=64 80 % 184 -> 169, 36864x9216 N=16
+// 80 % (288 rows: hardly any quantisation to begin with) 76.8 -> 73.4.  The chunks cost 0 to 0.7 % of that, at N = 64 1.3 %.
+// A CTA's share is bound by the shared-memory work of its tiles: of ~3300 cycles from one tile of a stage to the next at
+// 80 % (8 stages per SM: 412 per tile), 570 go to clearing the stage, 1140 to the 16-bit scatter stores (they wait for the
+// tensor core's operand reads), 1070 to getting the next tile's loads issued behind the other warps' stores, 430 to the
+// stage's hand-back.  Six stages per CTA, or one CTA of 8 or 12 warps per SM, are slower.
 #pragma once
 #include "spmm_kernel_direct_sm100.cuh"
 
@@ -155,16 +159,14 @@ struct TileStream {
 // Adds the parked parts of tile row `row` up in CTA order and finishes the output (the 128 epilogue threads).
 template<int N_TILE>
 __device__ __forceinline__ void
-sum_row_parts(const SpmmParams& p, long long tiles, int ctas, int row, int c_first, int c_last, int tid)
+sum_row_parts(const SpmmParams& p, int row, int c_first, int c_last, const float* first, int tid)
 {
-    const long long row_begin = static_cast<long long>(row) * p.k_tiles;
-    const size_t    slot      = static_cast<size_t>(N_TILE) * kTileM;
-    const bool      wide_out  = (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
-    // only the row's first CTA may have begun before the row: this is then its last segment, in its second slot
-    const float* const first = p.partial + slot * (2 * c_first + (stream_begin(tiles, ctas, c_first) < row_begin ? 1 : 0));
-    // Four groups of four outputs per thread and three parts at a time: twelve 16-byte loads in flight (a part is an L2
-    // round trip away, and a row of a narrow matrix may have twenty of them); added in CTA order.
-    constexpr int Q = 4, P = 3;
+    const size_t slot     = static_cast<size_t>(N_TILE) * kTileM;
+    const bool   wide_out = (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
+    // Two groups of four outputs per thread and five parts at a time: ten 16-byte loads in flight (a part is an L2 round
+    // trip away, and a row of a narrow matrix may have twenty of them); added in CTA order.  One part more and the kernel
+    // needs local memory, which costs every launch 0.5 us.
+    constexpr int Q = 2, P = 5;
     const int     quads = p.N * (kTileM / 4);
     for (int q0 = tid; q0 < quads; q0 += Q * 128) {
         float4 acc[Q];
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
 {
     static_assert(N_TILE == 16 || N_TILE == 32 || N_TILE == 64, "unsupported MMA N");
     constexpr uint32_t kBSlab    = N_TILE * kTileK * 2;              // one K tile of B in shared memory
-    constexpr uint32_t kTmemCols = 2 * N_TILE < 32 ? 32 : 2 * N_TILE;  // two accumulators
+    constexpr uint32_t kTmemCols = 4 * N_TILE;  // two accumulators and the sum of a segment's finished chunks; a power of two
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t raw_addr = ptx::smem_u32(smem_raw);
@@ -231,6 +233,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
 
     const int       b_stages = p.plan.b_stages;
     const int       KB       = p.plan.b_batch;
+    const int       chunk    = p.plan.chunk_tiles;
     const int       ctas     = gridDim.x;
     const int       cta      = blockIdx.x;
     const long long tiles    = static_cast<long long>(p.M / kTileM) * p.k_tiles;
@@ -359,41 +362,45 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
             const uint32_t idesc   = ptx::umma_idesc_f16_f32(kTileM, N_TILE);
             const uint64_t a_desc0 = ptx::umma_desc_kmajor_sw128(a_base);
             const uint64_t b_desc0 = ptx::umma_desc_kmajor_sw128(b_base);
-            int            s = 0, bs = 0, seg = 0;
+            int            s = 0, bs = 0, q = 0;
             uint32_t       a_par = 0, b_par = 0;
             bool           ok = true;
-            for (int j = 0, k = k0; ok && j < L; k = 0, ++seg) {
-                const int      len = L - j < p.k_tiles - k ? L - j : p.k_tiles - k;
-                const uint32_t acc = tmem_acc + static_cast<uint32_t>((seg & 1) * N_TILE);
-                ok = __all_sync(0xFFFFFFFFu, wait_bounded_converged(acc_empty + 8u * (seg & 1), ((seg >> 1) & 1u) ^ 1u, abort_flag,
-                                                                    p.status));
-                for (int i = 0, kb = 0; ok && i < len; ++i) {
-                    ok = wait_bounded_converged(a_full + 8u * s, a_par, abort_flag, p.status);
-                    if (kb == 0)
-                        ok = wait_bounded_converged(b_full + 8u * bs, b_par, abort_flag, p.status) && ok;
-                    ok = __all_sync(0xFFFFFFFFu, ok);
-                    if (!ok)
-                        break;
-                    const bool batch_done = kb + 1 == KB || i + 1 == len;
-                    ptx::tc_fence_after_sync();
-                    ptx::umma_tile_elect(acc, a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
-                                         b_desc0 + static_cast<uint32_t>((bs * KB + kb) * (kBSlab >> 4)), idesc, i != 0 ? 1u : 0u,
-                                         a_empty + 8u * s, b_empty + 8u * bs, batch_done ? 1u : 0u);
-                    if (++s == kStreamStages) {
-                        s = 0;
-                        a_par ^= 1u;
-                    }
-                    ++kb;
-                    if (batch_done) {
-                        kb = 0;
-                        if (++bs == b_stages) {
-                            bs = 0;
-                            b_par ^= 1u;
+            for (int j = 0, k = k0; ok && j < L; k = 0) {
+                const int len = L - j < p.k_tiles - k ? L - j : p.k_tiles - k;
+                int       kb  = 0;
+                for (int i0 = 0; ok && i0 < len; i0 += chunk, ++q) {
+                    const int      n   = len - i0 < chunk ? len - i0 : chunk;
+                    const uint32_t acc = tmem_acc + static_cast<uint32_t>((q & 1) * N_TILE);
+                    ok = __all_sync(0xFFFFFFFFu, wait_bounded_converged(acc_empty + 8u * (q & 1), ((q >> 1) & 1u) ^ 1u, abort_flag,
+                                                                        p.status));
+                    for (int i = 0; ok && i < n; ++i) {
+                        ok = wait_bounded_converged(a_full + 8u * s, a_par, abort_flag, p.status);
+                        if (kb == 0)
+                            ok = wait_bounded_converged(b_full + 8u * bs, b_par, abort_flag, p.status) && ok;
+                        ok = __all_sync(0xFFFFFFFFu, ok);
+                        if (!ok)
+                            break;
+                        const bool batch_done = kb + 1 == KB || i0 + i + 1 == len;
+                        ptx::tc_fence_after_sync();
+                        ptx::umma_tile_elect(acc, a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
+                                             b_desc0 + static_cast<uint32_t>((bs * KB + kb) * (kBSlab >> 4)), idesc, i != 0 ? 1u : 0u,
+                                             a_empty + 8u * s, b_empty + 8u * bs, batch_done ? 1u : 0u);
+                        if (++s == kStreamStages) {
+                            s = 0;
+                            a_par ^= 1u;
+                        }
+                        ++kb;
+                        if (batch_done) {
+                            kb = 0;
+                            if (++bs == b_stages) {
+                                bs = 0;
+                                b_par ^= 1u;
+                            }
                         }
                     }
+                    if (ok)
+                        ptx::umma_commit_elect(acc_full + 8u * (q & 1));
                 }
-                if (ok)
-                    ptx::umma_commit_elect(acc_full + 8u * (seg & 1));
                 j += len;
             }
         }
@@ -408,45 +415,75 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
         const int tid     = threadIdx.x - kStreamFirstEpi * 32;
         const int quarter = warp & 3;  // the tensor-memory lanes this warp may read
         const int r       = quarter * 32 + lane;
-        int       seg     = 0;
-        for (int j = 0, k = k0, row = row0; j < L; k = 0, ++row, ++seg) {
-            const int      len   = L - j < p.k_tiles - k ? L - j : p.k_tiles - k;
+        const uint32_t tmem_lanes = tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16);
+        const uint32_t tmem_sum   = tmem_lanes + 2u * N_TILE;
+        // eight columns of chunk q, added to the sum of the segment's chunks before it (`more`: there are such)
+        auto read_columns = [&](int q, int c0, bool more, float (&v)[8]) {
+            uint32_t t[8];
+            ptx::tmem_ld_x8(tmem_lanes + static_cast<uint32_t>((q & 1) * N_TILE + c0), t);
+            ptx::tmem_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                v[e] = __uint_as_float(t[e]);
+            if (more) {
+                ptx::tmem_ld_x8(tmem_sum + c0, t);
+                ptx::tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    v[e] += __uint_as_float(t[e]);
+            }
+            if (c0 + 8 == N_TILE) {  // the accumulator has been read: the issuer may start the chunk after next in it
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0)
+                    ptx::mbar_arrive(acc_empty + 8u * (q & 1));
+            }
+        };
+        int q = 0;
+        for (int row = row0;; ++row) {
+            const int j = row == row0 ? 0 : (row - row0) * p.k_tiles - k0;
+            if (j >= L)
+                break;
+            const int      len   = j == 0 ? min(L, p.k_tiles - k0) : min(L - j, p.k_tiles);
             const bool     whole = len == p.k_tiles;
-            const uint32_t acc   = tmem_acc + static_cast<uint32_t>((seg & 1) * N_TILE) + (static_cast<uint32_t>(quarter * 32) << 16);
-            bool           ok    = go && wait_bounded_converged(acc_full + 8u * (seg & 1), (seg >> 1) & 1u, abort_flag, p.status);
-            ok                   = __all_sync(0xFFFFFFFFu, ok);
-            ptx::tc_fence_after_sync();
-            float* const park = whole ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (seg == 0 ? 0 : 1)) + r;
-            if (ok) {
+            bool           ok    = go;
+            int            i     = 0;
+            for (; ok; i += chunk, ++q) {
+                ok = __all_sync(0xFFFFFFFFu, wait_bounded_converged(acc_full + 8u * (q & 1), (q >> 1) & 1u, abort_flag, p.status));
+                ptx::tc_fence_after_sync();
+                if (!ok || i + chunk >= len)
+                    break;
 #pragma unroll 1
                 for (int c0 = 0; c0 < N_TILE; c0 += 8) {
-                    uint32_t t[8];
-                    ptx::tmem_ld_x8(acc + c0, t);
-                    ptx::tmem_wait_ld();
-                    if (c0 + 8 == N_TILE) {  // the accumulator has been read: the issuer may start a segment in it
-                        ptx::tc_fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0)
-                            ptx::mbar_arrive(acc_empty + 8u * (seg & 1));
-                    }
                     float v[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        v[i] = __uint_as_float(t[i]);
+                    read_columns(q, c0, i != 0, v);
+                    ptx::tmem_st_x8(tmem_sum + c0, v);
+                }
+                ptx::tmem_wait_st();
+            }
+            float* const park = whole ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (j == 0 ? 0 : 1)) + r;
+            if (ok) {  // the segment's last chunk
+#pragma unroll 1
+                for (int c0 = 0; c0 < N_TILE; c0 += 8) {
+                    float v[8];
+                    read_columns(q, c0, i != 0, v);
                     if (park != nullptr) {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (c0 + i < p.N)
-                                __stcg(park + (c0 + i) * kTileM, v[i]);
+                        for (int e = 0; e < 8; ++e)
+                            if (c0 + e < p.N)
+                                __stcg(park + (c0 + e) * kTileM, v[e]);
                     }
                     else
                         finish_columns<8>(p, v, static_cast<size_t>(c0) * p.M + row * kTileM + r, p.N - c0, row * kTileM + r);
                 }
+                ++q;
             }
             if (!whole) {
                 const long long row_begin = static_cast<long long>(row) * p.k_tiles;
                 const int       c_first   = stream_owner(tiles, ctas, row_begin);
                 const int       c_last    = stream_owner(tiles, ctas, row_begin + p.k_tiles - 1);
+                // only the row's first CTA may have begun before the row: this is then its last segment, in its second slot
+                const int       slot      = 2 * c_first + (stream_begin(tiles, ctas, c_first) < row_begin ? 1 : 0);
                 const bool gave_up = barrier_any(1u, 128u, !ok);
                 if (tid == 0) {
                     // arrivals in the low half of the counter; a CTA that gave up also marks the high half, so that the
@@ -461,11 +498,10 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                 }
                 ptx::named_barrier_sync(1u, 128u);
                 if (abort_flag[kLastOfTile] == 1u) {
-                    sum_row_parts<N_TILE>(p, tiles, ctas, row, c_first, c_last, tid);
+                    sum_row_parts<N_TILE>(p, row, c_first, c_last, p.partial + static_cast<size_t>(N_TILE) * kTileM * slot, tid);
                 }
                 ptx::named_barrier_sync(1u, 128u);  // kLastOfTile is free again
             }
-            j += len;
         }
     }
 

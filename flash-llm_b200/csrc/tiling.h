@@ -54,7 +54,8 @@ constexpr int kPathWide   = 4;  // one CTA per tile row and 256..512 output colu
 
 struct SpmmPlan {
     int path;    // kPathRing, kPathDirect, kPathStream or kPathWide
-    int ctas;    // kPathStream: CTAs of the persistent grid
+    int ctas;         // kPathStream: CTAs of the persistent grid
+    int chunk_tiles;  // kPathStream: tiles added up in one accumulator of the tensor core
     int n_tile;  // output columns of a CTA: 16, 32, 64 or 128; kPathWide: 256, 384 or 512
     int cluster_k;
     int workspace_k;

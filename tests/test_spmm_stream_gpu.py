@@ -40,6 +40,33 @@ def test_shares_of_the_tile_sequence(lib, oracle, streaming, M, K, N, sparsity):
         assert np.array_equal(prob.run(), first)
 
 
+@pytest.mark.parametrize("M,K,N", [(27648, 9216, 16), (27648, 9216, 32), (49152, 4608, 64)])
+def test_sums_are_as_exact_as_the_row_forms(lib, M, K, N):
+    """The tensor core truncates its additions, so sums of positive products come out too small by a share that grows with
+    the tiles added up in one accumulator.  The mean of that share over all outputs, against 64-bit products, must not be
+    larger than the row form's; rounding to fp16 leaves the mean of 440 thousand and more outputs uncertain by
+    2^-11 / sqrt(12 * 440000) = 2e-7, so 1e-6 is allowed."""
+    from flash_llm_b200 import torch_op  # noqa: F401  (registers torch.ops.flashllm)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M + N)
+    A = torch.rand((M, K), generator=gen, device="cuda").half()
+    A *= torch.rand((M, K), generator=gen, device="cuda") >= 0.8
+    B = torch.rand((N, K), generator=gen, device="cuda").half()
+    want = torch.cat([B.double() @ A[r:r + 1024].double().T for r in range(0, M, 1024)], dim=1)
+    words, offs = torch.ops.flashllm.encode(A)
+    share = {}
+    try:
+        for path in (lib.api.PATH_STREAM, lib.api.PATH_DIRECT):
+            if path == lib.api.PATH_DIRECT:
+                lib.set_plan(path=path)
+            assert lib.get_plan(M, N, K, 1)["path"] == path
+            share[path] = float(((want - torch.ops.flashllm.spmm(words, offs, B, M).double()) / want).mean())
+    finally:
+        lib.set_plan()
+    assert lib.consume_status() == 0
+    assert abs(share[lib.api.PATH_STREAM]) <= abs(share[lib.api.PATH_DIRECT]) + 1e-6, share
+
+
 @pytest.mark.parametrize("bias,relu,residual", [(True, False, False), (True, True, False), (True, False, True), (False, True, True)])
 def test_output_epilogues(lib, oracle, streaming, bias, relu, residual):
     """Whole rows leave through one epilogue and summed rows through another; C only two-byte aligned takes narrow stores."""
