@@ -28,6 +28,10 @@ __host__ __device__ constexpr int wide_mma_n(int n_tile) { return n_tile <= 256 
 __host__ __device__ constexpr int wide_slabs(int n_tile) { return n_tile / wide_mma_n(n_tile); }
 __host__ __device__ constexpr int wide_a_stages(int n_tile) { return n_tile <= 384 ? 8 : 6; }
 __host__ __device__ constexpr int wide_b_stages(int n_tile) { return n_tile == 256 ? 3 : 4; }
+// Accumulators that the tiles take turns in.  Two halve the truncated additions of a sum; 384 and 512 columns leave no room
+// for a second one (see tiles_per_accumulator): 36864x9216 N = 512 at 80 % is 2.0755e-4 off its exact values in the 2-norm,
+// with 256 columns and two accumulators 2.0736e-4 and 29 % slower, where rounding to fp16 alone is 2.0730e-4.
+__host__ __device__ constexpr int wide_accumulators(int n_tile) { return n_tile <= 256 ? 2 : 1; }
 constexpr int kWideFirstScatter = 2;
 constexpr int kWideCap          = 24;  // vectors per lane kept in registers: tiles of up to 62.5 % sparsity
 
@@ -39,7 +43,8 @@ __global__ void __launch_bounds__((kWideFirstScatter + wide_a_stages(N_TILE)) * 
     constexpr int      kMmaN     = wide_mma_n(N_TILE), kSlabs = wide_slabs(N_TILE);
     constexpr int      STAGES    = wide_a_stages(N_TILE), B_STAGES = wide_b_stages(N_TILE);
     constexpr uint32_t kBSlab    = kMmaN * kTileK * 2;
-    constexpr uint32_t kTmemCols = N_TILE <= 256 ? 256 : 512;
+    constexpr int      kAccs     = wide_accumulators(N_TILE);
+    constexpr uint32_t kTmemCols = 512;
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t base = ptx::smem_u32(smem_raw);  // 1024-byte aligned, checked below
@@ -177,9 +182,9 @@ __global__ void __launch_bounds__((kWideFirstScatter + wide_a_stages(N_TILE)) * 
                         break;
                     ptx::tc_fence_after_sync();
                     // hands the B slab back, and with the tile's last slab the A stage
-                    ptx::umma_tile_elect(tmem_acc + static_cast<uint32_t>(h * kMmaN),
+                    ptx::umma_tile_elect(tmem_acc + static_cast<uint32_t>(j % kAccs * N_TILE + h * kMmaN),
                                          a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
-                                         b_desc0 + static_cast<uint32_t>(bs * (kBSlab >> 4)), idesc, j != 0 ? 1u : 0u,
+                                         b_desc0 + static_cast<uint32_t>(bs * (kBSlab >> 4)), idesc, j >= kAccs ? 1u : 0u,
                                          b_empty + 8u * bs, a_empty + 8u * s, h + 1 == kSlabs ? 1u : 0u);
                     if (++bs == B_STAGES) {
                         bs = 0;
@@ -204,8 +209,8 @@ __global__ void __launch_bounds__((kWideFirstScatter + wide_a_stages(N_TILE)) * 
         }
         acc_ok = __all_sync(0xFFFFFFFFu, acc_ok && (*abort_flag == 0u));
         ptx::tc_fence_after_sync();
-        accumulators_to_output<N_TILE, 32>(p, tmem_acc, 1, 0, warp & 3, lane, sw, STAGES >= 8 ? 2 : 1, S, G, g, n_idx, tile_row,
-                                           acc_ok, reinterpret_cast<float*>(smem));
+        accumulators_to_output<N_TILE, 32>(p, tmem_acc, L < kAccs ? L : kAccs, N_TILE, warp & 3, lane, sw, STAGES >= 8 ? 2 : 1, S, G,
+                                           g, n_idx, tile_row, acc_ok, reinterpret_cast<float*>(smem));
     }
 
     // ================================================================ cluster reduction and tear-down

@@ -78,6 +78,30 @@ def test_chosen_where_it_saves_decompression(lib, oracle):
     assert_close(DeviceProblem(lib, comp, offs, B, M, N, K, 1).run(), oracle.gemm_f32(A, B), "automatic")
 
 
+def test_two_accumulators_at_256_columns(lib):
+    """As the streaming form's test of the same kind: sums of positive products, whose mean shortfall against 64-bit products
+    must not be larger than that of 128 columns per CTA, which alternate between two accumulators (allowance 1e-6: ten times
+    the 2^-11 / sqrt(12 * 2400000) that rounding to fp16 leaves)."""
+    from flash_llm_b200 import torch_op  # noqa: F401  (registers torch.ops.flashllm)
+    M, K, N = 128 * 74, 9216, 256
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(7)
+    A = torch.rand((M, K), generator=gen, device="cuda").half()
+    A *= torch.rand((M, K), generator=gen, device="cuda") >= 0.8
+    B = torch.rand((N, K), generator=gen, device="cuda").half()
+    want = torch.cat([B.double() @ A[r:r + 1024].double().T for r in range(0, M, 1024)], dim=1)
+    words, offs = torch.ops.flashllm.encode(A)
+    share = {}
+    try:
+        for path, width in ((lib.api.PATH_WIDE, 2), (lib.api.PATH_DIRECT, 0)):
+            lib.set_plan(path=path, producers=width, cluster_k=1)
+            share[path] = float(((want - torch.ops.flashllm.spmm(words, offs, B, M).double()) / want).mean())
+    finally:
+        lib.set_plan()
+    assert lib.consume_status() == 0
+    assert abs(share[lib.api.PATH_WIDE]) <= abs(share[lib.api.PATH_DIRECT]) + 1e-6, share
+
+
 def test_malformed_offsets_are_reported_not_followed(lib, oracle, pinned):
     M, K, N = 384, 64 * 20, 256
     A, B = random_problem(lib, M, K, N, 0.8, 31)
