@@ -133,7 +133,8 @@ __global__ void __launch_bounds__(kEncodeWarps * 32)
 // 1024 groups at a time: it scans the groups' sums and then runs over their entries.
 __global__ void __launch_bounds__(1024) csl_scan_kernel(int* __restrict__ offs, int tiles, unsigned int* status)
 {
-    ptx::grid_launch_dependents();
+    // No launch_dependents, here and in the kernels that end an encoding: an SpMM with launch overlap on that follows reads
+    // offsets and words before its own wait.
     ptx::grid_dependency_wait();
     __shared__ int       s_before[1024];  // sum of the groups before this one
     __shared__ long long s_warp[32];
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(1024) csl_scan_kernel(int* __restrict__ offs, 
         offs[0]         = 0;
         offs[tiles + 1] = static_cast<int>(done);
     }
+    __threadfence();  // the offsets are in place for whatever starts once this grid has ended
 }
 
 // Step 2, reordered format, tiles with buckets of any height: counts, tabulates the per-height terms of q in shared
@@ -320,8 +322,7 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
                                                                                            uint32_t* __restrict__ out,
                                                                                            unsigned int* status)
 {
-    ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();
+    ptx::grid_dependency_wait();  // no launch_dependents (see csl_scan_kernel)
     // spare rows in front: words beyond kListRows land there
     __shared__ uint32_t s_list[kPackWarps][(kListRows + kSpareRows) * 32];
     static_assert(sizeof(s_list[0]) >= kHeightEntries * (sizeof(uint32_t) + sizeof(uint16_t)), "tables of a tall tile");
@@ -464,6 +465,7 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
         for (int i = repeat - 1; i >= 0; --i, q += 128)
             put(i * 32 + lane, make_uint4(pick(q + 96), pick(q + 64), pick(q + 32), pick(q)));
     }
+    __threadfence();  // the words are in place for whatever starts once this grid has ended
 }
 
 // Step 2, scan-order format (reference csrc/SpMM_API.cu:441-476): non-zeros in row-major order, with the first
@@ -476,8 +478,7 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_scan_kernel(const 
                                                                           uint32_t* __restrict__ out,
                                                                           unsigned int* status)
 {
-    ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();
+    ptx::grid_dependency_wait();  // no launch_dependents (see csl_scan_kernel)
     const int lane = threadIdx.x & 31;
     const int t    = blockIdx.x * kEncodeWarps + (threadIdx.x >> 5);
     if (t >= tiles)
@@ -523,6 +524,7 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_scan_kernel(const 
             dst[pos] = v1 | (static_cast<uint32_t>(r * kTileK + ((2 * lane + 1) ^ x)) << 16);
         emitted += __popc(b0) + __popc(b1);
     }
+    __threadfence();
 }
 
 }  // namespace flashllm

@@ -283,12 +283,14 @@ int FlashLLM_SpMM_SplitK_NoAlloc(void*       stream,
  * C[i] = fp16(sum_s float(Workspace[s*M*N + i])). */
 int FlashLLM_SplitK_Reduction(void* stream, void* C, const void* Reduction_Workspace, int M, int N, int Split_K);
 
-/* Launch overlap (no counterpart in the reference).  With enable != 0, SpMM kernels are launched with programmatic
- * stream serialisation: a kernel's CTAs may start while the previous kernel of the stream is still draining.  They
- * set up, and stream Compressed_A / TileOffsets, right away; B is read and C / the workspace written only after
- * everything enqueued before has completed.  The caller thereby promises that Compressed_A and TileOffsets of a call
- * are not being produced by work still running in the same stream (weights resident before the calls, the inference
- * case).  Off by default.  Process-wide. */
+/* Launch overlap (no counterpart in the reference).  Every kernel of this library is launched with programmatic stream
+ * serialisation: its CTAs may start and set up while the previous kernel of the stream is still draining, and wait for the
+ * end of everything enqueued before them before they touch any data.  With enable != 0 SpMM kernels stream Compressed_A and
+ * TileOffsets without that wait; B is read and C / the workspace written only after it, as ever.  The caller thereby
+ * promises that Compressed_A and TileOffsets of a call are not being produced by work still running in the same stream
+ * (weights resident before the calls, the inference case).  FlashLLM_EncodeOnDevice_TileOffsets and _Pack may directly
+ * precede the SpMM all the same: their last kernels let no kernel start before they have ended.  Off by default.
+ * Process-wide. */
 void FlashLLM_SetLaunchOverlap(int enable);
 
 /* Gives back the current device's scratch memory (about 20 MB for each of at most 8 streams).  An SpMM that runs as a

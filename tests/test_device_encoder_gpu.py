@@ -68,6 +68,35 @@ def test_device_encoded_buffers_feed_the_kernel(lib, oracle):
     assert_close(C.cpu().numpy(), oracle.gemm_f32(A.numpy(), B.numpy()), "device-encoded SpMM")
 
 
+@pytest.mark.parametrize("reorder", [1, 0])
+def test_an_overlapped_spmm_right_behind_the_encoder(lib, oracle, reorder):
+    """With launch overlap on an SpMM reads its words before it waits for its predecessors; enqueued right behind the encoder,
+    into buffers that still hold another matrix of another sparsity, it must find the new words and offsets."""
+    from helpers import assert_close
+    M, K, N = 4096, 2048, 16
+    B = lib.synthetic.dense_uniform_matrix(N, K, 10)
+    As = [lib.synthetic.sparse_uniform_matrix(M, K, s, seed) for seed, s in ((11, 0.8), (12, 0.6))]
+    wants = [oracle.gemm_f32(A.numpy(), B.numpy()) for A in As]
+    As, B_d = [A.cuda() for A in As], B.cuda()
+    words = torch.zeros(M * K, dtype=torch.int32, device="cuda")
+    offs = torch.zeros((M // 128) * (K // 64) + 2, dtype=torch.int32, device="cuda")
+    outs = [torch.empty((N, M), dtype=torch.float16, device="cuda") for _ in range(12)]
+    L, stream = lib.library(), torch.cuda.current_stream().cuda_stream
+    lib.set_launch_overlap(True)
+    try:
+        for i, C in enumerate(outs):
+            A = As[i % 2]
+            assert L.FlashLLM_EncodeOnDevice_TileOffsets(stream, A.data_ptr(), M, K, offs.data_ptr()) == 0
+            assert L.FlashLLM_EncodeOnDevice_Pack(stream, A.data_ptr(), M, K, offs.data_ptr(), words.data_ptr(), reorder) == 0
+            lib.SpMM_SplitK_API(stream, None, words.data_ptr(), offs.data_ptr(), B_d.data_ptr(), C.data_ptr(), M, N, K, None, 1)
+        torch.cuda.synchronize()
+    finally:
+        lib.set_launch_overlap(False)
+    assert lib.consume_status() == 0
+    for i, C in enumerate(outs):
+        assert_close(C.cpu().numpy(), wants[i % 2], f"call {i}")
+
+
 @pytest.mark.parametrize("shift", [0, 2])
 def test_tiles_of_every_density_and_special_values(lib, shift):
     """Tiles on both sides of the density that has a kernel of its own (1088 vectors), sparse ones with a full bucket (a warp's
