@@ -4,7 +4,7 @@
 // the compressed words never pass through shared memory as a stream:
 //
 //   * Every scatter warp owns one 16 KB stage and takes every NSW-th tile of the CTA's K range.  It fetches the words
-//     of its NEXT tile straight from global memory into registers (ld.global.nc, 16 bytes per lane and instruction,
+//     of its NEXT tile straight from global memory into registers (ld.global, 16 bytes per lane and instruction,
 //     the reference's LDG.128 scheme, csrc/SpMM_Kernel.cuh:17-62) right after it has published the current one, so
 //     a whole hand-back period of the stage (several microseconds) hides the memory latency, and as many tiles as
 //     there are scatter warps are in flight per CTA.  No copy ring, no producer warps, no per-chunk barriers.
@@ -16,17 +16,11 @@
 
 namespace flashllm {
 
-__device__ __forceinline__ uint4 ldg_stream16(const uint4* ptr)
-{
-    uint4 v;
+// Words are read once, so they get no line of L1; not through the read-only path (ld.global.nc): a kernel is launched before
+// its predecessors have ended, and that path is for data that nobody writes in a kernel's lifetime.
 #ifndef FLASHLLM_LDG_FLAVOUR
-#define FLASHLLM_LDG_FLAVOUR "ld.global.nc.L1::no_allocate.v4.u32"
+#define FLASHLLM_LDG_FLAVOUR "ld.global.L1::no_allocate.v4.u32"
 #endif
-    asm volatile(FLASHLLM_LDG_FLAVOUR " {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(ptr));
-    return v;
-}
 
 // Straight-line forms for the scatter warps' per-tile path.  That path is bound by the number of instructions and
 // branches a warp has to get through per tile, so a row of 32 vectors is loaded / scattered by predicated instructions

@@ -1044,11 +1044,14 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 #endif
 }
 
+// (Kernels take no __restrict__ pointers: their data may still be written when they start, and the compiler may load what it
+// knows to be read-only through the non-coherent path, or before the wait at the top.)
+//
 // Sums the fp32 partial matrices this library parks in the caller's workspace when workspace_k > 1 and rounds once:
 // C[i] = fp16(sum_s ws[s*count + i]); four outputs per thread.
-__global__ void splitk_reduce_f32_kernel(half* __restrict__ C, const float* __restrict__ ws, long long count, int parts,
-                                         const half* __restrict__ bias, int M, int activation,
-                                         const half* __restrict__ residual)
+__global__ void splitk_reduce_f32_kernel(half* C, const float* ws, long long count, int parts,
+                                         const half* bias, int M, int activation,
+                                         const half* residual)
 {
     ptx::grid_launch_dependents();  // the next SpMM may begin streaming its weights
     ptx::grid_dependency_wait();    // the partial matrices come from the SpMM launched just before
@@ -1075,7 +1078,7 @@ __global__ void splitk_reduce_f32_kernel(half* __restrict__ C, const float* __re
 
 // The reference's reduction semantics, kept as an entry point of its own (reference csrc/Reduction_Kernel.cuh:24-45):
 // C[i] = fp16(sum_s float(ws[s*count + i])) over fp16 partial matrices; eight outputs per thread, 16-byte accesses.
-__global__ void splitk_reduce_kernel(half* __restrict__ C, const half* __restrict__ ws, long long count, int parts)
+__global__ void splitk_reduce_kernel(half* C, const half* ws, long long count, int parts)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
@@ -1119,11 +1122,11 @@ constexpr unsigned kStatusPeerWaitExpired = 32u;  // a GPU of the group did not 
 // one polls).  With 0 the flags are the only dependency: this GPU's sender is the launch right before, all of whose
 // CTAs are resident or finished by the time a dependent launch starts, and the other senders run on other GPUs; the
 // kernel then neither waits for its predecessor to drain nor for its peer stores to be flushed.
-__global__ void allreduce_sum_kernel(half* __restrict__ C, const float* slots, long long slot_stride,
+__global__ void allreduce_sum_kernel(half* C, const float* slots, long long slot_stride,
                                      const unsigned int* flags, int flag_stride, unsigned int epoch, int world,
                                      int flags_per_tile, int tile_rows, int n_tile, long long count,
-                                     const half* __restrict__ bias, int M, int activation,
-                                     const half* __restrict__ residual, unsigned int* status,
+                                     const half* bias, int M, int activation,
+                                     const half* residual, unsigned int* status,
                                      unsigned long long wait_limit_ns, int stream_ordered)
 {
 #ifdef FLASHLLM_CTA_TIMES

@@ -82,7 +82,7 @@ __device__ __forceinline__ const uint16_t* tile_start(const uint16_t* A, int K, 
 constexpr int kCountTiles = kEncodeWarps * 4;
 
 __global__ void __launch_bounds__(kEncodeWarps * 32)
-    csl_count_kernel(const uint16_t* __restrict__ A, int K, int tiles, int k_tiles, int* __restrict__ offs)
+    csl_count_kernel(const uint16_t* A, int K, int tiles, int k_tiles, int* offs)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
@@ -100,13 +100,13 @@ __global__ void __launch_bounds__(kEncodeWarps * 32)
         if ((reinterpret_cast<uintptr_t>(A) & 15u) == 0) {
 #pragma unroll 16
             for (int r = 0; r < kTileM; ++r)
-                count(__ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * K)));
+                count(*reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * K));
         }
         else {  // A is 4-byte aligned
 #pragma unroll 4
             for (int r = 0; r < kTileM; ++r) {
                 const uint32_t* row = reinterpret_cast<const uint32_t*>(src + static_cast<size_t>(r) * K);
-                count(make_uint4(__ldg(row), __ldg(row + 1), __ldg(row + 2), __ldg(row + 3)));
+                count(make_uint4(row[0], row[1], row[2], row[3]));
             }
         }
     }
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kEncodeWarps * 32)
 
 // Step 1b: adds to every entry the sums of the groups before its own; offs[0] = 0, offs[tiles + 1] = offs[tiles].  One CTA,
 // 1024 groups at a time: it scans the groups' sums and then runs over their entries.
-__global__ void __launch_bounds__(1024) csl_scan_kernel(int* __restrict__ offs, int tiles, unsigned int* status)
+__global__ void __launch_bounds__(1024) csl_scan_kernel(int* offs, int tiles, unsigned int* status)
 {
     // No launch_dependents, here and in the kernels that end an encoding: an SpMM with launch overlap on that follows reads
     // offsets and words before its own wait.
@@ -258,12 +258,12 @@ __device__ __noinline__ void pack_tall_tile(const uint16_t* tile, int K, int vec
 // more warps per SM than that kernel's shared memory allows.  Persistent, so that it costs 4 to 9 us where there are none.
 constexpr int kListVectors = 1088;  // 136 words to a bucket: hardly ever one above 164
 
-__global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_dense_kernel(const uint16_t* __restrict__ A,
+__global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_dense_kernel(const uint16_t* A,
                                                                            int K,
                                                                            int tiles,
                                                                            int k_tiles,
-                                                                           const int* __restrict__ offs,
-                                                                           uint32_t* __restrict__ out,
+                                                                           const int* offs,
+                                                                           uint32_t* out,
                                                                            unsigned int* status)
 {
     ptx::grid_launch_dependents();
@@ -301,7 +301,7 @@ __device__ __forceinline__ void load_bucket(uint32_t (&pair)[kTileM], const uint
 {
 #pragma unroll
     for (int r = 0; r < kTileM; ++r) {
-        pair[r] = __ldg(reinterpret_cast<const uint32_t*>(tile + ((2 * lane) ^ ((r & 7) << 3))));
+        pair[r] = *reinterpret_cast<const uint32_t*>(tile + ((2 * lane) ^ ((r & 7) << 3)));
         tile += K;
     }
 }
@@ -314,12 +314,12 @@ __device__ __forceinline__ void prefetch_tile(const uint16_t* tile, int K, int l
         asm volatile("prefetch.global.L2 [%0];" ::"l"(tile + static_cast<size_t>(r + lane) * K));
 }
 
-__global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reorder_kernel(const uint16_t* __restrict__ A,
+__global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reorder_kernel(const uint16_t* A,
                                                                                            int K,
                                                                                            int tiles,
                                                                                            int k_tiles,
-                                                                                           const int* __restrict__ offs,
-                                                                                           uint32_t* __restrict__ out,
+                                                                                           const int* offs,
+                                                                                           uint32_t* out,
                                                                                            unsigned int* status)
 {
     ptx::grid_dependency_wait();  // no launch_dependents (see csl_scan_kernel)
@@ -470,24 +470,9 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
 
 // Step 2, scan-order format (reference csrc/SpMM_API.cu:441-476): non-zeros in row-major order, with the first
 // `pads` zero-testing cells of the tile kept in place as padding words (their bits preserved).
-__global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_scan_kernel(const uint16_t* __restrict__ A,
-                                                                          int K,
-                                                                          int tiles,
-                                                                          int k_tiles,
-                                                                          const int* __restrict__ offs,
-                                                                          uint32_t* __restrict__ out,
-                                                                          unsigned int* status)
+__device__ __forceinline__ void pack_scan_tile(const uint16_t* __restrict__ tile, int K, int words, uint32_t* __restrict__ dst,
+                                               int lane, unsigned int* status)
 {
-    ptx::grid_dependency_wait();  // no launch_dependents (see csl_scan_kernel)
-    const int lane = threadIdx.x & 31;
-    const int t    = blockIdx.x * kEncodeWarps + (threadIdx.x >> 5);
-    if (t >= tiles)
-        return;
-    const uint16_t* tile  = A + static_cast<size_t>(t / k_tiles) * kTileM * K + static_cast<size_t>(t % k_tiles) * kTileK;
-    const int       first = offs[t];
-    const int       words = (offs[t + 1] - first) * kVectorWords;
-    uint32_t*       dst   = out + static_cast<size_t>(first) * kVectorWords;
-
     int nnz = 0;
 #pragma unroll 8
     for (int r = 0; r < kTileM; ++r) {
@@ -524,6 +509,24 @@ __global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_scan_kernel(const 
             dst[pos] = v1 | (static_cast<uint32_t>(r * kTileK + ((2 * lane + 1) ^ x)) << 16);
         emitted += __popc(b0) + __popc(b1);
     }
+}
+
+__global__ void __launch_bounds__(kEncodeWarps * 32) csl_pack_scan_kernel(const uint16_t* A,
+                                                                          int K,
+                                                                          int tiles,
+                                                                          int k_tiles,
+                                                                          const int* offs,
+                                                                          uint32_t* out,
+                                                                          unsigned int* status)
+{
+    ptx::grid_dependency_wait();  // no launch_dependents (see csl_scan_kernel)
+    const int lane = threadIdx.x & 31;
+    const int t    = blockIdx.x * kEncodeWarps + (threadIdx.x >> 5);
+    if (t >= tiles)
+        return;
+    const int first = offs[t];
+    pack_scan_tile(tile_start(A, K, k_tiles, t), K, (offs[t + 1] - first) * kVectorWords,
+                   out + static_cast<size_t>(first) * kVectorWords, lane, status);
     __threadfence();
 }
 

@@ -1,0 +1,38 @@
+"""Kernels are launched before their predecessors on the stream have ended and wait at their top, or, for an SpMM's weights
+with launch overlap on, not at all.  That is only sound for ordinary loads: the read-only path (ld.global.nc, __ldg, and what
+the compiler makes of const __restrict__ kernel parameters) is for data that nobody writes during the kernel's lifetime.  A
+violation is a race that hardly ever shows, so the sources are checked."""
+import glob
+import os
+import re
+
+import pytest
+
+from conftest import ROOT
+
+SOURCES = sorted(glob.glob(os.path.join(ROOT, "flash-llm_b200", "csrc", "*.cu*")))
+
+
+def _code(path):
+    with open(path) as f:
+        text = f.read()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=[os.path.basename(p) for p in SOURCES])
+def test_no_load_takes_the_read_only_path(path):
+    code = _code(path)
+    assert not re.search(r"\bld\.global\.nc\b|__ldg\s*\(", code)
+    for kernel in re.finditer(r"__global__[^;{]*\{", code):
+        assert "__restrict__" not in kernel.group(0), kernel.group(0)
+
+
+def test_every_kernel_waits_for_its_predecessors():
+    kernels = 0
+    for path in SOURCES:
+        code = _code(path)
+        for kernel in re.finditer(r"__global__[^;{]*\{", code):
+            end = code.index("\n}\n", kernel.end())
+            assert "grid_dependency_wait()" in code[kernel.end():end], kernel.group(0)
+            kernels += 1
+    assert kernels >= 12
