@@ -32,6 +32,7 @@ from .api import (  # noqa: F401
     read_rank_lists,
     read_sparse_matrix_bin_files,
     release_scratch,
+    release_stream_scratch,
     set_launch_overlap,
     set_plan,
     splitk_reduction,

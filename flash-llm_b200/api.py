@@ -97,6 +97,8 @@ def library() -> C.CDLL:
     L.FlashLLM_SplitK_Reduction.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int]
     L.FlashLLM_ReleaseScratch.restype = C.c_int
     L.FlashLLM_ReleaseScratch.argtypes = []
+    L.FlashLLM_ReleaseStreamScratch.restype = C.c_int
+    L.FlashLLM_ReleaseStreamScratch.argtypes = [C.c_void_p]
     L.FlashLLM_SetLaunchOverlap.argtypes = [C.c_int]
     L.FlashLLM_SetPlan.argtypes = [_i32p, C.c_int]
     L.FlashLLM_GetPlan.restype = C.c_int
@@ -362,6 +364,12 @@ def set_launch_overlap(enable: bool) -> None:
 def release_scratch() -> None:
     """Free the current device's scratch of the streaming kernel (allocated per stream on first use); synchronises."""
     _check(library().FlashLLM_ReleaseScratch(), "ReleaseScratch")
+
+
+def release_stream_scratch(stream: int) -> None:
+    """Let another stream have the scratch that the streaming kernel keeps for ``stream``, before that stream is destroyed;
+    synchronises the stream."""
+    _check(library().FlashLLM_ReleaseStreamScratch(stream), "ReleaseStreamScratch")
 
 
 PLAN_FIELDS = ("cluster_k", "workspace_k", "a_stages", "b_stages", "b_batch", "ring_slots", "chunk_vectors",

@@ -50,14 +50,19 @@ constexpr int kMaxDevices = 64;
 
 // Scratch of the streaming form: one counter per tile row and two fp32 [N][128] parts per CTA of the largest grid at the
 // largest N it takes.  Launches on one stream follow one another, so a scratch belongs to a stream (by its unique id: a
-// handle may be reused while its old stream's work still runs).  It is allocated at the stream's first such call and kept;
-// at most kScratchStreams per device, further streams run the other forms.  FlashLLM_ReleaseScratch gives it back.
+// handle may be reused while its old stream's work still runs).  It is allocated at the stream's first such call and kept,
+// at most kScratchStreams per device; further streams run the other forms.  Nobody tells the library that a stream has been
+// destroyed or that its work has ended (a word that every CTA stores at its end made every launch 0.3 us longer, an event
+// behind every launch more), so a place stays its stream's until FlashLLM_ReleaseStreamScratch or FlashLLM_ReleaseScratch.
 constexpr int    kScratchStreams = 8, kScratchRows = 4096, kScratchCtas = 2 * 160, kScratchMaxN = 64;
 constexpr size_t kScratchBytes   = kScratchRows * sizeof(unsigned int)
                                  + size_t(2) * kScratchCtas * kScratchMaxN * kTileM * sizeof(float);
+// Calls of streams without a scratch between an allocation that failed and the next one.
+constexpr unsigned int kScratchRetryCalls = 256;
 
 struct StreamScratch {
     unsigned long long stream_id = 0;
+    bool               taken     = false;  // by the stream of that id; a place that was given back keeps its memory
     unsigned char*     memory    = nullptr;
 };
 
@@ -71,12 +76,21 @@ struct DeviceState {
     unsigned int*  tile_counters   = nullptr;  // device address of g_tile_counters on this device
     int            counter_streams = 0;        // streams that own a counter set so far
     cudaStream_t   counter_stream[kCounterSets] = {nullptr};
-    int            scratch_streams = 0;
     StreamScratch  scratch[kScratchStreams];
+    unsigned int   scratch_retry = 0;  // calls to go until an allocation that failed is tried again
 };
 
-// The scratch of `stream` on this device, allocated on first use; nullptr while the stream is being captured (a graph may
-// be replayed on any stream), when all places are taken, or when memory is short.
+// The place of the stream with this id, or nullptr.
+static StreamScratch* scratch_with_id(DeviceState* st, unsigned long long id)
+{
+    for (StreamScratch& place : st->scratch)
+        if (place.taken && place.stream_id == id)
+            return &place;
+    return nullptr;
+}
+
+// The scratch of `stream` on this device, set up on first use; nullptr while the stream is being captured (a graph may be
+// replayed on any stream), when all places are taken, or when memory is short.
 static unsigned char* scratch_of_stream(DeviceState* st, cudaStream_t stream)
 {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -87,27 +101,35 @@ static unsigned char* scratch_of_stream(DeviceState* st, cudaStream_t stream)
         return nullptr;
     }
     std::lock_guard<std::mutex> lock(st->mutex);
-    for (int i = 0; i < st->scratch_streams; ++i)
-        if (st->scratch[i].stream_id == id)
-            return st->scratch[i].memory;
-    if (st->scratch_streams >= kScratchStreams)
+    if (StreamScratch* mine = scratch_with_id(st, id))
+        return mine->memory;
+    StreamScratch* place = nullptr;  // a free one, with memory if there is such
+    for (StreamScratch& other : st->scratch)
+        if (!other.taken && (place == nullptr || (place->memory == nullptr && other.memory != nullptr)))
+            place = &other;
+    if (place == nullptr)
         return nullptr;
-    // Another thread may be capturing: allocate in relaxed mode, and clear the counters in this stream's own order.
-    unsigned char*        memory = nullptr;
-    cudaStreamCaptureMode mode   = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    bool ok = cudaMalloc(reinterpret_cast<void**>(&memory), kScratchBytes) == cudaSuccess;
-    if (ok && cudaMemsetAsync(memory, 0, kScratchRows * sizeof(unsigned int), stream) != cudaSuccess) {
-        cudaFree(memory);
-        ok = false;
+    if (place->memory == nullptr && st->scratch_retry > 0) {
+        --st->scratch_retry;
+        return nullptr;
     }
+    // Another thread may be capturing: allocate in relaxed mode, and clear the counters in this stream's own order.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (place->memory == nullptr && cudaMalloc(reinterpret_cast<void**>(&place->memory), kScratchBytes) != cudaSuccess) {
+        place->memory     = nullptr;
+        st->scratch_retry = kScratchRetryCalls;
+    }
+    const bool ok = place->memory != nullptr
+                    && cudaMemsetAsync(place->memory, 0, kScratchRows * sizeof(unsigned int), stream) == cudaSuccess;
     cudaThreadExchangeStreamCaptureMode(&mode);
     if (!ok) {
         cudaGetLastError();
         return nullptr;
     }
-    st->scratch[st->scratch_streams++] = {id, memory};
-    return memory;
+    place->stream_id = id;
+    place->taken     = true;
+    return place->memory;
 }
 
 // The counter set of `stream` on this device, or nullptr when all sets are taken by other streams.
@@ -1126,9 +1148,27 @@ int FlashLLM_ReleaseScratch(void)
     if ((err = cudaDeviceSynchronize()) != cudaSuccess)
         return static_cast<int>(err);
     std::lock_guard<std::mutex> lock(st->mutex);
-    for (int i = 0; i < st->scratch_streams; ++i)
-        cudaFree(st->scratch[i].memory);
-    st->scratch_streams = 0;
+    for (StreamScratch& place : st->scratch) {
+        cudaFree(place.memory);
+        place = StreamScratch();
+    }
+    st->scratch_retry = 0;
+    return 0;
+}
+
+int FlashLLM_ReleaseStreamScratch(void* stream)
+{
+    cudaError_t  err = cudaSuccess;
+    DeviceState* st  = device_state(&err);
+    if (!st)
+        return static_cast<int>(err);
+    const cudaStream_t s  = static_cast<cudaStream_t>(stream);
+    unsigned long long id = 0;
+    if ((err = cudaStreamGetId(s, &id)) != cudaSuccess || (err = cudaStreamSynchronize(s)) != cudaSuccess)
+        return static_cast<int>(err);
+    std::lock_guard<std::mutex> lock(st->mutex);
+    if (StreamScratch* place = scratch_with_id(st, id))
+        place->taken = false;
     return 0;
 }
 

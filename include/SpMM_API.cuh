@@ -293,12 +293,18 @@ int FlashLLM_SplitK_Reduction(void* stream, void* C, const void* Reduction_Works
  * Process-wide. */
 void FlashLLM_SetLaunchOverlap(int enable);
 
-/* Gives back the current device's scratch memory (about 20 MB for each of at most 8 streams).  An SpMM that runs as a
- * persistent grid over all tiles of the matrix parks the parts of tile rows shared between CTAs there; it is allocated at
- * a stream's first such call (never while the stream is being captured, nor by FlashLLM_SpMM_SplitK_NoAlloc: those calls
- * run the forms that need none).  Synchronises the device; no call may be made concurrently from another thread; the next
- * call allocates again. */
+/* Scratch memory of the library (21 MB for each of at most 8 streams of a device).  An SpMM that runs as a persistent grid
+ * over all tiles of the matrix parks the parts of tile rows shared between CTAs there; it is allocated at a stream's first
+ * such call.  A stream keeps its scratch when it is destroyed: a host that creates streams as it goes gives the scratch of
+ * each back before it destroys it.  Calls that get none run the forms that need none, which add up in another order and may
+ * differ in the last bit: calls of a stream that is being captured, of a ninth stream, of FlashLLM_SpMM_SplitK_NoAlloc, and
+ * where memory is short (tried again 256 calls later).
+ *
+ * FlashLLM_ReleaseScratch frees all of the current device's; synchronises the device; no call may be made concurrently from
+ * another thread; the next call allocates again.  FlashLLM_ReleaseStreamScratch lets another stream have the scratch of
+ * `stream`; synchronises that stream, on which no call may be made concurrently; its next call takes a scratch again. */
 int FlashLLM_ReleaseScratch(void);
+int FlashLLM_ReleaseStreamScratch(void* stream);
 
 /* Tuning hook replacing the reference's compile-time TilingConfig<...> choice (csrc/TilingConfig.h:36-52,
  * csrc/SpMM_API.cu:79-118): fixes launch-plan fields for subsequent calls from this process.  `fields` holds up to
@@ -330,8 +336,9 @@ int FlashLLM_ReleaseScratch(void);
  * FlashLLM_SetPlan(nullptr, 0) restores automatic choice. */
 void FlashLLM_SetPlan(const int* fields, int count);
 
-/* Describes the plan the next SpMM call with these sizes would use: out[0..10] as above, out[11] = dynamic shared
- * memory in bytes; `count` = entries available in `out`. */
+/* Describes the plan the next SpMM call with these sizes would use, on a stream that has or gets scratch (see
+ * FlashLLM_ReleaseScratch): out[0..10] as above, out[11] = dynamic shared memory in bytes; `count` = entries available in
+ * `out`. */
 int FlashLLM_GetPlan(int M, int N, int K, int Split_K, int* out, int count);
 
 /* Reads and clears the device-side status word of the current device (synchronises the device).  0 = no kernel of

@@ -90,19 +90,59 @@ def test_output_epilogues(lib, oracle, streaming, bias, relu, residual):
         assert_close(C.view(N, M).cpu().numpy(), want, f"bias={bias} relu={relu} residual={residual} shift={shift}")
 
 
+class _Forms:
+    """One problem that is streamed, with the bits of its result in the streaming and in the row form (they differ, since the
+    forms add up in another order)."""
+
+    def __init__(self, lib, oracle, seed):
+        self.lib = lib
+        M, K, N = 128 * 100, 64 * 40, 16
+        A, B = random_problem(lib, M, K, N, 0.8, seed)
+        comp, offs, _ = lib.InitSparseMatrixA_API(A)
+        self.want = oracle.gemm_f32(A, B)
+        assert lib.get_plan(M, N, K, 1)["path"] == lib.api.PATH_STREAM, "this case is meant to be streamed"
+        self.prob = DeviceProblem(lib, comp, offs, B, M, N, K, 1)
+        lib.release_scratch()
+        self.streamed = self.prob.run().copy()
+        lib.set_plan(path=lib.api.PATH_DIRECT)
+        self.by_rows = self.prob.run().copy()
+        lib.set_plan()
+        lib.release_scratch()
+        assert not np.array_equal(self.streamed, self.by_rows)
+
+    def enqueue(self, stream, C=None):
+        p = self.prob
+        self.lib.SpMM_SplitK_API(stream.cuda_stream, None, p.comp.data_ptr(), p.offs.data_ptr(), p.B.data_ptr(),
+                                 (p.C if C is None else C).data_ptr(), p.M, p.N, p.K, None, 1)
+
+
 def test_streams_without_a_scratch_of_their_own_run_another_form(lib, oracle):
     """At most eight streams hold scratch; calls on further streams, and after the scratch was given back, are still right."""
-    M, K, N = 128 * 100, 64 * 40, 16
-    A, B = random_problem(lib, M, K, N, 0.8, 23)
-    comp, offs, _ = lib.InitSparseMatrixA_API(A)
-    want = oracle.gemm_f32(A, B)
-    assert lib.get_plan(M, N, K, 1)["path"] == lib.api.PATH_STREAM, "this case is meant to be streamed"
-    prob = DeviceProblem(lib, comp, offs, B, M, N, K, 1)
-    for s in [torch.cuda.current_stream()] + [torch.cuda.Stream() for _ in range(12)]:
+    f = _Forms(lib, oracle, 23)
+    for i, s in enumerate([torch.cuda.current_stream()] + [torch.cuda.Stream() for _ in range(12)]):
         with torch.cuda.stream(s):
-            assert_close(prob.run(), want, "one of many streams")
+            got = f.prob.run()
+        assert_close(got, f.want, "one of many streams")
+        assert np.array_equal(got, f.streamed if i < 8 else f.by_rows), i
     lib.release_scratch()
-    assert_close(prob.run(), want, "after the scratch was released")
+    assert np.array_equal(f.prob.run(), f.streamed), "after the scratch was released"
+
+
+def test_streams_that_come_and_go_give_their_scratch_back(lib, oracle):
+    """More streams than places, each giving its scratch back at its end, right behind work that it has not waited for."""
+    f = _Forms(lib, oracle, 24)
+    outs = [torch.full_like(f.prob.C, float("nan")) for _ in range(20)]
+    torch.cuda.synchronize()
+    for C in outs:
+        stream = torch.cuda.Stream()
+        for _ in range(5):
+            f.enqueue(stream, C)
+        lib.release_stream_scratch(stream.cuda_stream)
+        assert stream.query(), "waits for the stream's work"
+    for C in outs:
+        assert np.array_equal(C.cpu().numpy(), f.streamed)
+    lib.release_stream_scratch(torch.cuda.Stream().cuda_stream)  # one that has none
+    assert lib.consume_status() == 0
 
 
 def test_a_captured_call_needs_no_scratch(lib, oracle):
