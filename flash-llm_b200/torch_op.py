@@ -35,7 +35,7 @@ _LIB.define("spmm_epilogue(Tensor compressed, Tensor tile_offsets, Tensor B, int
 def _load_operators() -> None:
     """Registers the CUDA implementations and binds them to the library build that :mod:`api` has loaded."""
     if not os.path.exists(OPERATORS_PATH):
-        raise api.FlashLLMError(f"{OPERATORS_PATH} is missing: build it with `make -C flash-llm_b200/csrc` "
+        raise api.FlashLLMError(f"{OPERATORS_PATH} is missing: build it with `make -C flash-llm_b200/csrc all operators` "
                                 "(or __graft_entry__.build()); there is no fallback implementation")
     library = api.library()
     torch.ops.load_library(OPERATORS_PATH)
@@ -46,7 +46,18 @@ def _load_operators() -> None:
                                                      library.FlashLLM_EncodeOnDevice_Pack)), api.FlashLLMError)
 
 
-_load_operators()
+try:
+    _load_operators()
+except (api.FlashLLMError, OSError) as _error:
+    # Schemas and shape inference work without the library (a build of torch without CUDA, a host that only traces);
+    # whoever runs an operator is told.
+    _reason = str(_error)
+
+    def _refuse_cuda(*args, **kwargs):
+        raise api.FlashLLMError(f"the flashllm operators could not be loaded: {_reason}")
+
+    for _name in ("encode", "spmm", "spmm_epilogue"):
+        _LIB.impl(_name, _refuse_cuda, "CUDA")
 
 
 def _refuse_cpu(*args, **kwargs):

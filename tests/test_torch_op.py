@@ -39,6 +39,41 @@ def test_cpu_tensors_are_refused_not_computed(ops):
         ops.encode(torch.zeros((128, 64), dtype=torch.float16))
 
 
+def test_shapes_are_inferred_without_a_built_library(tmp_path):
+    """A host that only traces has neither library: the import succeeds, running an operator would say what is missing."""
+    import shutil
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    shutil.copy(f"{ROOT}/flash_llm_b200.py", tmp_path)
+    shutil.copytree(f"{ROOT}/flash-llm_b200", tmp_path / "flash-llm_b200", ignore=shutil.ignore_patterns("csrc", "__pycache__"))
+    script = ("import torch\nfrom flash_llm_b200 import torch_op\n"
+              "comp, offs = (torch.empty(n, dtype=torch.int32, device='meta') for n in (1024, 18))\n"
+              "B = torch.empty((16, 512), dtype=torch.float16, device='meta')\n"
+              "assert torch.ops.flashllm.spmm(comp, offs, B, 256).shape == (16, 256)\n"
+              "try:\n    torch_op._refuse_cuda()\nexcept torch_op.api.FlashLLMError as e:\n    print(e)\n")
+    done = subprocess.run([sys.executable, "-c", script], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+    assert "is missing: build it with" in done.stdout
+
+
+def test_the_library_builds_without_torch():
+    """The default target is what C and C++ hosts build; the operators are a target of their own."""
+    import shutil
+    import subprocess
+
+    from conftest import ROOT
+    if shutil.which("make") is None:
+        pytest.skip("no make here")
+    dry = lambda *what: subprocess.run(["make", "-n", "-B", "-C", f"{ROOT}/flash-llm_b200/csrc", *what], capture_output=True,  # noqa: E731
+                                       text=True, timeout=60)
+    everything = dry("PYTHON=/nonexistent")
+    assert everything.returncode == 0 and "libSpMM_API.so" in everything.stdout
+    assert "torch" not in everything.stdout + everything.stderr
+    assert "torch_ops.cpp" in dry("operators").stdout
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,K,N,split_k", [(512, 1024, 16, 4), (256, 2048, 64, 1), (384, 768, 128, 2)])
 def test_encode_then_spmm_matches_the_oracle(lib, oracle, ops, M, K, N, split_k):
