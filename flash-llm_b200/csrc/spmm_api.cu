@@ -376,8 +376,11 @@ constexpr int kClustersResident1[kMaxClusterK + 1] = {0, 148, 74, 45, 33, 26, 22
 // N >= 256: output columns per CTA, cluster parts S and workspace parts G by the cheapest estimate, in SM cycles; what the
 // caller pinned is kept.  A CTA of the wide form takes kTileCycles per tile (by hundreds of columns; 128 columns are the
 // register-streaming form, whose own choice follows when that is the cheapest: then cudaErrorInvalidConfiguration), 8000 to
-// 14000 around them, 2000 per 128 columns more for a cluster sum; a second kernel costs 5000 and its bytes.  From 36864x9216
-// (288 rows), 9216x9216 and 4736x7232 at N = 256, 384, 512 with every width and S: the choice is the fastest or within 4 %.
+// 14000 around them, 2000 per 128 columns more for a cluster sum; a second kernel costs 5000 and its bytes.  The cycles were
+// fitted when 384 columns had 6 + 5 stages.  With the shapes as they are, over six matrices (36864x9216, 18944x9216,
+// 9216x9216, 4736x7232, 9472x4096, 2048x8192) at N = 256, 384, 512, 640, 768 against every width at its cheapest S: the choice
+// is the fastest or within 5 %, but for N = 384 at 4736x7232 (36.7 us, 384 columns in 3 parts 34.5) and at 9472x4096 (33.1 us,
+// 256 columns uncut 29.5).
 static cudaError_t make_wide_plan(const DeviceState* st, SpmmPlan pl, const PlanOverride& ov, int tile_rows, int k_tiles, int N,
                                   int max_extra, SpmmPlan* out)
 {
@@ -514,7 +517,9 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     pl.reduce           = sends ? kReduceLastCta : (ov.v[kPlanReduce] ? ov.v[kPlanReduce] : kReduceSecondKernel);
     if (ctas_flat > kCounterTiles)
         pl.reduce = kReduceSecondKernel;
-    // (without launch overlap a second kernel costs a whole launch: small problems then do better with clusters alone)
+    // (Without launch overlap a second kernel used to cost a whole launch, and small problems did better with clusters alone.
+    // This rule and the costs below were fitted before every kernel was launched with programmatic serialisation;
+    // one_row_cost, which prices the choice against the streaming form, was fitted since.)
     const bool no_second = pl.reduce == kReduceSecondKernel && static_cast<long long>(tile_rows) * k_tiles <= 4096
                            && g_launch_overlap.load(std::memory_order_relaxed) == 0;
     int    best_s = 1, best_g = 1;

@@ -21,9 +21,10 @@
 // registers.  Issued from a branch taken by one lane, the four MMAs and the commit of a tile cost 271 cycles instead of
 // the 170 the tensor core needs for them (M128 N16 K16), which took two issuing warps to hide.
 //
-// Measured (B200, back to back on one stream, against one CTA or cluster per tile row): 27648x9216 N=8 90 % 62.8 -> 45.3 us,
-// 25600x9216 N=16 80 % 75.9 -> 53.0, 9216x36864 N=32 70 % 106.5 -> 106.2, 49152x12288 N=64 80 % 184 -> 169, 36864x9216 N=16
-// 80 % (288 rows: hardly any quantisation to begin with) 76.8 -> 73.4.  The chunks cost 0 to 0.7 % of that, at N = 64 1.3 %.
+// Measured (B200, back to back on one stream, two matrices in turn, against one CTA or cluster per tile row): 27648x9216 N=8
+// 90 % 62.2 -> 45.4 us, 2048x32768 N=16 70 % 27.0 -> 25.2, 9216x36864 N=32 70 % 100 -> 97, 49152x12288 N=64 80 % 170 -> 144,
+// 36864x9216 N=16 80 % (288 rows: hardly any quantisation to begin with) 75.9 -> 71.3.  The chunks cost 0 to 0.7 % of that, at
+// N = 64 1.3 %.
 // A CTA's share is bound by the shared-memory work of its tiles: of ~3300 cycles from one tile of a stage to the next at
 // 80 % (8 stages per SM: 412 per tile), 570 go to clearing the stage, 1140 to the 16-bit scatter stores (they wait for the
 // tensor core's operand reads), 1070 to getting the next tile's loads issued behind the other warps' stores, 430 to the

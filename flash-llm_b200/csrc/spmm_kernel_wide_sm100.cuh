@@ -10,9 +10,9 @@
 //   * warp 1, converged, issues the MMAs of a tile slab by slab; the last one hands the A stage back;
 //   * one scatter warp per A stage, as in the streaming form; they are the epilogue warps at the end.
 //
-// Measured (B200, 80 %, us per call, 128 columns per CTA -> this form): 36864x9216 N = 256 / 384 / 512: 211 / 312 / 414 ->
-// 139 / 186 / 228 (1.53 PFLOP/s of dense contraction); 9216x9216: 51 / 100 / 99 -> 42 / 59 / 66; 4736x7232: 29 / 42 / 42 ->
-// 27 / 36 / 35 (384 columns with 6 + 5 stages, before 8 + 4).  512 columns are bound by the MMAs (1024 cycles of the 1300 per tile), 256 by the shared-memory path.  Tried
+// Measured (B200, 80 %, us per call, 128 columns per CTA -> this form): 36864x9216 N = 256 / 384 / 512: 211 / 397 / 408 ->
+// 135 / 207 / 223 (1.56 PFLOP/s of dense contraction); 9216x9216: 55 / 103 / 108 -> 45 / 62 / 65; 4736x7232 at 75 %:
+// 32 / 44 / 42 -> 29 / 35 / 36.  512 columns are bound by the MMAs (1024 cycles of the 1300 per tile), 256 by the shared-memory path.  Tried
 // and not kept: CTA pairs (cta_group::2, M = 256, half of B each), 1..6 % faster where the rows come out even and up to
 // 40 % slower where K has to be cut (33 clusters of four fit the GPU, 74 of two).
 #pragma once

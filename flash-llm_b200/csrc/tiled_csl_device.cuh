@@ -10,7 +10,7 @@
 //
 // Bound by HBM: the dense matrix has to be read twice, because the size of the result is only known after the first pass.
 // 36864x9216 at 80 % (680 MB dense, 272 MB of words), both passes with the host's wait and
-// the allocation between them: 333 us (906 with every tile read twice and its words stored one by one); counting alone
+// the allocation between them: 327 us (906 with every tile read twice and its words stored one by one); counting alone
 // 113 us, 6.0 TB/s.
 #pragma once
 #include <cuda_fp16.h>
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kPackWarps * 32, kPackCtasPerSm) csl_pack_reor
         if (vectors2 <= kListVectors)
             prefetch_tile(tile_start(A, K, k_tiles, t - 2 * stride), K, lane);
         const int count = static_cast<int>(bottom - at) >> 7;
-        if (__any_sync(0xFFFFFFFFu, count > kListRows - kVectorWords)) {  // (a column that overflowed counts at least kListRows)
+        if (__any_sync(0xFFFFFFFFu, count > kListRows - kVectorWords)) {  // (a column that overflowed counts at least kListRows - 1)
             __syncwarp();
             pack_tall_tile(tile_start(A, K, k_tiles, t), K, vectors, dst, list, reinterpret_cast<uint16_t*>(list + kHeightEntries),
                            lane, status);
