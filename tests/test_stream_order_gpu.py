@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 def form(request, lib):
     """N of a form that every call is pinned to, whatever its sizes."""
     kind, N = request.param.split("-")
+    lib.release_scratch()  # a place for every stream below, whatever streams earlier tests have used
     if kind == "stream":
         lib.set_plan(path=lib.api.PATH_STREAM)
     else:
@@ -114,7 +115,6 @@ def test_two_streams_at_once(lib, form, overlap):
     Bs = [_activations(N, w.K, 30 + i) for i, w in enumerate(ws)]
     outs = [[torch.full((N, w.M), float("nan"), dtype=torch.float16, device="cuda") for _ in range(20)] for w in ws]
     streams = [torch.cuda.Stream() for _ in ws]
-    lib.release_scratch()  # places for both, whatever streams earlier tests have used
     torch.cuda.synchronize()
     lib.set_launch_overlap(overlap)
     for i in range(20):
