@@ -40,6 +40,19 @@ __device__ __forceinline__ uint32_t atom_add_acq_rel_gpu(unsigned int* ptr, uint
     return before;
 }
 
+// A look at such a counter, and what makes the stores that were counted in visible once the count has been seen.
+__device__ __forceinline__ uint32_t ld_relaxed_gpu_u32(const unsigned int* ptr)
+{
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void fence_acq_rel_gpu()
+{
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
+
 __device__ __forceinline__ uint64_t globaltimer_ns()
 {
     uint64_t t;

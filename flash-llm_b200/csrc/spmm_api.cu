@@ -308,7 +308,7 @@ static bool is_pow2(int v)
 static int stream_smem_bytes(const SpmmPlan& pl)
 {
     return kStreamStages * kDenseTileBytes + pl.b_stages * pl.b_batch * pl.n_tile * kTileK * 2
-           + 8 * (2 * kStreamStages + 4 + 2 * pl.b_stages) + 16 + 4 * pl.offsets_staged;
+           + 8 * (2 * kStreamStages + 4 + 2 * pl.b_stages) + 16 + kStreamSumBytes + 4 * pl.offsets_staged;
 }
 
 // K tiles that the tensor core adds up in one accumulator when K is cut into `parts` and every CTA alternates between two.
@@ -829,6 +829,11 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
     params.N            = N_Global;
     params.K            = K_Global;
     params.k_tiles      = K_Global / kTileK;
+    if (pl.path == kPathStream) {
+        const unsigned long long tiles = static_cast<unsigned long long>(M_Global / kTileM) * params.k_tiles;
+        params.stream_share            = ((tiles << 32) + pl.ctas - 1) / pl.ctas;
+        params.ctas_per_tile           = static_cast<float>(static_cast<double>(pl.ctas) / static_cast<double>(tiles));
+    }
 
     if (memo->has_map) {
         if (g_replace_address(&memo->map, const_cast<half*>(B)) != CUDA_SUCCESS)

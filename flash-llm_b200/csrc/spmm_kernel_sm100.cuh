@@ -52,6 +52,9 @@ struct SpmmParams {
     // partial tile, then counts itself in on the tile's counter; the CTA that finds all the others already counted adds
     // the parts up in part order and finishes the output.  Nobody waits.  Counters are zero between launches.
     unsigned int* tile_counters;
+    // Streaming form: the CTAs' shares of the tile sequence (stream_begin).
+    unsigned long long stream_share;
+    float              ctas_per_tile;
     int           push_world;
     unsigned int  push_epoch;                  // value the flags are raised to by this call
     float*        push_slot[kMaxPushWorld];    // [N][M] fp32 slot of this rank in GPU w's receive buffer
@@ -87,12 +90,16 @@ __device__ __forceinline__ half finish_output(float acc, const half* bias, int m
 // C or none of them lie inside it (`columns` left: N is 8 or a multiple of C wherever this is called).  Nothing is decided
 // per element: with a chain of branches on p's pointers for every element the 128 columns of one tile took 10 us of a
 // 13.0 us launch (128x64, N = 128), this way the launch takes 7.2 us.  Adding -0.0 leaves every value as it is.
+__device__ __forceinline__ float bias_of(const SpmmParams& p, int m)
+{
+    return p.bias != nullptr ? __half2float(p.bias[m]) : -0.0f;
+}
+
 template<int C>
-__device__ __forceinline__ void finish_columns(const SpmmParams& p, float (&v)[C], size_t at, int columns, int m)
+__device__ __forceinline__ void finish_columns(const SpmmParams& p, float (&v)[C], size_t at, int columns, float bias)
 {
     if (columns < C)
         return;
-    const float  bias = p.bias != nullptr ? __half2float(p.bias[m]) : -0.0f;
     const bool   relu = p.activation == kActRelu;
     const size_t step = static_cast<size_t>(p.M);
 #pragma unroll
@@ -392,7 +399,7 @@ __device__ __forceinline__ void accumulators_to_output(const SpmmParams& p, uint
                             p.push_slot[w][tile_off + at + static_cast<size_t>(i) * p.M] = r[i];
             }
             else
-                finish_columns<BATCH>(p, r, tile_off + at, n_valid - c0, tile_row * kTileM + row_in_tile);
+                finish_columns<BATCH>(p, r, tile_off + at, n_valid - c0, bias_of(p, tile_row * kTileM + row_in_tile));
         }
     }
     if (S == 1 && part_tile != nullptr && p.tile_counters != nullptr)

@@ -1,7 +1,7 @@
 // Load-as-Sparse / Compute-as-Dense SpMM for sm_100a, streaming form: a persistent grid over the linear tile sequence.
 //
 // The tiles of A in the order of TileOffsets (tile row by tile row, K tile by K tile) are ONE sequence, and so are their
-// words in Compressed_A.  CTA c of P takes tiles [T*c/P, T*(c+1)/P) of it, whatever rows they belong to, so every SM gets
+// words in Compressed_A.  CTA c of P takes tiles T*c/P up to T*(c+1)/P of it (to a rounding), whatever rows they belong to, so every SM gets
 // the same share of the matrix for any number of tile rows.  (One CTA per tile row leaves SMs idle whenever the rows do
 // not fill the last wave: 216 rows on 296 CTA slots, 384 rows on 296.)  A maximal run of a CTA's tiles inside one tile row
 // is a segment:
@@ -17,13 +17,19 @@
 //     on the row's counter, and whoever completes the count adds the parts up in CTA order (the same bits whoever comes
 //     last) and finishes the output.  No CTA waits for another.
 //
+// What a call takes after its last MMA is no other CTA's work any more, so it is kept short.  The first of two CTAs that share
+// a row usually finds the other's part parked, takes it into tensor memory while its own is being multiplied and finishes the
+// row without parking.  Other rows are added up when the CTA's roles are done, by all of its threads instead of the four
+// epilogue warps: a part is an L2 round trip away.  Both together, us per call: 2048x32768 N=16 70 % (19 parts a row) 26.5 ->
+// 24.5, 9216x36864 N=32 70 % (5 parts) 97.1 -> 93.4, 49152x12288 N=64 143.8 -> 141.1, 36864x9216 N=16 71.4 -> 70.6.
+//
 // The MMA-issuing warp runs converged and elects one lane inside the instruction block: operands then stay in uniform
 // registers.  Issued from a branch taken by one lane, the four MMAs and the commit of a tile cost 271 cycles instead of
 // the 170 the tensor core needs for them (M128 N16 K16), which took two issuing warps to hide.
 //
 // Measured (B200, back to back on one stream, two matrices in turn, against one CTA or cluster per tile row): 27648x9216 N=8
-// 90 % 62.2 -> 45.4 us, 2048x32768 N=16 70 % 27.0 -> 25.2, 9216x36864 N=32 70 % 100 -> 97, 49152x12288 N=64 80 % 170 -> 144,
-// 36864x9216 N=16 80 % (288 rows: hardly any quantisation to begin with) 75.9 -> 71.3.  The chunks cost 0 to 0.7 % of that, at
+// 90 % 62.2 -> 45.4 us, 2048x32768 N=16 70 % 27.0 -> 24.5, 9216x36864 N=32 70 % 100 -> 93, 49152x12288 N=64 80 % 170 -> 141,
+// 36864x9216 N=16 80 % (288 rows: hardly any quantisation to begin with) 75.9 -> 70.6.  The chunks cost 0 to 0.7 % of that, at
 // N = 64 1.3 %.
 // A CTA's share is bound by the shared-memory work of its tiles: of ~3300 cycles from one tile of a stage to the next at
 // 80 % (8 stages per SM: 412 per tile), 570 go to clearing the stage, 1140 to the 16-bit scatter stores (they wait for the
@@ -39,15 +45,24 @@ constexpr int kStreamCtasPerSm    = 2;
 constexpr int kStreamFirstScatter = 2;  // warp 0 loads B, warp 1 issues MMAs
 constexpr int kStreamFirstEpi     = kStreamFirstScatter + kStreamStages;
 constexpr int kStreamWarps        = kStreamFirstEpi + 4;
+constexpr int kStreamSumBytes     = 32;    // two rows' number, first and last CTA
+constexpr int kStreamLooks        = 4096;  // at another CTA's arrival while this one's own sums are being completed
 
-// First tile of CTA c's share, and the CTA whose share holds tile t.
-__device__ __forceinline__ int stream_begin(long long tiles, int ctas, int c)
+// First tile of CTA c's share, and the CTA whose share holds tile t.  No division, which the last part of
+// a row would wait for.  stream_share = 2^32 tiles / CTAs, rounded up: exact at c = 0 and c = CTAs.
+__host__ __device__ __forceinline__ int stream_begin(unsigned long long stream_share, int c)
 {
-    return static_cast<int>(tiles * c / ctas);
+    return static_cast<int>((stream_share * static_cast<unsigned>(c)) >> 32);
 }
-__device__ __forceinline__ int stream_owner(long long tiles, int ctas, long long t)
+__device__ __forceinline__ int stream_owner(const SpmmParams& p, int ctas, int t)
 {
-    return static_cast<int>(((t + 1) * ctas - 1) / tiles);
+    int c = static_cast<int>(t * p.ctas_per_tile);  // a guess, right to a CTA
+    c     = c < ctas ? c : ctas - 1;
+    while (stream_begin(p.stream_share, c) > t)
+        --c;
+    while (stream_begin(p.stream_share, c + 1) <= t)
+        ++c;
+    return c;
 }
 
 // Warp-collective bounded wait: every lane probes (the probe parks the warp for a while), one answer for all lanes.
@@ -157,32 +172,32 @@ struct TileStream {
     }
 };
 
-// Adds the parked parts of tile row `row` up in CTA order and finishes the output (the 128 epilogue threads).
+// Adds the parked parts of tile row `row` up in CTA order and finishes the output.  Called by all `threads` threads of a CTA
+// when its other work is done: a part is an L2 round trip away, so what counts is how many loads are in flight.
 template<int N_TILE>
 __device__ __forceinline__ void
-sum_row_parts(const SpmmParams& p, int row, int c_first, int c_last, const float* first, int tid)
+sum_row_parts(const SpmmParams& p, int row, int c_first, int c_last, const float* first, int tid, int threads)
 {
     const size_t slot     = static_cast<size_t>(N_TILE) * kTileM;
     const bool   wide_out = (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
-    // Two groups of four outputs per thread and five parts at a time: ten 16-byte loads in flight (a part is an L2 round
-    // trip away, and a row of a narrow matrix may have twenty of them); added in CTA order.  One part more and the kernel
-    // needs local memory, which costs every launch 0.5 us.
-    constexpr int Q = 2, P = 5;
+    // Q groups of four outputs per thread and P parts at a time, added in CTA order: ten or twelve 16-byte loads in flight.
+    // More and the kernel needs local memory, which costs every launch 0.5 us.
+    constexpr int Q = N_TILE <= 32 ? 2 : 4, P = N_TILE <= 32 ? 5 : 2;
     const int     quads = p.N * (kTileM / 4);
-    for (int q0 = tid; q0 < quads; q0 += Q * 128) {
+    for (int q0 = tid; q0 < quads; q0 += Q * threads) {
         float4 acc[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i)
-            if (q0 + i * 128 < quads)
-                acc[i] = __ldcg(reinterpret_cast<const float4*>(first) + q0 + i * 128);
+            if (q0 + i * threads < quads)
+                acc[i] = __ldcg(reinterpret_cast<const float4*>(first) + q0 + i * threads);
         for (int c = c_first + 1; c <= c_last; c += P) {
             float4 v[P][Q];
 #pragma unroll
             for (int j = 0; j < P; ++j)
 #pragma unroll
                 for (int i = 0; i < Q; ++i)
-                    if (c + j <= c_last && q0 + i * 128 < quads)
-                        v[j][i] = __ldcg(reinterpret_cast<const float4*>(p.partial + slot * (2 * (c + j))) + q0 + i * 128);
+                    if (c + j <= c_last && q0 + i * threads < quads)
+                        v[j][i] = __ldcg(reinterpret_cast<const float4*>(p.partial + slot * (2 * (c + j))) + q0 + i * threads);
 #pragma unroll
             for (int j = 0; j < P; ++j)
 #pragma unroll
@@ -196,7 +211,7 @@ sum_row_parts(const SpmmParams& p, int row, int c_first, int c_last, const float
         }
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-            const int q = q0 + i * 128;
+            const int q = q0 + i * threads;
             if (q >= quads)
                 break;
             const int    n = q / (kTileM / 4), out_row = row * kTileM + (q % (kTileM / 4)) * 4;
@@ -237,9 +252,8 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
     const int       chunk    = p.plan.chunk_tiles;
     const int       ctas     = gridDim.x;
     const int       cta      = blockIdx.x;
-    const long long tiles    = static_cast<long long>(p.M / kTileM) * p.k_tiles;
-    const int       t_begin  = stream_begin(tiles, ctas, cta);
-    const int       L        = stream_begin(tiles, ctas, cta + 1) - t_begin;  // >= 1: the grid has at most `tiles` CTAs
+    const int       t_begin  = stream_begin(p.stream_share, cta);
+    const int       L        = stream_begin(p.stream_share, cta + 1) - t_begin;  // >= 1: the grid has at most `tiles` CTAs
     const int       row0     = t_begin / p.k_tiles;
     const int       k0       = t_begin - row0 * p.k_tiles;  // K tile the CTA starts at
 
@@ -255,7 +269,8 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
     const uint32_t misc_off  = (b_empty + 8u * b_stages) - base;
     volatile uint32_t* const tmem_slot  = reinterpret_cast<volatile uint32_t*>(smem + misc_off);
     volatile uint32_t* const abort_flag = reinterpret_cast<volatile uint32_t*>(smem + misc_off + 4);
-    int* const               offs_stage = reinterpret_cast<int*>(smem + misc_off + 16);  // plan.offsets_staged ints
+    int* const               sums       = reinterpret_cast<int*>(smem + misc_off + 16);  // rows to add up at the end
+    int* const               offs_stage = reinterpret_cast<int*>(smem + misc_off + 16 + kStreamSumBytes);  // plan.offsets_staged ints
 
     const int* const offs_global = p.tile_offsets + t_begin;
     const bool       staged      = (L + 1 <= p.plan.offsets_staged);
@@ -440,7 +455,8 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                     ptx::mbar_arrive(acc_empty + 8u * (q & 1));
             }
         };
-        int q = 0;
+        int          q    = 0;
+        unsigned int todo = 0;  // tid 0: rows this CTA has completed the count of, its first or its last or both
         for (int row = row0;; ++row) {
             const int j = row == row0 ? 0 : (row - row0) * p.k_tiles - k0;
             if (j >= L)
@@ -449,10 +465,45 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
             const bool     whole = len == p.k_tiles;
             bool           ok    = go;
             int            i     = 0;
+            // A row of two CTAs, the first one's last segment: usually the other, which began with its part, has parked that
+            // long ago.  Then this CTA takes it into tensor memory ahead of time and finishes the row, parking nothing.
+            const int  row_begin = row * p.k_tiles;
+            const int  c_last    = whole ? cta : stream_owner(p, ctas, row_begin + p.k_tiles - 1);
+            const bool ask       = c_last == cta + 1 && t_begin <= row_begin;
+            bool       asked = false, complete = false;
+            const float bias = bias_of(p, row * kTileM + r);
+            auto       other_has_parked = [&](bool look) {  // every epilogue warp asks once
+                asked             = true;
+                unsigned int seen = 0u;
+                if (look && tid == 0) {
+                    ptx::grid_dependency_wait();  // counters may be in use by the stream's previous launch until it is over
+                    seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
+                    for (int n = 1; seen == 0u && n < kStreamLooks && !ptx::mbar_test_wait(acc_full + 8u * (q & 1), (q >> 1) & 1u); ++n)
+                        seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
+                    ptx::fence_acq_rel_gpu();
+                }
+                return barrier_any(1u, 128u, seen == 1u);
+            };
             for (; ok; i += chunk, ++q) {
+                const bool last_chunk = i + chunk >= len;
+                if (last_chunk && ask) {
+                    complete = other_has_parked(true);
+                    if (complete) {
+                        const float* from = p.partial + static_cast<size_t>(N_TILE * kTileM) * (2 * c_last) + r;
+#pragma unroll 1
+                        for (int c0 = 0; c0 < N_TILE; c0 += 8, from += 8 * kTileM) {
+                            float v[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e)
+                                v[e] = c0 < p.N ? __ldcg(from + e * kTileM) : 0.0f;
+                            ptx::tmem_st_x8(tmem_sum + N_TILE + c0, v);
+                        }
+                        ptx::tmem_wait_st();
+                    }
+                }
                 ok = __all_sync(0xFFFFFFFFu, wait_bounded_converged(acc_full + 8u * (q & 1), (q >> 1) & 1u, abort_flag, p.status));
                 ptx::tc_fence_after_sync();
-                if (!ok || i + chunk >= len)
+                if (!ok || last_chunk)
                     break;
 #pragma unroll 1
                 for (int c0 = 0; c0 < N_TILE; c0 += 8) {
@@ -462,12 +513,22 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                 }
                 ptx::tmem_wait_st();
             }
-            float* const park = whole ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (j == 0 ? 0 : 1)) + r;
+            if (ask && !asked)  // gave up on the way
+                complete = other_has_parked(false);
+            float* const park = whole || complete ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (j == 0 ? 0 : 1)) + r;
             if (ok) {  // the segment's last chunk
 #pragma unroll 1
                 for (int c0 = 0; c0 < N_TILE; c0 += 8) {
                     float v[8];
                     read_columns(q, c0, i != 0, v);
+                    if (complete) {
+                        uint32_t t[8];
+                        ptx::tmem_ld_x8(tmem_sum + N_TILE + c0, t);
+                        ptx::tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            v[e] += __uint_as_float(t[e]);
+                    }
                     if (park != nullptr) {
 #pragma unroll
                         for (int e = 0; e < 8; ++e)
@@ -475,42 +536,53 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                                 __stcg(park + (c0 + e) * kTileM, v[e]);
                     }
                     else
-                        finish_columns<8>(p, v, static_cast<size_t>(c0) * p.M + row * kTileM + r, p.N - c0, row * kTileM + r);
+                        finish_columns<8>(p, v, static_cast<size_t>(c0) * p.M + row * kTileM + r, p.N - c0, bias);
                 }
                 ++q;
             }
-            if (!whole) {
-                const long long row_begin = static_cast<long long>(row) * p.k_tiles;
-                const int       c_first   = stream_owner(tiles, ctas, row_begin);
-                const int       c_last    = stream_owner(tiles, ctas, row_begin + p.k_tiles - 1);
-                // only the row's first CTA may have begun before the row: this is then its last segment, in its second slot
-                const int       slot      = 2 * c_first + (stream_begin(tiles, ctas, c_first) < row_begin ? 1 : 0);
+            if (complete) {
+                if (tid == 0)
+                    p.tile_counters[row] = 0u;  // nobody else touches it again in this launch
+            }
+            else if (!whole) {
                 const bool gave_up = barrier_any(1u, 128u, !ok);
                 if (tid == 0) {
                     // arrivals in the low half of the counter; a CTA that gave up also marks the high half, so that the
                     // last one knows the row's sum is not to be trusted
                     const unsigned int mine = gave_up ? 0x10001u : 1u;
-                    ptx::grid_dependency_wait();  // counters may be in use by the stream's previous launch until it is over
-                    const unsigned int before = ptx::atom_add_acq_rel_gpu(p.tile_counters + row, mine);
-                    const bool         last   = (before & 0xFFFFu) + 1u == static_cast<unsigned int>(c_last - c_first + 1);
-                    if (last)
+                    ptx::grid_dependency_wait();  // (as above)
+                    const int          c_first = stream_owner(p, ctas, row_begin);
+                    const unsigned int before  = ptx::atom_add_acq_rel_gpu(p.tile_counters + row, mine);
+                    if ((before & 0xFFFFu) + 1u == static_cast<unsigned int>(c_last - c_first + 1)) {
                         p.tile_counters[row] = 0u;  // nobody else touches it again in this launch
-                    abort_flag[kLastOfTile] = last ? (((before + mine) >> 16) != 0u ? 2u : 1u) : 0u;
+                        if (((before + mine) >> 16) == 0u) {
+                            sums[3 * todo]     = row;
+                            sums[3 * todo + 1] = c_first;
+                            sums[3 * todo + 2] = c_last;
+                            ++todo;
+                        }
+                    }
                 }
-                ptx::named_barrier_sync(1u, 128u);
-                if (abort_flag[kLastOfTile] == 1u) {
-                    sum_row_parts<N_TILE>(p, row, c_first, c_last, p.partial + static_cast<size_t>(N_TILE) * kTileM * slot, tid);
-                }
-                ptx::named_barrier_sync(1u, 128u);  // kLastOfTile is free again
             }
         }
+        if (tid == 0)
+            abort_flag[kLastOfTile] = todo;
     }
 
-    // ================================================================ tear-down
+    // ================================================================ tear-down, and the sums of rows that became complete here
     ptx::tc_fence_before_sync();
     __syncthreads();
     if (warp == 1)
         ptx::tmem_dealloc(tmem_acc, kTmemCols);
+    const unsigned int todo = abort_flag[kLastOfTile];
+#pragma unroll 1
+    for (unsigned int i = 0; i < todo; ++i) {
+        const int row = sums[3 * i], c_first = sums[3 * i + 1], c_last = sums[3 * i + 2];
+        // only the row's first CTA may have begun before the row: this is then its last segment, in its second slot
+        const int slot = 2 * c_first + (stream_begin(p.stream_share, c_first) < row * p.k_tiles ? 1 : 0);
+        sum_row_parts<N_TILE>(p, row, c_first, c_last, p.partial + static_cast<size_t>(N_TILE) * kTileM * slot, threadIdx.x,
+                              kStreamWarps * 32);
+    }
 }
 
 }  // namespace flashllm

@@ -40,6 +40,32 @@ def test_shares_of_the_tile_sequence(lib, oracle, streaming, M, K, N, sparsity):
         assert np.array_equal(prob.run(), first)
 
 
+@pytest.mark.parametrize("M,K", [
+    (128 * 300, 64 * 40),  # 40.5 tiles a CTA, 40 a row: last segments of one tile and more, first ones of 39 and fewer
+    (128 * 150, 64 * 64),  # 32.4 tiles a CTA: every row is cut once or twice
+    (128 * 148, 64 * 24),  # 12 tiles a CTA: every row belongs to two, neither of which has begun before it
+])
+@pytest.mark.parametrize("N", [8, 32, 64])
+def test_rows_of_two_shares(lib, streaming, M, K, N):
+    """The CTA that holds a row's first part finishes the row from tensor memory when the other part is there already, and
+    parks its own when it is not; either way the same bits."""
+    from flash_llm_b200 import torch_op  # noqa: F401  (registers torch.ops.flashllm)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M + K + N)
+    A = (torch.rand((M, K), generator=gen, device="cuda") - 0.5).half()
+    A *= torch.rand((M, K), generator=gen, device="cuda") >= 0.8
+    B = (torch.rand((N, K), generator=gen, device="cuda") - 0.5).half()
+    bias = (torch.rand(M, generator=gen, device="cuda") - 0.5).half()
+    residual = (torch.rand((N, M), generator=gen, device="cuda") - 0.5).half()
+    words, offs = torch.ops.flashllm.encode(A)
+    want = (B.double() @ A.double().T + bias.double() + residual.double()).float().cpu().numpy()
+    first = torch.ops.flashllm.spmm_epilogue(words, offs, B, M, 1, bias, 0, residual)
+    assert_close(first.cpu().numpy(), want, f"M={M} K={K} N={N}")
+    for _ in range(20):
+        assert torch.equal(torch.ops.flashllm.spmm_epilogue(words, offs, B, M, 1, bias, 0, residual), first)
+    assert lib.consume_status() == 0
+
+
 @pytest.mark.parametrize("M,K,N", [(27648, 9216, 16), (27648, 9216, 32), (49152, 4608, 64)])
 def test_sums_are_as_exact_as_the_row_forms(lib, M, K, N):
     """The tensor core truncates its additions, so sums of positive products come out too small by a share that grows with
