@@ -157,6 +157,12 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void* src, uint32_t bytes
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+// Asks for one line in L2; a hint that reads nothing.
+__device__ __forceinline__ void prefetch_l2(const void* line)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+}
+
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

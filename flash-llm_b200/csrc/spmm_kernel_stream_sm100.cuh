@@ -316,6 +316,11 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
         ptx::tmem_relinquish();
     }
     if (!p.early_weights) {
+        // The offsets are the first of two memory latencies in a row that a call starts with.  No value may be read before the
+        // wait, but they may be on their way to L2: 36864x9216 N=16 70.6 -> 69.9 us, 9216x36864 N=32 93.5 -> 92.8.
+        if (warp >= kStreamFirstEpi)
+            for (int i = (threadIdx.x - kStreamFirstEpi * 32) * 32; i <= L; i += 128 * 32)
+                ptx::prefetch_l2(offs_global + i);
         ptx::grid_dependency_wait();
         if (scatters)
             stream.fetch_first(p, offs_global, sw, L, lane);
