@@ -287,6 +287,7 @@ static std::atomic<int> g_launch_overlap{0};
 
 
 constexpr int kDefaultPath = kPathDirect;
+constexpr int kSmemPerSm   = 228 * 1024;  // for all resident CTAs, 1 KB of it each for the system
 
 static int n_tile_for(int N)
 {
@@ -295,9 +296,9 @@ static int n_tile_for(int N)
 
 static int plan_smem_bytes(const SpmmPlan& pl)
 {
-    const int bars = 8 * (2 * pl.ring_slots + 2 * pl.a_stages + 2 * pl.b_stages + 1) + 16 + 4 * pl.offsets_staged;
+    const int bars = 8 * (2 * pl.ring_slots + 2 * pl.a_stages + 2 * pl.b_stages + 2) + 16 + 4 * pl.offsets_staged;
     return pl.a_stages * kDenseTileBytes + pl.b_stages * pl.b_batch * pl.n_tile * kTileK * 2
-           + pl.ring_slots * pl.chunk_vectors * 16 + bars;
+           + pl.ring_slots * pl.chunk_vectors * 16 + pl.sum_bytes + bars;
 }
 
 static bool is_pow2(int v)
@@ -564,6 +565,14 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // room for this CTA's slice of TileOffsets (K tiles of the longest part, plus one), up to 8 KB
     const int longest = (k_tiles + pl.cluster_k * pl.workspace_k - 1) / (pl.cluster_k * pl.workspace_k) + 1;
     pl.offsets_staged = longest + 1 <= 2048 ? ((longest + 1 + 3) / 4) * 4 : 0;
+    // Room of its own for the peers' partial sums where it costs no resident CTA: they may then arrive while this CTA still
+    // multiplies.  (Wide outputs take the operands' buffers, once everybody's MMAs are over.)
+    if (direct && pl.cluster_k > 1) {
+        pl.sum_bytes   = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
+        const int room = two_resident ? kSmemPerSm / 2 - 1024 : st->smem_optin;
+        if (plan_smem_bytes(pl) > room)
+            pl.sum_bytes = 0;
+    }
     pl.smem_bytes     = plan_smem_bytes(pl);
 
     const bool ring_ok = pl.scatter_warps >= 4 && pl.scatter_warps <= kMaxScatterWarps
@@ -581,8 +590,10 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
                     && pl.b_batch >= 1 && pl.b_batch <= 256 && pl.cluster_k >= 1 && pl.cluster_k <= kMaxClusterK
                     && pl.workspace_k >= 1 && (pl.reduce == kReduceSecondKernel || pl.reduce == kReduceLastCta)
                     && pl.smem_bytes <= st->smem_optin
-                    // the fp32 partial tile of the cluster reduction is parked over the pipeline buffers
-                    && pl.smem_bytes - 1024 - 4 * pl.offsets_staged >= pl.n_tile * kTileM * 4;
+                    // the fp32 partial tiles of the cluster reduction are parked over the pipeline buffers
+                    && pl.smem_bytes - 1024 - 4 * pl.offsets_staged >= pl.n_tile * kTileM * 4
+                    && (!direct || pl.cluster_k == 1 || pl.sum_bytes > 0
+                        || pl.a_stages * kDenseTileBytes + pl.b_stages * pl.b_batch * slab >= cluster_sum_bytes(pl.n_tile, pl.cluster_k));
     if (!ok)
         return cudaErrorInvalidConfiguration;
     *out = pl;

@@ -16,6 +16,57 @@
 
 namespace flashllm {
 
+// Warp-collective bounded wait: every lane probes (the probe parks the warp for a while), one answer for all lanes.
+__device__ __forceinline__ bool
+wait_bounded_converged(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int* status)
+{
+    if (ptx::mbar_try_wait(bar, parity))
+        return true;
+    uint64_t t0 = 0;
+    bool     ok = true;
+    for (uint32_t it = 1; ok && !ptx::mbar_try_wait(bar, parity); ++it) {
+        if ((it & 255u) == 0u) {
+            if (*abort_flag)
+                ok = false;
+            else if (abort_flag[kDepsResolved] == 0u)  // still behind the previous kernel of the stream: no clock yet
+                t0 = 0;
+            else {
+                const uint64_t now = ptx::globaltimer_ns();
+                if (t0 == 0)
+                    t0 = now;
+                else if (now - t0 > kWaitLimitNs) {
+                    *abort_flag = 1u;
+                    atomicOr(status, kStatusWaitExpired);
+                    ok = false;
+                }
+            }
+        }
+    }
+    return ok;
+}
+
+// Warp-collective bounded wait for what the CTAs of the cluster store here: every lane probes (the probe parks the warp for a
+// while).  A peer that is late is late by its own bounded waits, so the clock runs twice as long.  A CTA that gave up
+// on the way sends what it has, so that its peers' waits end.
+__device__ __forceinline__ bool
+wait_bounded_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int* status)
+{
+    uint64_t t0 = 0;
+    for (uint32_t it = 1; !ptx::mbar_try_wait_cluster(bar, parity); ++it) {
+        if ((it & 255u) == 0u) {
+            const uint64_t now = ptx::globaltimer_ns();
+            if (t0 == 0)
+                t0 = now;
+            else if (now - t0 > 2 * kWaitLimitNs) {
+                *abort_flag = 1u;
+                atomicOr(status, kStatusWaitExpired);
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
 // Words are read once, so they get no line of L1; not through the read-only path (ld.global.nc): a kernel is launched before
 // its predecessors have ended, and that path is for data that nobody writes in a kernel's lifetime.
 #ifndef FLASHLLM_LDG_FLAVOUR
@@ -147,6 +198,105 @@ constexpr int kPrefetchAhead = FLASHLLM_PREFETCH_AHEAD;
 // Warps of the register-streaming kernel: one B loader, kDirectIssuers MMA issuers, then the scatter warps.
 constexpr int kDirectIssuers = 2;
 
+// Sum over the CTAs of a cluster: rank q finishes rows [128 q / S, 128 (q + 1) / S) of the output tile, and every CTA sends it
+// those rows of its partial tile, [S ranks][rows][columns + 4 for the banks' sake].  The stores count themselves in on the
+// receiver's mbarrier, so nobody asks a peer for data or waits for it beyond that.  With the partial tiles parked at home and
+// fetched between two cluster barriers the sum took 2.4 of the 6.3 us of 1024x1024 N = 8 in clusters of eight.  us per call
+// before and after, with the waits that park the warp in place of sleeping ones: that call 5.6 -> 4.5, 4096x4096 N = 16
+// (eight) 9.9 -> 8.7, 9216x1152 N = 16 (three) 9.1 -> 8.1, 4736x7232 N = 32 (seven) 19.0 -> 18.6.
+__host__ __device__ constexpr int cluster_sum_rows(int S)
+{
+    return (kTileM + S - 1) / S;
+}
+__host__ __device__ constexpr int cluster_sum_bytes(int n_tile, int S)
+{
+    return S * cluster_sum_rows(S) * (n_tile + 4) * 4;
+}
+
+// One scatter warp's share of the accumulators (as in accumulators_to_output) to the CTAs that finish its rows.
+template<int N_TILE>
+__device__ __forceinline__ void accumulators_to_peers(uint32_t tmem_acc, int accumulators, int n_valid, int quarter, int lane, int sw,
+                                                      int per_quarter, int S, int rank, uint32_t sum_base, uint32_t sum_bar)
+{
+    if (sw >= 4 * per_quarter)
+        return;
+    const int col_share = (N_TILE / per_quarter) < 8 ? 8 : (N_TILE / per_quarter);
+    const int col_begin = (sw / 4) * col_share;
+    const int col_end   = (col_begin + col_share) < n_valid ? (col_begin + col_share) : n_valid;
+    const int row = quarter * 32 + lane;
+    const int q   = ((row + 1) * S - 1) / kTileM;  // who finishes this row
+    const uint32_t bar = ptx::map_to_rank(sum_bar, q);
+    const uint32_t to  = ptx::map_to_rank(sum_base, q)
+                        + static_cast<uint32_t>((rank * cluster_sum_rows(S) + row - kTileM * q / S) * (N_TILE + 4)) * 4u;
+    const uint32_t acc = tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16);
+    for (int c0 = col_begin; c0 < col_end; c0 += 8) {
+        float    v[8];
+        uint32_t t[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            v[i] = 0.0f;
+        for (int a = 0; a < accumulators; ++a) {
+            ptx::tmem_ld_x8(acc + a * N_TILE + c0, t);
+            ptx::tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = a == 0 ? __uint_as_float(t[i]) : v[i] + __uint_as_float(t[i]);
+        }
+        ptx::st_async_v4_f32(to + c0 * 4, v, bar);
+        ptx::st_async_v4_f32(to + c0 * 4 + 16, v + 4, bar);
+    }
+}
+
+// The rows this CTA finishes, once all its peers' parts are there: added in rank order, four columns per thread.
+template<int N_TILE>
+__device__ __forceinline__ void finish_cluster_rows(const SpmmParams& p, uint32_t sum_base, int rank, int S, int G, int g, int n_idx,
+                                                    int tile_row, int n_valid, int tid, int threads)
+{
+    const int    row0     = kTileM * rank / S;
+    const int    rows     = kTileM * (rank + 1) / S - row0;
+    const size_t tile_off = static_cast<size_t>(n_idx) * N_TILE * p.M + static_cast<size_t>(tile_row) * kTileM;
+    const uint32_t step  = static_cast<uint32_t>(cluster_sum_rows(S) * (N_TILE + 4)) * 4u;
+    const int      shift = 32 - __clz(rows - 1);  // rows, rounded up to a power of two, are 16 to 64
+    for (int e = tid; e < (n_valid / 4) << shift; e += threads) {
+        const int r = e & ((1 << shift) - 1), c = (e >> shift) * 4;
+        if (r >= rows)
+            continue;
+        const uint32_t from = sum_base + static_cast<uint32_t>(r * (N_TILE + 4) + c) * 4u;
+        float          v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        uint4          w[kMaxClusterK];
+#pragma unroll
+        for (int s = 0; s < kMaxClusterK; ++s)
+            if (s < S)
+                w[s] = lds16(from + s * step);
+#pragma unroll
+        for (int s = 0; s < kMaxClusterK; ++s)
+            if (s < S) {
+                v[0] += __uint_as_float(w[s].x);
+                v[1] += __uint_as_float(w[s].y);
+                v[2] += __uint_as_float(w[s].z);
+                v[3] += __uint_as_float(w[s].w);
+            }
+        const int    m  = row0 + r;
+        const size_t at = static_cast<size_t>(c) * p.M + m;
+        if (G > 1) {
+            float* const part = p.partial + static_cast<size_t>(g) * p.M * p.N + tile_off + at;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                part[static_cast<size_t>(i) * p.M] = v[i];
+        }
+        else if (p.push_world > 0) {
+            for (int w = 0; w < p.push_world; ++w)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    p.push_slot[w][tile_off + at + static_cast<size_t>(i) * p.M] = v[i];
+        }
+        else
+            finish_columns<4>(p, v, tile_off + at, 4, bias_of(p, tile_row * kTileM + m));
+    }
+    if (G > 1 && p.tile_counters != nullptr)
+        __threadfence();
+}
+
 // CAP: vectors per lane kept in registers.  WARPS: stages = tiles in flight per CTA.  WPT: warps that share one tile
 // (row q of warp h is the tile's row q * WPT + h), so a tile of up to 32 * CAP * WPT vectors is handled without the
 // overflow loop and a warp's instruction stream per tile is 1 / WPT as long.  MIN_BLOCKS: CTAs per SM the register
@@ -198,13 +348,16 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     // ---- shared memory carve-up
     const uint32_t a_base   = base;
     const uint32_t b_base   = a_base + a_stages * kDenseTileBytes;
-    const uint32_t bar_base = b_base + b_stages * KB * kBSlab;
+    const uint32_t sum_area = b_base + b_stages * KB * kBSlab;  // plan.sum_bytes: the peers' partial sums
+    const uint32_t bar_base = sum_area + plan.sum_bytes;
     const uint32_t a_full   = bar_base;
     const uint32_t a_empty  = a_full + 8u * a_stages;
     const uint32_t b_full   = a_empty + 8u * a_stages;
     const uint32_t b_empty  = b_full + 8u * b_stages;
     const uint32_t acc_full = b_empty + 8u * b_stages;
-    const uint32_t misc_off = (acc_full + 8u) - base;
+    const uint32_t sum_full = acc_full + 8u;
+    const uint32_t misc_off = (sum_full + 8u) - base;
+    const uint32_t sum_base = plan.sum_bytes > 0 ? sum_area : a_base;
     volatile uint32_t* const tmem_slot  = reinterpret_cast<volatile uint32_t*>(smem + misc_off);
     volatile uint32_t* const abort_flag = reinterpret_cast<volatile uint32_t*>(smem + misc_off + 4);
     int* const               offs_stage = reinterpret_cast<int*>(smem + misc_off + 16);  // plan.offsets_staged ints
@@ -268,6 +421,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
             ptx::mbar_init(b_empty + 8u * i, MI);  // every issuer hands a batch back
         }
         ptx::mbar_init(acc_full, MI);
+        ptx::mbar_init(sum_full, 1);
         abort_flag[0]             = 0u;  // a launch never inherits a give-up from an earlier one: the status word only reports
         abort_flag[kDepsResolved] = 0u;
         ptx::fence_mbar_init();
@@ -299,6 +453,15 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
         *abort_flag = 1u;
     }
     const uint32_t tmem_acc = *tmem_slot;
+    const int      n_valid  = (p.N - n_idx * N_TILE) < N_TILE ? (p.N - n_idx * N_TILE) : N_TILE;
+    if (S > 1) {
+        if (threadIdx.x == 0)  // everything the peers (and this CTA) will store here
+            ptx::mbar_arrive_expect_tx(sum_full,
+                                       static_cast<uint32_t>(S * (kTileM * (rank + 1) / S - kTileM * rank / S) * n_valid) * 4u);
+        __syncwarp();
+        if (plan.sum_bytes > 0)
+            ptx::cluster_arrive_relaxed();  // this CTA runs and its barrier is ready
+    }
     // A following kernel of this library may start its set-up and weight streaming while this grid drains; it waits
     // (in its B loader) before it touches anything this grid or its predecessors produce.
     if (threadIdx.x == 0)
@@ -401,7 +564,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
                     FL_TRACE(0, j);
                 bool ok = !bad;
                 if (ok && use > 0)
-                    ok = wait_bounded_warp(empty_bar, (use & 1u) ^ 1u, abort_flag, p.status);
+                    ok = __all_sync(0xFFFFFFFFu, wait_bounded_converged(empty_bar, (use & 1u) ^ 1u, abort_flag, p.status));
                 if (!ok) {  // uniform across the warps that share the tile: they watch the same barrier and flag
                     if (bad)
                         *abort_flag = 1u;
@@ -476,28 +639,34 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
         // ================================================================ epilogue (same warps)
         bool acc_ok = go;
         if (L > 0 && go)
-            acc_ok = wait_bounded_warp(acc_full, 0u, abort_flag, p.status);
+            acc_ok = wait_bounded_converged(acc_full, 0u, abort_flag, p.status);
         acc_ok = __all_sync(0xFFFFFFFFu, acc_ok && (*abort_flag == 0u));
         ptx::tc_fence_after_sync();
         if (sw == 0 && lane == 0)
             FL_CTA_TIME(2);
 
-        accumulators_to_output<N_TILE>(p, tmem_acc, L < MI ? L : MI, N_TILE, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, G, g,
-                                       n_idx, tile_row, acc_ok, reinterpret_cast<float*>(smem));
+        if (S == 1)
+            accumulators_to_output<N_TILE>(p, tmem_acc, L < MI ? L : MI, N_TILE, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, 1, G, g, n_idx,
+                                           tile_row, acc_ok, nullptr);
     }
 
     // ================================================================ cluster reduction and tear-down
-    ptx::tc_fence_before_sync();
-    __syncthreads();
     if (S > 1) {
         __syncwarp();
-        ptx::cluster_sync_all();  // every CTA's partial tile is parked in its shared memory
-        if (warp >= first_sw)
-            cluster_reduce_store<N_TILE>(p, base, rank, S, G, g, n_idx, tile_row, threadIdx.x - first_sw * 32, NTS,
-                                         *abort_flag == 0u);
-        __syncwarp();
-        ptx::cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
+        if (plan.sum_bytes > 0)
+            ptx::cluster_wait();  // long over: the peers have started
+        else
+            ptx::cluster_sync_all();  // nobody multiplies any more, the stages are free
+        if (warp >= first_sw) {
+            ptx::tc_fence_after_sync();
+            accumulators_to_peers<N_TILE>(tmem_acc, L < MI ? L : MI, n_valid, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, rank, sum_base,
+                                          sum_full);
+            if (__all_sync(0xFFFFFFFFu, wait_bounded_cluster(sum_full, 0u, abort_flag, p.status)) && *abort_flag == 0u)
+                finish_cluster_rows<N_TILE>(p, sum_base, rank, S, G, g, n_idx, tile_row, n_valid, threadIdx.x - first_sw * 32, NTS);
+        }
     }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
     finish_tile<N_TILE>(p, S, G, n_idx, tile_row, abort_flag);
     if (threadIdx.x == 0)
         FL_CTA_TIME(3);

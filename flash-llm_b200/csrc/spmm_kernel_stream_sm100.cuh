@@ -65,35 +65,6 @@ __device__ __forceinline__ int stream_owner(const SpmmParams& p, int ctas, int t
     return c;
 }
 
-// Warp-collective bounded wait: every lane probes (the probe parks the warp for a while), one answer for all lanes.
-__device__ __forceinline__ bool
-wait_bounded_converged(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int* status)
-{
-    if (ptx::mbar_try_wait(bar, parity))
-        return true;
-    uint64_t t0 = 0;
-    bool     ok = true;
-    for (uint32_t it = 1; ok && !ptx::mbar_try_wait(bar, parity); ++it) {
-        if ((it & 255u) == 0u) {
-            if (*abort_flag)
-                ok = false;
-            else if (abort_flag[kDepsResolved] == 0u)  // still behind the previous kernel of the stream: no clock yet
-                t0 = 0;
-            else {
-                const uint64_t now = ptx::globaltimer_ns();
-                if (t0 == 0)
-                    t0 = now;
-                else if (now - t0 > kWaitLimitNs) {
-                    *abort_flag = 1u;
-                    atomicOr(status, kStatusWaitExpired);
-                    ok = false;
-                }
-            }
-        }
-    }
-    return ok;
-}
-
 // A scatter warp's tiles sw, sw + STAGES, ... of a CTA's L tiles: the words of the next one wait in registers (up to CAP
 // 16-byte vectors per lane) while the warp's stage is still being multiplied.
 template<int CAP, int STAGES>

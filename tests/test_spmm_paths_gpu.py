@@ -78,6 +78,36 @@ def test_k_splits(lib, oracle, form, reduce, cluster_k, workspace_k, split_k):
            dict(cluster_k=cluster_k, workspace_k=workspace_k, reduce=reduce, **form), "K split")
 
 
+@pytest.mark.parametrize("form", FORMS[1:], ids=FORM_IDS[1:])
+@pytest.mark.parametrize("cluster_k", [2, 3, 7, 8])
+@pytest.mark.parametrize("N", [8, 32, 64, 128, 256])
+def test_cluster_sums_of_every_width(lib, oracle, form, cluster_k, N):
+    """The CTAs of a cluster send one another their rows of the partial tile: into shared memory set aside for that (up to 64
+    columns, where two CTAs per SM leave the room) or over the operands; rows that the cluster size does not divide, columns
+    beyond N, an epilogue, and the same bits every time."""
+    M, K = 384, 64 * 19
+    A, B = random_problem(lib, M, K, N, 0.8, 700 + N + cluster_k)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    bias = torch.rand(M, device="cuda").half()
+    want = oracle.gemm_f32(A, B) + bias.float().cpu().numpy()
+    lib.set_plan(cluster_k=cluster_k, **form)
+    try:
+        prob = DeviceProblem(lib, comp, offs, B, M, N, K, 1)
+        stream = torch.cuda.current_stream().cuda_stream
+        outs = []
+        for _ in range(3):
+            C = torch.full((N, M), float("nan"), dtype=torch.float16, device="cuda")
+            lib.spmm_splitk_epilogue(stream, prob.comp.data_ptr(), prob.offs.data_ptr(), prob.B.data_ptr(), C.data_ptr(), M, N, K,
+                                     None, 1, bias.data_ptr())
+            outs.append(C)
+        assert lib.get_plan(M, N, K, 1)["cluster_k"] == cluster_k
+    finally:
+        lib.set_plan()
+    assert lib.consume_status() == 0
+    assert_close(outs[0].cpu().numpy(), want, f"N={N} S={cluster_k} {form}")
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 @pytest.mark.parametrize("N", [16, 64, 256])
 def test_sum_by_last_cta_is_deterministic_and_leaves_its_counters_clean(lib, oracle, N):
     """The order in which the CTAs of an output tile finish changes from launch to launch; the sum must not.  Repeated
