@@ -312,11 +312,14 @@ static int stream_smem_bytes(const SpmmPlan& pl)
            + 8 * (2 * kStreamStages + 4 + 2 * pl.b_stages) + 16 + kStreamSumBytes + 4 * pl.offsets_staged;
 }
 
-// K tiles that the tensor core adds up in one accumulator when K is cut into `parts` and every CTA alternates between two.
-// The tensor core truncates each of its additions, so the error of a sum grows with their number (measured: 7e-8 of the sum
-// per tile of four); the streaming form keeps to what the plan of one CTA or cluster per tile row comes to at the same sizes.
-static int tiles_per_accumulator(int k_tiles, int parts)
+// K tiles that the tensor core may add up in one accumulator.  It truncates each of its additions, so the error of a sum grows
+// with their number (measured: 7e-8 of the sum per tile of four).  No more than when K is cut into `parts`, or into as many parts
+// as fill the GPU (in clusters and in the caller's workspace) if that is more, and every part alternates between two.
+static int tiles_per_accumulator(const DeviceState* st, int tile_rows, int k_tiles, int max_extra, int parts)
 {
+    const int most = kMaxClusterK * max_extra, fill = kStreamCtasPerSm * st->sm_count / tile_rows;
+    const int cut  = fill < most ? fill : most;
+    parts          = parts < cut ? cut : parts;
     return ((k_tiles + parts - 1) / parts + 1) / 2;
 }
 
@@ -346,33 +349,70 @@ static cudaError_t make_stream_plan(const DeviceState* st, SpmmPlan pl, int tile
     return cudaSuccess;
 }
 
-// What a launch costs, in tiles of one CTA while two share an SM (0.49 us at N = 16, 80 % sparsity; 0.54 us at N = 64).
-// Fitted to launches of 8..288 tile rows by 16..512 K tiles, B200, back to back on one stream:
-//   one CTA (cluster) per tile row  10.5 + 2.3 with a cluster sum + the tiles of a CTA per wave, two thirds of that while
-//                                   no SM holds two CTAs; + 4 for a second kernel
-//   streaming form                  0.93 of the tiles of a CTA + 15 + 0.32 per part of a row at N <= 16, more for wider
-//                                   parts (the last part's CTA sums the row while everybody else has finished).  At 0.45
-//                                   for N <= 16 some forty shapes of 4..56 rows went by rows, 2..43 % slower: 2048x16384
-//                                   70 % 23.5 us against 16.4, 512x32768 30.4 / 22.8, 2048x32768 26.5 / 24.5; below 0.3
-//                                   512x22400 90 % (17.9 / 21.5) and 32000x1536 (18.2 / 19.4) would change too
-static double one_row_cost(const DeviceState* st, long long capacity, int ctas_flat, int k_tiles, int s, int g, int n_tile)
-{
-    const long long clusters = static_cast<long long>(ctas_flat) * g;
-    const double    waves    = static_cast<double>((clusters + capacity - 1) / capacity);
-    const double    tiles    = static_cast<double>((k_tiles + s * g - 1) / (s * g)) * (clusters * s <= st->sm_count ? 0.66 : 1.0);
-    return waves * (tiles + 10.5 + (n_tile - 16) * 0.15 + (s > 1 ? 2.3 : 0.0)) + (g > 1 ? 4.0 : 0.0);
-}
-
-static double stream_cost(const SpmmPlan& pl, int tile_rows, int k_tiles)
-{
-    const double tiles = static_cast<double>(tile_rows) * k_tiles / pl.ctas;
-    const double parts = 1.0 + static_cast<double>(pl.ctas) / tile_rows;
-    return 0.93 * tiles + 15.0 + (pl.n_tile - 16) * 0.15 + parts * (pl.n_tile <= 16 ? 0.32 : 0.225 + pl.n_tile * 0.45 / 32.0);
-}
-
 // Clusters of S CTAs resident at a time on 148 SMs (measured), two CTAs or one per SM.
 constexpr int kClustersResident2[kMaxClusterK + 1] = {0, 296, 148, 92, 71, 56, 45, 37, 33};
 constexpr int kClustersResident1[kMaxClusterK + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+
+static long long clusters_resident(const DeviceState* st, const int* table, int s)
+{
+    const long long c = static_cast<long long>(table[s]) * st->sm_count / 148;
+    return c < 1 ? 1ll : c;
+}
+
+// What a launch with N <= 64 costs, in us, back to back on one stream: fitted to 4..200 tile rows by 16..512 K tiles at 80 %
+// sparsity on a B200, launch overlap off and on, with every cluster size and the streaming form timed at each; against the
+// fastest of them the choice then loses 0.8 % on average, where one cost for all K cuts lost 6.1.
+struct FormCosts {
+    double whole, cluster, per_rank;  // fixed part: uncut, in clusters, and what their sum adds for the rows a CTA sums
+    double crowded, full;             // more with two CTAs per SM, and when a grid leaves no place for the next one's clusters
+    double tile_alone, tile_shared;   // per tile of a CTA with an SM to itself, or not
+    double second_kernel;             // of a sum over workspace parts
+    double stream, stream_tile, stream_part;
+};
+static const FormCosts kFormCosts[2][3] = {{{3.3, 4.0, 1.3, 0.35, 0.5, 0.280, 0.46, 2.5, 6.2, 0.450, 0.07},
+                                            {3.85, 4.2, 3.3, 0.8, 0.9, 0.295, 0.50, 2.5, 6.9, 0.475, 0.17},
+                                            {4.75, 5.4, 3.7, 2.0, 2.0, 0.315, 0.53, 2.5, 8.7, 0.525, 0.41}},
+                                           {{3.0, 3.7, 0.0, 0.0, 1.0, 0.280, 0.45, 1.6, 5.0, 0.440, 0.07},
+                                            {3.6, 4.8, 0.0, 0.0, 1.3, 0.295, 0.48, 1.6, 6.0, 0.465, 0.17},
+                                            {4.3, 7.2, 0.0, 0.0, 2.2, 0.315, 0.51, 1.6, 7.6, 0.500, 0.41}}};
+
+static const FormCosts& form_costs(bool overlap, int n_tile)
+{
+    return kFormCosts[overlap ? 1 : 0][n_tile == 16 ? 0 : n_tile == 32 ? 1 : 2];
+}
+
+// One CTA or cluster of S CTAs per tile row (and workspace part).
+static double row_form_us(const DeviceState* st, int ctas_flat, int k_tiles, int s, int g, int n_tile, bool overlap)
+{
+    const FormCosts& f        = form_costs(overlap, n_tile);
+    const long long  clusters = static_cast<long long>(ctas_flat) * g;
+    const long long  held = clusters_resident(st, kClustersResident2, s), apart = clusters_resident(st, kClustersResident1, s);
+    const double     fixed  = s == 1 ? f.whole : f.cluster + f.per_rank / s;
+    const double     tiles  = static_cast<double>((k_tiles + s * g - 1) / (s * g));
+    const double     alone  = fixed + f.tile_alone * tiles;
+    const double     shared = fixed + (s > 1 ? f.crowded + (10 * clusters > 9 * held ? f.full : 0.0) : 0.0) + f.tile_shared * tiles;
+    // Who has an SM to itself.  The last few clusters of three and more do not find their SMs empty (25 of five, of which 148
+    // SMs hold 26, took 17.7 us where 24 take 12.5), and with overlap the next launch's CTAs are there early and pair up, unless
+    // there are few of them or one for every SM (96 rows by 113 tiles, N = 16: 49 us; 148 rows: 35).
+    bool to_itself = s <= 2 ? clusters <= apart : 100 * clusters <= 93 * apart;
+    if (overlap)
+        to_itself = to_itself && (s == 1 ? clusters <= 32 || 100 * clusters > 95 * apart : clusters * s <= 64);
+    return (to_itself ? alone : (clusters + held - 1) / held * shared) + (g > 1 ? f.second_kernel + 0.1 * g : 0.0);
+}
+
+// The row form was fitted to matrices that L2 holds a part of; 288 rows by 144 take 75.9 us from DRAM, not 69.5.
+static double row_form_margin(int tile_rows, int k_tiles)
+{
+    return static_cast<long long>(tile_rows) * k_tiles < 4000 ? 1.0 : 1.05;
+}
+
+// The streaming form: a CTA's tiles, and the parts that the CTA which completes a row adds up.
+static double stream_form_us(const SpmmPlan& pl, int tile_rows, int k_tiles, bool overlap)
+{
+    const FormCosts& f     = form_costs(overlap, pl.n_tile);
+    const double     tiles = static_cast<double>(tile_rows) * k_tiles / pl.ctas;
+    return f.stream + f.stream_tile * tiles + f.stream_part * (1.0 + static_cast<double>(pl.ctas) / tile_rows);
+}
 
 // N >= 256: output columns per CTA, cluster parts S and workspace parts G by the cheapest estimate, in SM cycles; what the
 // caller pinned is kept.  A CTA of the wide form takes kTileCycles per tile (by hundreds of columns; 128 columns are the
@@ -500,17 +540,14 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // G parts through fp32 partial tiles in the workspace (summed by the last CTA of a tile to finish, or by a second
     // kernel).  A launch of rows*G clusters of S CTAs runs in ceil(rows*G / capacity(S)) waves, where capacity(S) is
     // the number of clusters of S CTAs the GPU holds at a time -- measured, and well below slots/S for S >= 3 (71
-    // clusters of 4, 33 of 8 on 296 slots): one cluster more than that and the launch takes twice as long.  Every
+    // clusters of 4, 33 of 8 on 296 slots): one cluster more than that and the launch takes twice as long.  Up to 64
+    // columns row_form_us prices a cut.  Elsewhere every
     // CTA processes k_tiles/(S*G) tiles after a fixed cost worth about 16 tiles; a cluster sum costs about 3 more,
     // the sum by the last CTA 2 + 0.1 per part (8 + 0.1 per part in a fused all-reduce, where the peers wait for that
     // CTA: measured on 2 GPUs, 9216x1152 ... 9216x18432), a second kernel half a tile per part.  The cheapest (S, G) wins,
     // fewer parts on a tie.  Replaces the reference's hand-tuned Split_K tables (kernel_benchmark/benchmark.sh:13-15).
     const bool two_resident = two_per_sm && ((direct && pl.producers == 1) ? kDirectBlocks : 2) == 2;
     const int* resident     = two_resident ? kClustersResident2 : kClustersResident1;
-    auto capacity = [&](int S_) {  // the table is for 148 SMs
-        const long long c = static_cast<long long>(resident[S_]) * st->sm_count / 148;
-        return c < 1 ? 1ll : c;
-    };
     const int max_extra = max_parts > 1 ? max_parts : 1;
     // (measured on eleven shapes from 9216x1152 to 9216x36864: with launch overlap the second kernel hides behind its
     // neighbours and beats the sum by the last CTA, which sits on every tile's critical path, by ~2 us per call;
@@ -519,18 +556,29 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     if (ctas_flat > kCounterTiles)
         pl.reduce = kReduceSecondKernel;
     // (Without launch overlap a second kernel used to cost a whole launch, and small problems did better with clusters alone.
-    // This rule and the costs below were fitted before every kernel was launched with programmatic serialisation;
-    // one_row_cost, which prices the choice against the streaming form, was fitted since.)
+    // This rule and the costs in tiles below were fitted before every kernel was launched with programmatic serialisation.)
     const bool no_second = pl.reduce == kReduceSecondKernel && static_cast<long long>(tile_rows) * k_tiles <= 4096
                            && g_launch_overlap.load(std::memory_order_relaxed) == 0;
+    const bool overlap = g_launch_overlap.load(std::memory_order_relaxed) != 0;
+    // Priced in us where the row form with two CTAs per SM and the streaming form are the choice.
+    const bool priced = direct && two_resident && pl.n_tile <= kScratchMaxN && !sends;
     int    best_s = 1, best_g = 1;
     double best_cost = 0.0;
     for (int s_ = 1; s_ <= kMaxClusterK && s_ <= k_tiles; ++s_) {
         for (int g = 1; g <= max_extra && g <= 32 && s_ * g <= k_tiles; ++g) {
             if (g > 1 && no_second)
                 break;
-            const long long clusters = static_cast<long long>(ctas_flat) * g;
-            const double    waves    = static_cast<double>((clusters + capacity(s_) - 1) / capacity(s_));
+            if (priced) {
+                const double cost = row_form_us(st, ctas_flat, k_tiles, s_, g, pl.n_tile, overlap);
+                if ((s_ == 1 && g == 1) || cost < best_cost) {
+                    best_cost = cost;
+                    best_s    = s_;
+                    best_g    = g;
+                }
+                continue;
+            }
+            const long long clusters = static_cast<long long>(ctas_flat) * g, capacity = clusters_resident(st, resident, s_);
+            const double    waves    = static_cast<double>((clusters + capacity - 1) / capacity);
             const double    per_cta  = static_cast<double>((k_tiles + s_ * g - 1) / (s_ * g)) + 16.0 + (s_ > 1 ? 3.0 : 0.0)
                                     + (g > 1 && pl.reduce == kReduceLastCta ? (sends ? 8.0 : 2.0) + 0.1 * g : 0.0);
             const double cost = waves * per_cta + (g > 1 && pl.reduce == kReduceSecondKernel ? 0.5 * g : 0.0);
@@ -542,11 +590,11 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
             }
         }
     }
-    if (may_stream && !pinned && !sends) {
+    if (may_stream && !pinned && priced) {
         SpmmPlan sp = pl;
         sp.path     = kPathStream;
-        if (make_stream_plan(st, sp, tile_rows, k_tiles, tiles_per_accumulator(k_tiles, best_s * best_g), &sp) == cudaSuccess
-            && stream_cost(sp, tile_rows, k_tiles) < one_row_cost(st, capacity(best_s), ctas_flat, k_tiles, best_s, best_g, pl.n_tile)) {
+        if (make_stream_plan(st, sp, tile_rows, k_tiles, tiles_per_accumulator(st, tile_rows, k_tiles, max_extra, best_s * best_g), &sp) == cudaSuccess
+            && stream_form_us(sp, tile_rows, k_tiles, overlap) < row_form_margin(tile_rows, k_tiles) * best_cost) {
             *out = sp;
             return cudaSuccess;
         }
@@ -562,12 +610,18 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     if (extra < 1)
         extra = 1;
     pl.workspace_k = extra;
+    // A K range that is longer than if K were cut into as many parts as fill the GPU takes turns with four accumulators, so that
+    // no sum in the tensor core gets longer for it.
+    pl.accumulators = kDirectIssuers;
+    const int parts = pl.cluster_k * extra;
+    if (direct && (k_tiles + parts - 1) / parts > 2 * tiles_per_accumulator(st, tile_rows, k_tiles, max_extra, parts))
+        pl.accumulators = direct_accumulators(pl.n_tile);
     // room for this CTA's slice of TileOffsets (K tiles of the longest part, plus one), up to 8 KB
     const int longest = (k_tiles + pl.cluster_k * pl.workspace_k - 1) / (pl.cluster_k * pl.workspace_k) + 1;
     pl.offsets_staged = longest + 1 <= 2048 ? ((longest + 1 + 3) / 4) * 4 : 0;
     // Room of its own for the peers' partial sums where it costs no resident CTA: they may then arrive while this CTA still
     // multiplies.  (Wide outputs take the operands' buffers, once everybody's MMAs are over.)
-    if (direct && pl.cluster_k > 1) {
+    if (direct && pl.cluster_k > 1 && pl.n_tile <= kPushMaxN) {
         pl.sum_bytes   = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
         const int room = two_resident ? kSmemPerSm / 2 - 1024 : st->smem_optin;
         if (plan_smem_bytes(pl) > room)
@@ -593,7 +647,7 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
                     // the fp32 partial tiles of the cluster reduction are parked over the pipeline buffers
                     && pl.smem_bytes - 1024 - 4 * pl.offsets_staged >= pl.n_tile * kTileM * 4
                     && (!direct || pl.cluster_k == 1 || pl.sum_bytes > 0
-                        || pl.a_stages * kDenseTileBytes + pl.b_stages * pl.b_batch * slab >= cluster_sum_bytes(pl.n_tile, pl.cluster_k));
+                        || pl.n_tile > kPushMaxN || pl.a_stages * kDenseTileBytes + pl.b_stages * pl.b_batch * slab >= cluster_sum_bytes(pl.n_tile, pl.cluster_k));
     if (!ok)
         return cudaErrorInvalidConfiguration;
     *out = pl;

@@ -198,12 +198,25 @@ constexpr int kPrefetchAhead = FLASHLLM_PREFETCH_AHEAD;
 // Warps of the register-streaming kernel: one B loader, kDirectIssuers MMA issuers, then the scatter warps.
 constexpr int kDirectIssuers = 2;
 
+// The most accumulators that the tiles of a CTA may take turns with (plan.accumulators: this many or kDirectIssuers).  The
+// tensor core truncates every addition, so a sum's error grows with the tiles added up in one accumulator: with four of them a
+// K range may be twice as long as with two.
+__host__ __device__ constexpr int direct_accumulators(int n_tile)
+{
+    return n_tile <= 64 ? 2 * kDirectIssuers : kDirectIssuers;
+}
+
 // Sum over the CTAs of a cluster: rank q finishes rows [128 q / S, 128 (q + 1) / S) of the output tile, and every CTA sends it
 // those rows of its partial tile, [S ranks][rows][columns + 4 for the banks' sake].  The stores count themselves in on the
 // receiver's mbarrier, so nobody asks a peer for data or waits for it beyond that.  With the partial tiles parked at home and
 // fetched between two cluster barriers the sum took 2.4 of the 6.3 us of 1024x1024 N = 8 in clusters of eight.  us per call
 // before and after, with the waits that park the warp in place of sleeping ones: that call 5.6 -> 4.5, 4096x4096 N = 16
 // (eight) 9.9 -> 8.7, 9216x1152 N = 16 (three) 9.1 -> 8.1, 4736x7232 N = 32 (seven) 19.0 -> 18.6.
+//
+// 128 columns are parked at home and fetched as before: a row per lane makes for stores of 16 bytes to as many places, and
+// 2688x8960 N = 128 in clusters of six takes 16.6 us that way instead of 15.4.
+constexpr int kPushMaxN = 64;
+
 __host__ __device__ constexpr int cluster_sum_rows(int S)
 {
     return (kTileM + S - 1) / S;
@@ -229,19 +242,24 @@ __device__ __forceinline__ void accumulators_to_peers(uint32_t tmem_acc, int acc
     const uint32_t to  = ptx::map_to_rank(sum_base, q)
                         + static_cast<uint32_t>((rank * cluster_sum_rows(S) + row - kTileM * q / S) * (N_TILE + 4)) * 4u;
     const uint32_t acc = tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16);
+    constexpr int  A   = direct_accumulators(N_TILE);
     for (int c0 = col_begin; c0 < col_end; c0 += 8) {
         float    v[8];
-        uint32_t t[8];
+        uint32_t t[A][8];
+#pragma unroll
+        for (int a = 0; a < A; ++a)
+            if (a < accumulators)
+                ptx::tmem_ld_x8(acc + a * N_TILE + c0, t[a]);
+        ptx::tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            v[i] = 0.0f;
-        for (int a = 0; a < accumulators; ++a) {
-            ptx::tmem_ld_x8(acc + a * N_TILE + c0, t);
-            ptx::tmem_wait_ld();
+            v[i] = accumulators > 0 ? __uint_as_float(t[0][i]) : 0.0f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                v[i] = a == 0 ? __uint_as_float(t[i]) : v[i] + __uint_as_float(t[i]);
-        }
+        for (int a = 1; a < A; ++a)
+            if (a < accumulators)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    v[i] += __uint_as_float(t[a][i]);
         ptx::st_async_v4_f32(to + c0 * 4, v, bar);
         ptx::st_async_v4_f32(to + c0 * 4 + 16, v + 4, bar);
     }
@@ -304,7 +322,7 @@ __device__ __forceinline__ void finish_cluster_rows(const SpmmParams& p, uint32_
 //
 // One thread cannot issue tcgen05.mma as fast as the tensor core retires them (measured: 4 MMAs and the commit that
 // hands a stage back cost an issuing thread ~400 cycles, the tensor core ~180), so tiles alternate between
-// kDirectIssuers issuing threads, each with an accumulator of its own in tensor memory; the epilogue adds them.
+// kDirectIssuers issuing threads, each with accumulators of its own in tensor memory; the epilogue adds them.
 template<int N_TILE, int CAP, int WARPS, int MIN_BLOCKS, int WPT = 1>
 __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_BLOCKS)
     spmm_tcgen05_direct_kernel(const __grid_constant__ CUtensorMap tmap_b, const SpmmParams p)
@@ -316,7 +334,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     constexpr uint32_t kBSlab    = N_TILE * kTileK * 2;  // one K tile of B in shared memory
     constexpr int      MI        = kDirectIssuers;
     static_assert(WARPS % MI == 0, "every issuer serves the same stages on every lap");
-    constexpr uint32_t kTmemCols = MI * N_TILE < 32 ? 32 : MI * N_TILE;  // a power of two for MI = 2
+    constexpr uint32_t kTmemCols = direct_accumulators(N_TILE) * N_TILE;  // a power of two
     constexpr int      NSW       = WARPS * WPT;  // scatter warps
     constexpr int      a_stages  = WARPS;
 
@@ -340,6 +358,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     const int       KB       = plan.b_batch;
     const int       S        = plan.cluster_k;
     const int       G        = plan.workspace_k;
+    const int       accs     = plan.accumulators;  // a power of two
     constexpr int   b_warp   = 0;  // warp that loads B
     constexpr int   mma_warp = 1;       // first of the MI warps that issue MMAs; it owns the TMEM allocation
     constexpr int   first_sw = 1 + MI;  // first scatter warp
@@ -454,7 +473,8 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     }
     const uint32_t tmem_acc = *tmem_slot;
     const int      n_valid  = (p.N - n_idx * N_TILE) < N_TILE ? (p.N - n_idx * N_TILE) : N_TILE;
-    if (S > 1) {
+    constexpr bool kPush = N_TILE <= kPushMaxN;
+    if (kPush && S > 1) {
         if (threadIdx.x == 0)  // everything the peers (and this CTA) will store here
             ptx::mbar_arrive_expect_tx(sum_full,
                                        static_cast<uint32_t>(S * (kTileM * (rank + 1) / S - kTileM * rank / S) * n_valid) * 4u);
@@ -486,7 +506,6 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
                 const uint32_t idesc   = ptx::umma_idesc_f16_f32(kTileM, N_TILE);
                 const uint64_t a_desc0 = ptx::umma_desc_kmajor_sw128(a_base);
                 const uint64_t b_desc0 = ptx::umma_desc_kmajor_sw128(b_base);
-                const uint32_t acc     = tmem_acc + static_cast<uint32_t>(m * N_TILE);
                 int            s = m, bs = 0, kb = m;
                 uint32_t       a_par = 0, b_par = 0;
                 bool           ready = false, first_in_batch = true;
@@ -525,8 +544,8 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
                     if (false)
 #endif
                     ready = ptx::umma_tile_commit_probe(
-                        acc, a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
-                        b_desc0 + static_cast<uint32_t>((bs * KB + kb) * (kBSlab >> 4)), idesc, j != m ? 1u : 0u, a_empty + 8u * s,
+                        tmem_acc + static_cast<uint32_t>((j & (accs - 1)) * N_TILE), a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
+                        b_desc0 + static_cast<uint32_t>((bs * KB + kb) * (kBSlab >> 4)), idesc, j >= accs ? 1u : 0u, a_empty + 8u * s,
                         b_empty + 8u * bs, (batch_done || !has_next) ? 1u : 0u, a_full + 8u * s_n, a_par_n, b_full + 8u * bs_n,
                         b_par_n, has_next ? 1u : 0u, (has_next && batch_done) ? 1u : 0u);
                     if (m == 0)
@@ -645,13 +664,22 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
         if (sw == 0 && lane == 0)
             FL_CTA_TIME(2);
 
-        if (S == 1)
-            accumulators_to_output<N_TILE>(p, tmem_acc, L < MI ? L : MI, N_TILE, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, 1, G, g, n_idx,
-                                           tile_row, acc_ok, nullptr);
+        if (!kPush || S == 1)
+            accumulators_to_output<N_TILE>(p, tmem_acc, L < accs ? L : accs, N_TILE, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, G, g, n_idx,
+                                           tile_row, acc_ok, reinterpret_cast<float*>(smem));
     }
 
     // ================================================================ cluster reduction and tear-down
-    if (S > 1) {
+    if (!kPush && S > 1) {
+        __syncwarp();
+        ptx::cluster_sync_all();  // every CTA's partial tile is parked in its shared memory
+        if (warp >= first_sw)
+            cluster_reduce_store<N_TILE>(p, base, rank, S, G, g, n_idx, tile_row, threadIdx.x - first_sw * 32, NTS,
+                                         *abort_flag == 0u);
+        __syncwarp();
+        ptx::cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
+    }
+    else if (S > 1) {
         __syncwarp();
         if (plan.sum_bytes > 0)
             ptx::cluster_wait();  // long over: the peers have started
@@ -659,7 +687,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
             ptx::cluster_sync_all();  // nobody multiplies any more, the stages are free
         if (warp >= first_sw) {
             ptx::tc_fence_after_sync();
-            accumulators_to_peers<N_TILE>(tmem_acc, L < MI ? L : MI, n_valid, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, rank, sum_base,
+            accumulators_to_peers<N_TILE>(tmem_acc, L < accs ? L : accs, n_valid, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, rank, sum_base,
                                           sum_full);
             if (__all_sync(0xFFFFFFFFu, wait_bounded_cluster(sum_full, 0u, abort_flag, p.status)) && *abort_flag == 0u)
                 finish_cluster_rows<N_TILE>(p, sum_base, rank, S, G, g, n_idx, tile_row, n_valid, threadIdx.x - first_sw * 32, NTS);

@@ -371,9 +371,9 @@ __device__ __forceinline__ void accumulators_to_output(const SpmmParams& p, uint
         }
         else
             load(acc + c0, r);
-        if (accumulators == 2) {
+        for (int a = 1; a < accumulators; ++a) {
             float more[BATCH];
-            load(acc + acc_stride + c0, more);
+            load(acc + a * acc_stride + c0, more);
 #pragma unroll
             for (int i = 0; i < BATCH; ++i)
                 r[i] += more[i];
