@@ -75,7 +75,7 @@ int FlashLLM_EncodeOnDevice_TileOffsets(void* stream, const void* A_d, int M, in
         return rc;
     const int    k_tiles = K / kTileK, tiles = (M / kTileM) * k_tiles;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaError_t  e = launch_in_stream_order(csl_count_kernel, dim3((tiles + kCountTiles - 1) / kCountTiles), dim3(kEncodeWarps * 32),
+    cudaError_t  e = launch_in_stream_order(csl_count_kernel, dim3((tiles + kCountTiles - 1) / kCountTiles), dim3(kCountWarps * 32),
                                            0, s, 1, static_cast<const uint16_t*>(A_d), K, tiles, k_tiles, TileOffsets_d);
     if (e == cudaSuccess)
         e = launch_in_stream_order(csl_scan_kernel, dim3(1), dim3(1024), 0, s, 1, TileOffsets_d, tiles, status);

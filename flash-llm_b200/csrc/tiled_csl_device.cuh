@@ -10,7 +10,7 @@
 //
 // Bound by HBM: the dense matrix has to be read twice, because the size of the result is only known after the first pass.
 // 36864x9216 at 80 % (680 MB dense, 272 MB of words), both passes with the host's wait and
-// the allocation between them: 327 us (906 with every tile read twice and its words stored one by one); counting alone
+// the allocation between them: 322 us (906 with every tile read twice and its words stored one by one); counting alone
 // 113 us, 6.0 TB/s.
 #pragma once
 #include <cuda_fp16.h>
@@ -76,35 +76,37 @@ __device__ __forceinline__ const uint16_t* tile_start(const uint16_t* A, int K, 
 }
 
 // Step 1a: offs[t + 1] = 16-byte vectors (non-zeros rounded up to a multiple of four) of tile t and of the tiles before it
-// in its CTA's group of kCountTiles.  A warp counts four neighbouring tiles, eight lanes to a tile and 16 bytes to a lane,
-// so that it reads 512 bytes of a row in one piece; counts are kept in fp16 pairs, exact up to 2048 and never above 512
-// here.
-constexpr int kCountTiles = kEncodeWarps * 4;
+// in its CTA's group of kCountTiles.  A warp counts a quarter of the rows of four neighbouring tiles, eight lanes to a tile and
+// 16 bytes to a lane, so that it reads 512 bytes of a row in one piece; counts are kept in fp16 pairs, exact up to 2048 and
+// never above 128 here.  (With one warp to all rows of its tiles the counts of 1024x1024 took eight memory latencies in a row:
+// both launches of this step 12.2 us, in quarters 8.0; an encoding of 36864x9216 in all 326 -> 323.)
+constexpr int kCountTiles = 32, kCountRowParts = 4, kCountWarps = kCountTiles / 4 * kCountRowParts;
 
-__global__ void __launch_bounds__(kEncodeWarps * 32)
+__global__ void __launch_bounds__(kCountWarps * 32)
     csl_count_kernel(const uint16_t* A, int K, int tiles, int k_tiles, int* offs)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
-    __shared__ int s_vectors[kCountTiles];
+    __shared__ int s_words[kCountRowParts][kCountTiles];
     static_assert(kCountTiles == 32, "one lane per tile of the group");
-    const int lane = threadIdx.x & 31;
-    const int slot = (threadIdx.x >> 5) * 4 + (lane >> 3);
+    constexpr int kRows = kTileM / kCountRowParts;
+    const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % kCountRowParts;
+    const int slot = (threadIdx.x >> 5) / kCountRowParts * 4 + (lane >> 3);
     const int t    = blockIdx.x * kCountTiles + slot;
     uint32_t  n2   = 0;
     if (t < tiles) {
-        const uint16_t* src   = tile_start(A, K, k_tiles, t) + (lane & 7) * 8;
+        const uint16_t* src   = tile_start(A, K, k_tiles, t) + static_cast<size_t>(part * kRows) * K + (lane & 7) * 8;
         auto            count = [&](uint4 v) {
             n2 = add_f16x2(n2, add_f16x2(add_f16x2(kept_pair(v.x), kept_pair(v.y)), add_f16x2(kept_pair(v.z), kept_pair(v.w))));
         };
         if ((reinterpret_cast<uintptr_t>(A) & 15u) == 0) {
 #pragma unroll 16
-            for (int r = 0; r < kTileM; ++r)
+            for (int r = 0; r < kRows; ++r)
                 count(*reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * K));
         }
         else {  // A is 4-byte aligned
 #pragma unroll 4
-            for (int r = 0; r < kTileM; ++r) {
+            for (int r = 0; r < kRows; ++r) {
                 const uint32_t* row = reinterpret_cast<const uint32_t*>(src + static_cast<size_t>(r) * K);
                 count(make_uint4(row[0], row[1], row[2], row[3]));
             }
@@ -115,10 +117,14 @@ __global__ void __launch_bounds__(kEncodeWarps * 32)
     for (int d = 1; d < 8; d <<= 1)
         n += __shfl_xor_sync(0xFFFFFFFFu, n, d);
     if ((lane & 7) == 0)
-        s_vectors[slot] = (n + kVectorWords - 1) / kVectorWords;
+        s_words[part][slot] = n;
     __syncthreads();
     if (threadIdx.x < 32) {
-        int v = s_vectors[lane];
+        int words = 0;
+#pragma unroll
+        for (int i = 0; i < kCountRowParts; ++i)
+            words += s_words[i][lane];
+        int v = (words + kVectorWords - 1) / kVectorWords;
         for (int d = 1; d < 32; d <<= 1) {
             const int below = __shfl_up_sync(0xFFFFFFFFu, v, d);
             v += lane >= d ? below : 0;
