@@ -3,6 +3,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <fstream>
@@ -82,6 +83,25 @@ int FlashLLM_EncodeOnDevice_TileOffsets(void* stream, const void* A_d, int M, in
     return static_cast<int>(e);
 }
 
+// SMs of the current device, whose first packing also sets the reordering kernel's carveout there: its grid is persistent, and
+// L1, which holds the loads in flight, keeps what kPackCtasPerSm CTAs' shared memory leaves of 228 KB.
+static cudaError_t pack_grid(int* sms)
+{
+    constexpr int           kDevices = 64;
+    static std::atomic<int> known[kDevices];
+    int                     device = 0;
+    cudaError_t             e      = cudaGetDevice(&device);
+    if (e == cudaSuccess && device >= 0 && device < kDevices && (*sms = known[device].load(std::memory_order_relaxed)) > 0)
+        return cudaSuccess;
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(csl_pack_reorder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kPackCarveoutPercent);
+    if (e == cudaSuccess && device >= 0 && device < kDevices)
+        known[device].store(*sms, std::memory_order_relaxed);
+    return e;
+}
+
 int FlashLLM_EncodeOnDevice_Pack(void* stream, const void* A_d, int M, int K, const int* TileOffsets_d,
                                  uint32_t* Compressed_A_d, int reorder)
 {
@@ -100,13 +120,8 @@ int FlashLLM_EncodeOnDevice_Pack(void* stream, const void* A_d, int M, int K, co
     };
     if (!reorder)
         return launch(csl_pack_scan_kernel, (tiles + kEncodeWarps - 1) / kEncodeWarps, kEncodeWarps);
-    // A persistent grid; L1 keeps what kPackCtasPerSm CTAs' shared memory leaves of 228 KB (it holds the loads in flight).
-    int         device = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess)
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(csl_pack_reorder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kPackCarveoutPercent);
+    int               sms = 0;
+    const cudaError_t e   = pack_grid(&sms);
     if (e != cudaSuccess)
         return static_cast<int>(e);
     const int groups = (tiles + kEncodeWarps - 1) / kEncodeWarps;

@@ -98,13 +98,15 @@ std::tuple<at::Tensor, at::Tensor> encode(const at::Tensor& A)
     int                        code    = g_tile_offsets(stream, A.const_data_ptr(), static_cast<int>(M), static_cast<int>(K), offs_d);
     if (code != 0)
         raise_library_error("EncodeOnDevice_TileOffsets", code);
-    int vectors = 0;  // the size of the result depends on the data: the one wait of an encoding
-    code        = cudaMemcpyAsync(&vectors, offs_d + tiles + 1, sizeof(int), cudaMemcpyDeviceToHost, stream);
+    // The size of the result depends on the data: the one wait of an encoding.  Through page-locked memory (PyTorch's pool of
+    // it), a copy to any other is staged.
+    const at::Tensor size = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    code = cudaMemcpyAsync(size.mutable_data_ptr(), offs_d + tiles + 1, sizeof(int), cudaMemcpyDeviceToHost, stream);
     if (code == 0)
         code = cudaStreamSynchronize(stream);
     if (code != 0)
         raise_library_error("reading the size of the encoding", code);
-    const int64_t    words = static_cast<int64_t>(vectors) * 4;
+    const int64_t    words = static_cast<int64_t>(*static_cast<const int*>(size.const_data_ptr())) * 4;
     const at::Tensor comp  = at::empty({words > 4 ? words : 4}, options);
     code = g_pack(stream, A.const_data_ptr(), static_cast<int>(M), static_cast<int>(K), offs_d,
                   static_cast<uint32_t*>(comp.mutable_data_ptr()), 1);
