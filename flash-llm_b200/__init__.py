@@ -38,6 +38,7 @@ from .api import (  # noqa: F401
     splitk_reduction,
     spmm_splitk_bias_act,
     spmm_splitk_epilogue,
+    spmm_splitk_strided,
     spmm_splitk_allreduce,
     spmm_splitk_no_alloc,
     write_rank_lists,

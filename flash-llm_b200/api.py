@@ -52,6 +52,9 @@ def library() -> C.CDLL:
     L.FlashLLM_SpMM_SplitK_Epilogue.restype = C.c_int
     L.FlashLLM_SpMM_SplitK_Epilogue.argtypes = ([C.c_void_p] * 5 + [C.c_int] * 3
                                                 + [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p])
+    L.FlashLLM_SpMM_SplitK_Strided.restype = C.c_int
+    L.FlashLLM_SpMM_SplitK_Strided.argtypes = ([C.c_void_p] * 4 + [C.c_int, C.c_void_p] + [C.c_int] * 3
+                                               + [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p])
     for name in ("FlashLLM_InitSparseMatrixA", "FlashLLM_InitSparseMatrixA_NoReorder"):
         f = getattr(L, name)
         f.restype = C.c_int
@@ -260,6 +263,17 @@ def spmm_splitk_epilogue(stream: int, Compressed_A: int, TileOffsets: int, B: in
                                                    Reduction_Workspace, Split_K, bias, activation, residual)
     if code:
         _check(code, f"SpMM_SplitK_Epilogue(M={M}, N={N}, K={K}, Split_K={Split_K})")
+
+
+def spmm_splitk_strided(stream: int, Compressed_A: int, TileOffsets: int, B: int, ldb: int, C_out: int, M: int, N: int, K: int,
+                        Reduction_Workspace: int | None, Split_K: int, bias: int | None = None,
+                        activation: int = ACT_NONE, residual: int | None = None) -> None:
+    """``spmm_splitk_epilogue`` for a B whose rows lie ``ldb`` halves apart (``ldb >= K`` and a multiple of 8): a slice of
+    the columns of a wider matrix."""
+    code = library().FlashLLM_SpMM_SplitK_Strided(stream, Compressed_A, TileOffsets, B, ldb, C_out, M, N, K,
+                                                  Reduction_Workspace, Split_K, bias, activation, residual)
+    if code:
+        _check(code, f"SpMM_SplitK_Strided(M={M}, N={N}, K={K}, ldb={ldb}, Split_K={Split_K})")
 
 
 def spmm_splitk_no_alloc(stream: int, Compressed_A: int, TileOffsets: int, B: int, C_out: int, M: int, N: int, K: int,

@@ -655,11 +655,11 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
 }
 
 // B as a 3-D tensor {64 K-elements (inner), N, K/64}: one box = b_batch K tiles of [n_tile x 64] (wide form: of one MMA's columns), each stored as a
-// 128-byte-swizzled slab; rows past N and K tiles past K/64 read as 0.
-static cudaError_t encode_b_map(const half* B, int N, int K, const SpmmPlan& pl, CUtensorMap* map)
+// 128-byte-swizzled slab; rows past N and K tiles past K/64 read as 0.  ldb: halves from one row of B to the next.
+static cudaError_t encode_b_map(const half* B, int N, int K, int ldb, const SpmmPlan& pl, CUtensorMap* map)
 {
     const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(kTileK), static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(K / kTileK)};
-    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K) * 2, static_cast<cuuint64_t>(kTileK) * 2};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ldb) * 2, static_cast<cuuint64_t>(kTileK) * 2};
     const int        columns    = pl.path == kPathWide ? wide_mma_n(pl.n_tile) : pl.n_tile;
     const cuuint32_t box[3]     = {static_cast<cuuint32_t>(kTileK), static_cast<cuuint32_t>(columns),
                                    static_cast<cuuint32_t>(pl.b_batch)};
@@ -674,12 +674,12 @@ static cudaError_t encode_b_map(const half* B, int N, int K, const SpmmPlan& pl,
 // K cuts and the tensor map's encoding are 2 us of each, a third of a small call.  The map's address is set on every call.
 struct CallKey {
     const DeviceState* device;
-    int                M, N, K, max_parts;
+    int                M, N, K, ldb, max_parts;
     bool               sends, may_stream, overlap;
     unsigned           override_version;
     bool operator==(const CallKey& o) const
     {
-        return device == o.device && M == o.M && N == o.N && K == o.K && max_parts == o.max_parts && sends == o.sends
+        return device == o.device && M == o.M && N == o.N && K == o.K && ldb == o.ldb && max_parts == o.max_parts && sends == o.sends
                && may_stream == o.may_stream && overlap == o.overlap && override_version == o.override_version;
     }
 };
@@ -830,7 +830,8 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
                                    const half*  residual = nullptr,
                                    FlashLLMComm* comm = nullptr,
                                    int           phases = 3,
-                                   bool          may_allocate = true)
+                                   bool          may_allocate = true,
+                                   int           ldb          = 0)  // halves between the rows of B, 0 = K_Global
 {
     if (!n_supported(N_Global)) {
         printf("MM_Sparse_API Error: Unsupported N dimension %d!\n", N_Global);
@@ -839,7 +840,7 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
     if (M_Global <= 0 || K_Global <= 0 || M_Global % kTileM != 0 || K_Global % kTileK != 0 || Split_K < 1
         || Compressed_A == nullptr || TileOffsets == nullptr || B == nullptr || C == nullptr
         || (reinterpret_cast<uintptr_t>(Compressed_A) & 15u) != 0 || (reinterpret_cast<uintptr_t>(B) & 15u) != 0
-        || (reinterpret_cast<uintptr_t>(C) & 1u) != 0 || (Split_K > 1 && Reduction_Workspace == nullptr))
+        || (ldb != 0 && (ldb < K_Global || ldb % 8 != 0)) || (reinterpret_cast<uintptr_t>(C) & 1u) != 0 || (Split_K > 1 && Reduction_Workspace == nullptr))
         return cudaErrorInvalidValue;
 
     cudaError_t  err = cudaSuccess;
@@ -851,7 +852,7 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
 
     SpmmParams params{};
     SpmmPlan&  pl = params.plan;
-    CallKey    key{st,           M_Global,     N_Global, K_Global, comm ? kCommLocalParts : Split_K / 2,
+    CallKey    key{st,           M_Global,     N_Global, K_Global, ldb ? ldb : K_Global, comm ? kCommLocalParts : Split_K / 2,
                 comm != nullptr, may_allocate, g_launch_overlap.load(std::memory_order_relaxed) != 0,
                 g_override_version.load(std::memory_order_relaxed)};
     CallMemo*  memo = nullptr;
@@ -905,7 +906,7 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
             return cudaErrorInvalidValue;
     }
     else {
-        if ((err = encode_b_map(B, N_Global, K_Global, pl, &memo->map)) != cudaSuccess)
+        if ((err = encode_b_map(B, N_Global, K_Global, key.ldb, pl, &memo->map)) != cudaSuccess)
             return err;
         memo->has_map = true;
     }
@@ -1048,6 +1049,29 @@ int FlashLLM_SpMM_SplitK_Epilogue(void*       stream,
                                             static_cast<half*>(Reduction_Workspace), Split_K,
                                             static_cast<const half*>(bias), activation,
                                             static_cast<const half*>(residual)));
+}
+
+int FlashLLM_SpMM_SplitK_Strided(void*       stream,
+                                 const void* Compressed_A,
+                                 const int*  TileOffsets,
+                                 const void* B,
+                                 int         ldb,
+                                 void*       C,
+                                 int         M,
+                                 int         N,
+                                 int         K,
+                                 void*       Reduction_Workspace,
+                                 int         Split_K,
+                                 const void* bias,
+                                 int         activation,
+                                 const void* residual)
+{
+    if ((activation != kActNone && activation != kActRelu) || (residual != nullptr && residual == C) || ldb <= 0)
+        return static_cast<int>(cudaErrorInvalidValue);
+    return static_cast<int>(spmm_launch_all(static_cast<cudaStream_t>(stream), static_cast<const uint4*>(Compressed_A),
+                                            TileOffsets, static_cast<const half*>(B), static_cast<half*>(C), M, N, K,
+                                            static_cast<half*>(Reduction_Workspace), Split_K, static_cast<const half*>(bias),
+                                            activation, static_cast<const half*>(residual), nullptr, 3, true, ldb));
 }
 
 int FlashLLM_SpMM_SplitK(void*       stream,

@@ -195,6 +195,23 @@ int FlashLLM_SpMM_SplitK_Epilogue(void*       stream,
                                   int         activation,
                                   const void* residual);
 
+/* The same for a B whose rows lie `ldb` halves apart (a slice of the columns of a wider matrix, as the V third of a QKV
+ * projection is for the attention output projection): ldb >= K and a multiple of 8, B 16-byte aligned as ever. */
+int FlashLLM_SpMM_SplitK_Strided(void*       stream,
+                                 const void* Compressed_A,
+                                 const int*  TileOffsets,
+                                 const void* B,
+                                 int         ldb,
+                                 void*       C,
+                                 int         M,
+                                 int         N,
+                                 int         K,
+                                 void*       Reduction_Workspace,
+                                 int         Split_K,
+                                 const void* bias,
+                                 int         activation,
+                                 const void* residual);
+
 /* ------------------------------------------------------------------------------------------------------------
  * Row-parallel SpMM with the all-reduce fused in (tensor-parallel inference: the attention output projection and
  * the second feed-forward matmul hold a slice of K on every GPU, so every GPU's product is a partial sum).  The

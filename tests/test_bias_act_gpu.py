@@ -84,3 +84,34 @@ def test_residual_overlapping_the_output_is_refused(lib):
 
 def test_unknown_activation_is_refused(lib):
     assert lib.library().FlashLLM_SpMM_SplitK_BiasAct(None, 0x1000, 0x1000, 0x1000, 0x1000, 128, 16, 64, None, 1, None, 7) == 1
+
+
+@pytest.mark.parametrize("M,K,N,plan", [
+    (384, 64 * 19, 8, {}), (128 * 37, 64 * 40, 32, dict(path=3)), (384, 64 * 19, 64, dict(path=2, cluster_k=3)),
+    (256, 64 * 9, 16, dict(path=1)), (256, 64 * 9, 128, {}), (384, 64 * 9, 256, dict(path=4, producers=2)), (128, 64, 16, {}),
+])
+def test_b_as_a_slice_of_a_wider_matrix(lib, M, K, N, plan):
+    """B's rows further apart than K: the bits of the same B copied out, whatever lies between the rows."""
+    A, B = random_problem(lib, M, K, N, 0.8, 31 + N)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    comp_d, offs_d = torch.from_numpy(comp.view(np.int32)).cuda(), torch.from_numpy(offs).cuda()
+    wide = torch.full((N, 3 * K + 8), float("nan"), dtype=torch.float16, device="cuda")
+    wide[:, K:2 * K] = torch.from_numpy(np.ascontiguousarray(B)).cuda()
+    part = wide[:, K:2 * K]
+    whole = part.contiguous()
+    bias = torch.rand(M, device="cuda").half()
+    got, want = (torch.empty((N, M), dtype=torch.float16, device="cuda") for _ in range(2))
+    stream = torch.cuda.current_stream().cuda_stream
+    lib.set_plan(**plan)
+    try:
+        lib.spmm_splitk_epilogue(stream, comp_d.data_ptr(), offs_d.data_ptr(), whole.data_ptr(), want.data_ptr(), M, N, K, None, 1,
+                                 bias.data_ptr())
+        lib.spmm_splitk_strided(stream, comp_d.data_ptr(), offs_d.data_ptr(), part.data_ptr(), part.stride(0), got.data_ptr(), M, N,
+                                K, None, 1, bias.data_ptr())
+    finally:
+        lib.set_plan()
+    assert torch.equal(got, want) and not torch.isnan(got).any()
+    assert lib.consume_status() == 0
+    for ldb in (K - 8, K + 4, 0, -8):
+        assert lib.library().FlashLLM_SpMM_SplitK_Strided(stream, comp_d.data_ptr(), offs_d.data_ptr(), part.data_ptr(), ldb,
+                                                          got.data_ptr(), M, N, K, None, 1, None, 0, None) != 0
