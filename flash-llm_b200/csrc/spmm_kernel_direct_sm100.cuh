@@ -265,16 +265,27 @@ __device__ __forceinline__ void accumulators_to_peers(uint32_t tmem_acc, int acc
     }
 }
 
-// The rows this CTA finishes, once all its peers' parts are there: added in rank order, four columns per thread.
-template<int N_TILE>
+// The rows this CTA finishes, once all its peers' parts are there (`arrived`): added in rank order, four columns per thread.
+// What a thread's first outputs need from memory is asked for before that.
+template<int N_TILE, typename Arrived>
 __device__ __forceinline__ void finish_cluster_rows(const SpmmParams& p, uint32_t sum_base, int rank, int S, int G, int g, int n_idx,
-                                                    int tile_row, int n_valid, int tid, int threads)
+                                                    int tile_row, int n_valid, int tid, int threads, Arrived arrived)
 {
     const int    row0     = kTileM * rank / S;
     const int    rows     = kTileM * (rank + 1) / S - row0;
     const size_t tile_off = static_cast<size_t>(n_idx) * N_TILE * p.M + static_cast<size_t>(tile_row) * kTileM;
     const uint32_t step  = static_cast<uint32_t>(cluster_sum_rows(S) * (N_TILE + 4)) * 4u;
     const int      shift = 32 - __clz(rows - 1);  // rows, rounded up to a power of two, are 16 to 64
+    const int      r_1   = tid & ((1 << shift) - 1), c_1 = (tid >> shift) * 4;
+    const bool     direct = G == 1 && p.push_world == 0, first = direct && r_1 < rows && c_1 < n_valid;
+    float          bias_1 = -0.0f;
+    half           res_1[4];
+    if (first)
+        bias_1 = bias_of(p, tile_row * kTileM + row0 + r_1);
+    if (first && p.residual != nullptr)
+        load_residual<4>(p, res_1, tile_off + static_cast<size_t>(c_1) * p.M + row0 + r_1);
+    if (!arrived())
+        return;
     for (int e = tid; e < (n_valid / 4) << shift; e += threads) {
         const int r = e & ((1 << shift) - 1), c = (e >> shift) * 4;
         if (r >= rows)
@@ -308,6 +319,8 @@ __device__ __forceinline__ void finish_cluster_rows(const SpmmParams& p, uint32_
                 for (int i = 0; i < 4; ++i)
                     p.push_slot[w][tile_off + at + static_cast<size_t>(i) * p.M] = v[i];
         }
+        else if (e == tid)
+            finish_columns<4>(p, v, tile_off + at, 4, bias_1, res_1);
         else
             finish_columns<4>(p, v, tile_off + at, 4, bias_of(p, tile_row * kTileM + m));
     }
@@ -689,8 +702,9 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
             ptx::tc_fence_after_sync();
             accumulators_to_peers<N_TILE>(tmem_acc, L < accs ? L : accs, n_valid, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, rank, sum_base,
                                           sum_full);
-            if (__all_sync(0xFFFFFFFFu, wait_bounded_cluster(sum_full, 0u, abort_flag, p.status)) && *abort_flag == 0u)
-                finish_cluster_rows<N_TILE>(p, sum_base, rank, S, G, g, n_idx, tile_row, n_valid, threadIdx.x - first_sw * 32, NTS);
+            finish_cluster_rows<N_TILE>(p, sum_base, rank, S, G, g, n_idx, tile_row, n_valid, threadIdx.x - first_sw * 32, NTS, [&]() {
+                return __all_sync(0xFFFFFFFFu, wait_bounded_cluster(sum_full, 0u, abort_flag, p.status)) && *abort_flag == 0u;
+            });
         }
     }
     ptx::tc_fence_before_sync();

@@ -96,7 +96,17 @@ __device__ __forceinline__ float bias_of(const SpmmParams& p, int m)
 }
 
 template<int C>
-__device__ __forceinline__ void finish_columns(const SpmmParams& p, float (&v)[C], size_t at, int columns, float bias)
+__device__ __forceinline__ void load_residual(const SpmmParams& p, half (&res)[C], size_t at)
+{
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+        res[i] = p.residual[at + i * static_cast<size_t>(p.M)];
+}
+
+// `loaded`: the residual's values, where the caller has asked for them before it had the sums.
+template<int C>
+__device__ __forceinline__ void finish_columns(const SpmmParams& p, float (&v)[C], size_t at, int columns, float bias,
+                                               const half* loaded = nullptr)
 {
     if (columns < C)
         return;
@@ -109,12 +119,11 @@ __device__ __forceinline__ void finish_columns(const SpmmParams& p, float (&v)[C
     }
     if (p.residual != nullptr) {
         half res[C];
+        if (loaded == nullptr)
+            load_residual<C>(p, res, at);
 #pragma unroll
         for (int i = 0; i < C; ++i)
-            res[i] = p.residual[at + i * step];
-#pragma unroll
-        for (int i = 0; i < C; ++i)
-            v[i] += __half2float(res[i]);
+            v[i] += __half2float(loaded != nullptr ? loaded[i] : res[i]);
     }
     half* out = p.out + at;
 #pragma unroll
