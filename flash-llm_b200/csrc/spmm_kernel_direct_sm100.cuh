@@ -709,6 +709,11 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     }
     ptx::tc_fence_before_sync();
     __syncthreads();
+    // A CTA that gave up leaves only when its peers have left or given up too: until then they may store into its shared memory.
+    if (kPush && S > 1 && *abort_flag != 0u) {
+        __syncwarp();
+        ptx::cluster_sync_all();
+    }
     finish_tile<N_TILE>(p, S, G, n_idx, tile_row, abort_flag);
     if (threadIdx.x == 0)
         FL_CTA_TIME(3);
