@@ -404,6 +404,9 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
     }
     else {
         // ================================================================ epilogue warps
+        // Bias, residual, parked parts and counters may belong to the stream's earlier work; with launch overlap on nothing has
+        // waited for that here.
+        ptx::grid_dependency_wait();
         const int tid     = threadIdx.x - kStreamFirstEpi * 32;
         const int quarter = warp & 3;  // the tensor-memory lanes this warp may read
         const int r       = quarter * 32 + lane;
@@ -452,7 +455,6 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                 asked             = true;
                 unsigned int seen = 0u;
                 if (look && tid == 0) {
-                    ptx::grid_dependency_wait();  // counters may be in use by the stream's previous launch until it is over
                     seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
                     for (int n = 1; seen == 0u && n < kStreamLooks && !ptx::mbar_test_wait(acc_full + 8u * (q & 1), (q >> 1) & 1u); ++n)
                         seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
@@ -526,7 +528,6 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                     // arrivals in the low half of the counter; a CTA that gave up also marks the high half, so that the
                     // last one knows the row's sum is not to be trusted
                     const unsigned int mine = gave_up ? 0x10001u : 1u;
-                    ptx::grid_dependency_wait();  // (as above)
                     const int          c_first = stream_owner(p, ctas, row_begin);
                     const unsigned int before  = ptx::atom_add_acq_rel_gpu(p.tile_counters + row, mine);
                     if ((before & 0xFFFFu) + 1u == static_cast<unsigned int>(c_last - c_first + 1)) {

@@ -160,3 +160,47 @@ def test_encoding_into_buffers_an_spmm_has_just_read(lib, N, overlap):
     for i, C in enumerate(outs):
         want = (B.double() @ As[i % 2].double().T).float().cpu().numpy()
         assert_close(C.cpu().numpy(), want, f"call {i}")
+
+
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("operand", ["bias", "residual"])
+@pytest.mark.parametrize("N", [16, 64])
+@pytest.mark.parametrize("plan", [dict(path=3), dict(path=2, cluster_k=1), dict(path=2, cluster_k=3)],
+                         ids=["stream", "rows", "clusters"])
+def test_bias_and_residual_written_by_the_call_before(lib, plan, N, operand, overlap):
+    """The call before runs on few SMs and for long, so that the next one's CTAs are there while it still computes what they
+    are to add; the operand holds another call's values until then."""
+    first, second = _Weights(128 * 16, 64 * 256, 0.8, 50), _Weights(128 * 16, 64 * 45, 0.8, 51)
+    X = [_activations(N, first.K, 60 + i) for i in range(3)]
+    Y = _activations(N, second.K, 70)
+    H = torch.full((N, first.M), float("nan"), dtype=torch.float16, device="cuda")
+    outs = [torch.full((N, second.M), float("nan"), dtype=torch.float16, device="cuda") for _ in range(12)]
+    bias, residual = (H.data_ptr(), None) if operand == "bias" else (None, H.data_ptr())
+    stream = torch.cuda.current_stream()
+    lib.release_scratch()
+    torch.cuda.synchronize()
+    lib.set_launch_overlap(overlap)
+    try:
+        for i, C in enumerate(outs):
+            lib.set_plan(path=lib.api.PATH_DIRECT, cluster_k=1)
+            _call(lib, stream, first.words, first.offs, X[i % 3], H, first)
+            lib.set_plan(**plan)
+            lib.spmm_splitk_epilogue(stream.cuda_stream, second.words.data_ptr(), second.offs.data_ptr(), Y.data_ptr(), C.data_ptr(),
+                                     second.M, N, second.K, None, 1, bias, lib.ACT_NONE, residual)
+        torch.cuda.synchronize()
+    finally:
+        lib.set_plan()
+        lib.set_launch_overlap(False)
+    assert lib.consume_status() == 0
+    product = second.exact(Y)
+    added = []  # what the call before computes when it runs alone: a value it rounds the other way may be an ulp of 2^-5
+    lib.set_plan(path=lib.api.PATH_DIRECT, cluster_k=1)
+    try:
+        for x in X:
+            _call(lib, stream, first.words, first.offs, x, H, first)
+            assert_close(H.cpu().numpy(), first.exact(x), "the call before")
+            added.append(H.float().cpu().numpy())
+    finally:
+        lib.set_plan()
+    for i, C in enumerate(outs):
+        assert_close(C.cpu().numpy(), product + (added[i % 3][:1] if operand == "bias" else added[i % 3]), f"call {i}")

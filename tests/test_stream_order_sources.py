@@ -36,3 +36,13 @@ def test_every_kernel_waits_for_its_predecessors():
             assert "grid_dependency_wait()" in code[kernel.end():end], kernel.group(0)
             kernels += 1
     assert kernels >= 12
+
+
+def test_the_streaming_epilogue_waits_before_it_reads_anything():
+    """The epilogue warps read bias, residual, parked parts and counters, all of which earlier work in the stream may be
+    writing; with launch overlap on they have not waited for it at the kernel's top."""
+    code = _code(os.path.join(ROOT, "flash-llm_b200", "csrc", "spmm_kernel_stream_sm100.cuh"))
+    body = code[code.index("spmm_tcgen05_stream_kernel("):]
+    epilogue = body[re.search(r"else if \(warp < kStreamFirstEpi\).*?else \{", body, re.S).end():]
+    before = epilogue[:epilogue.index("grid_dependency_wait()")]
+    assert not re.search(r"\bp\.|bias_of|load_residual|for\s*\(|if\s*\(", before), before
