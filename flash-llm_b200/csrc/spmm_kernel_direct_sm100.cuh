@@ -226,10 +226,11 @@ __host__ __device__ constexpr int cluster_sum_bytes(int n_tile, int S)
     return S * cluster_sum_rows(S) * (n_tile + 4) * 4;
 }
 
-// One scatter warp's share of the accumulators (as in accumulators_to_output) to the CTAs that finish its rows.
+// One scatter warp's share of the accumulators (as in accumulators_to_output) to the CTAs that finish its rows; NaN from a
+// CTA that gave up, whose tensor memory may hold anything.
 template<int N_TILE>
 __device__ __forceinline__ void accumulators_to_peers(uint32_t tmem_acc, int accumulators, int n_valid, int quarter, int lane, int sw,
-                                                      int per_quarter, int S, int rank, uint32_t sum_base, uint32_t sum_bar)
+                                                      int per_quarter, int S, int rank, uint32_t sum_base, uint32_t sum_bar, bool ok)
 {
     if (sw >= 4 * per_quarter)
         return;
@@ -260,6 +261,9 @@ __device__ __forceinline__ void accumulators_to_peers(uint32_t tmem_acc, int acc
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     v[i] += __uint_as_float(t[a][i]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            v[i] = ok ? v[i] : __int_as_float(0x7FFFFFFF);
         ptx::st_async_v4_f32(to + c0 * 4, v, bar);
         ptx::st_async_v4_f32(to + c0 * 4 + 16, v + 4, bar);
     }
@@ -479,7 +483,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     ptx::tc_fence_before_sync();
     bad_slice = __syncthreads_or(bad_slice ? 1 : 0) != 0;
     ptx::tc_fence_after_sync();
-    const bool go = !bad_slice && (*abort_flag == 0u);  // false: every role skips its work and nothing is stored
+    const bool go = !bad_slice && (*abort_flag == 0u);  // false: every role skips its work and no sum leaves this CTA
     if (bad_slice && threadIdx.x == 0) {
         atomicOr(p.status, kStatusBadTileOffsets);
         *abort_flag = 1u;
@@ -502,6 +506,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     if (threadIdx.x == 0)
         FL_CTA_TIME(1);
 
+    bool acc_ok = false;  // scatter warps: the CTA's sums are complete
     if (warp == b_warp) {
         // ================================================================ B loader: KB K tiles per TMA instruction
         if (lane == 0 && L > 0 && go) {
@@ -669,7 +674,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
         }
 
         // ================================================================ epilogue (same warps)
-        bool acc_ok = go;
+        acc_ok = go;
         if (L > 0 && go)
             acc_ok = wait_bounded_converged(acc_full, 0u, abort_flag, p.status);
         acc_ok = __all_sync(0xFFFFFFFFu, acc_ok && (*abort_flag == 0u));
@@ -701,7 +706,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
         if (warp >= first_sw) {
             ptx::tc_fence_after_sync();
             accumulators_to_peers<N_TILE>(tmem_acc, L < accs ? L : accs, n_valid, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, rank, sum_base,
-                                          sum_full);
+                                          sum_full, acc_ok);
             finish_cluster_rows<N_TILE>(p, sum_base, rank, S, G, g, n_idx, tile_row, n_valid, threadIdx.x - first_sw * 32, NTS, [&]() {
                 return __all_sync(0xFFFFFFFFu, wait_bounded_cluster(sum_full, 0u, abort_flag, p.status)) && *abort_flag == 0u;
             });

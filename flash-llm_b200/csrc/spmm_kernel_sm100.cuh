@@ -347,7 +347,7 @@ __device__ __forceinline__ void load_b_batches(const CUtensorMap* tmap, int batc
 // first 4 * per_quarter scatter warps split the N_TILE columns, the others idle), summed over the `accumulators`
 // accumulators that hold tiles (they lie `acc_stride` columns apart; 0 of them = an empty K range, output 0), then
 // stored as fp16 C, as an fp32 partial tile in the workspace, or parked in shared memory (`red`, [N_TILE][128] fp32
-// over the idle A stages) for the cluster sum.
+// over the idle A stages) for the cluster sum.  A CTA that gave up stores nothing, and parks NaN: its peers add it up.
 template<int N_TILE, int BATCH = 8>
 __device__ __forceinline__ void accumulators_to_output(const SpmmParams& p, uint32_t tmem_acc, int accumulators, int acc_stride,
                                                        int quarter, int lane, int sw, int per_quarter, int S, int G, int g,
@@ -390,7 +390,7 @@ __device__ __forceinline__ void accumulators_to_output(const SpmmParams& p, uint
         if (S > 1) {
 #pragma unroll
             for (int i = 0; i < BATCH; ++i)
-                red[(c0 + i) * kTileM + row_in_tile] = r[i];
+                red[(c0 + i) * kTileM + row_in_tile] = acc_ok ? r[i] : __int_as_float(0x7FFFFFFF);
         }
         else if (acc_ok) {
             const size_t at = static_cast<size_t>(c0) * p.M + row_in_tile;
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     ptx::tc_fence_before_sync();
     bad_slice = __syncthreads_or(bad_slice ? 1 : 0) != 0;
     ptx::tc_fence_after_sync();
-    const bool go = !bad_slice && (*abort_flag == 0u);  // false: every role skips its work and nothing is stored
+    const bool go = !bad_slice && (*abort_flag == 0u);  // false: every role skips its work and no sum leaves this CTA
     if (bad_slice && threadIdx.x == 0) {
         atomicOr(p.status, kStatusBadTileOffsets);
         *abort_flag = 1u;

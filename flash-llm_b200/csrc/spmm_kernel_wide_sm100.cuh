@@ -124,7 +124,7 @@ __global__ void __launch_bounds__((kWideFirstScatter + wide_a_stages(N_TILE)) * 
     bad_slice = __syncthreads_or(bad_slice ? 1 : 0) != 0;
     ptx::tc_fence_after_sync();
     const bool aligned = (base & 1023u) == 0u;
-    const bool go      = aligned && !bad_slice;  // false: every role skips its work and nothing is stored
+    const bool go      = aligned && !bad_slice;  // false: every role skips its work and no sum leaves this CTA
     if (!go && threadIdx.x == 0) {
         atomicOr(p.status, bad_slice ? kStatusBadTileOffsets : kStatusSmemMisaligned);
         *abort_flag = 1u;

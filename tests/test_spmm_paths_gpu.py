@@ -184,6 +184,29 @@ def test_malformed_offsets_are_reported_not_followed(lib, oracle, form):
     assert lib.consume_status() == 0
 
 
+@pytest.mark.parametrize("form,N", [(f, N) for f in FORMS for N in (16, 64, 128)] + [(dict(path=4, producers=2), 256)],
+                         ids=[f"{i}-{N}" for i in FORM_IDS for N in (16, 64, 128)] + ["wide-256"])
+def test_a_cta_that_gives_up_does_not_leave_its_cluster_with_wrong_sums(lib, oracle, form, N):
+    """Of a tile row's three CTAs the first finds its offsets malformed: the row's outputs are not stored or not a number,
+    never what happened to lie in tensor memory; the other row is as ever."""
+    M, K = 256, 1024
+    A, B = random_problem(lib, M, K, N, 0.8, 43)
+    comp, offs, _ = lib.InitSparseMatrixA_API(A)
+    want = oracle.gemm_f32(A, B)
+    bad = offs.copy()
+    bad[3] = bad[2] - 3
+    lib.set_plan(cluster_k=3, **form)
+    try:
+        for _ in range(2):  # the second time tensor memory holds the sums of a good call
+            got = DeviceProblem(lib, comp, bad, B, M, N, K, 1).run(check_status=False)
+            assert lib.consume_status() & 2
+            assert np.isnan(got[:, :128]).all()
+            assert_close(got[:, 128:], want[:, 128:], "the other row")
+            assert_close(DeviceProblem(lib, comp, offs, B, M, N, K, 1).run(), want, "call after a malformed one")
+    finally:
+        lib.set_plan()
+
+
 @pytest.mark.parametrize("form", FORMS, ids=FORM_IDS)
 @pytest.mark.parametrize("N", [256, 384])
 def test_n_beyond_one_mma_tile(lib, oracle, form, N):
