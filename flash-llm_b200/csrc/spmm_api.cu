@@ -287,7 +287,8 @@ static std::atomic<int> g_launch_overlap{0};
 
 
 constexpr int kDefaultPath = kPathDirect;
-constexpr int kSmemPerSm   = 228 * 1024;  // for all resident CTAs, 1 KB of it each for the system
+constexpr int kSmemPerSm   = 228 * 1024;  // for all resident CTAs, 1 KB of it each for the system; L1 then keeps 28 KB
+constexpr int kSmemForL1   = 196 * 1024;  // the next lower carveout, with 60 KB of L1
 
 static int n_tile_for(int N)
 {
@@ -620,10 +621,15 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     const int longest = (k_tiles + pl.cluster_k * pl.workspace_k - 1) / (pl.cluster_k * pl.workspace_k) + 1;
     pl.offsets_staged = longest + 1 <= 2048 ? ((longest + 1 + 3) / 4) * 4 : 0;
     // Room of its own for the peers' partial sums where it costs no resident CTA: they may then arrive while this CTA still
-    // multiplies.  (Wide outputs take the operands' buffers, once everybody's MMAs are over.)
+    // multiplies.  (Wide outputs take the operands' buffers, once everybody's MMAs are over.)  That saves a call 0.1 to 0.6 us,
+    // but an L1 too small for the loads in flight (8 warps x 13 rows of 512 bytes at 80 %) costs every tile: two CTAs of 32
+    // columns with such room leave 28 KB, and 9216x36864 70 % in clusters of two took 102.5 us instead of 97.8.  They have it
+    // for short K ranges only; time without it / with it by tiles per CTA (72 x 4 and 148 x 2 CTAs, 65 to 80 %): overlap off
+    // 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %: 1.00 .. 1.07).
     if (direct && pl.cluster_k > 1 && pl.n_tile <= kPushMaxN) {
-        pl.sum_bytes   = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
-        const int room = two_resident ? kSmemPerSm / 2 - 1024 : st->smem_optin;
+        pl.sum_bytes       = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
+        const bool short_k = (k_tiles + parts - 1) / parts <= (overlap ? 16 : 4);
+        const int  room    = two_resident ? (short_k ? kSmemPerSm : kSmemForL1) / 2 - 1024 : st->smem_optin;
         if (plan_smem_bytes(pl) > room)
             pl.sum_bytes = 0;
     }

@@ -108,6 +108,41 @@ def test_cluster_sums_of_every_width(lib, oracle, form, cluster_k, N):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("rows,tiles,cluster_k,N", [
+    (3, 8, 2, 32), (3, 9, 2, 32), (3, 10, 2, 32),     # 4 tiles a CTA and more: the receiving area goes, launch overlap off
+    (3, 32, 2, 32), (3, 33, 2, 32), (3, 115, 7, 32),  # 16 and more: it goes with launch overlap on
+    (100, 38, 2, 32), (100, 38, 2, 64), (40, 33, 7, 64), (12, 16, 4, 64), (13, 16, 4, 64), (8, 24, 6, 64), (72, 9, 2, 64),
+    (75, 9, 2, 64), (16, 16, 8, 64),                  # 64 columns: CTAs with an SM to themselves, and pairs on every SM
+])
+def test_cluster_sums_by_length_and_crowding(lib, rows, tiles, cluster_k, N, overlap):
+    """What a cluster's sum goes through (an area of its own, the operands' buffers, the parked tiles) depends on the K tiles of
+    a CTA, on how many CTAs there are and on launch overlap.  Calls back to back, the same bits every time."""
+    from flash_llm_b200 import torch_op  # noqa: F401  (registers torch.ops.flashllm)
+    M, K = 128 * rows, 64 * tiles
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows * tiles + N)
+    A = (torch.rand((M, K), generator=gen, device="cuda") * 2 - 1).half()
+    A *= torch.rand((M, K), generator=gen, device="cuda") >= 0.8
+    B = (torch.rand((N, K), generator=gen, device="cuda") * 2 - 1).half()
+    bias = (torch.rand(M, generator=gen, device="cuda") - 0.5).half()
+    residual = (torch.rand((N, M), generator=gen, device="cuda") - 0.5).half()
+    want = (B.double() @ A.double().T + bias.double() + residual.double()).float().cpu().numpy()
+    words, offs = torch.ops.flashllm.encode(A)
+    torch.cuda.synchronize()
+    lib.set_launch_overlap(overlap)
+    lib.set_plan(path=lib.api.PATH_DIRECT, cluster_k=cluster_k)
+    try:
+        outs = [torch.ops.flashllm.spmm_epilogue(words, offs, B, M, 1, bias, 0, residual) for _ in range(6)]
+        torch.cuda.synchronize()
+    finally:
+        lib.set_plan()
+        lib.set_launch_overlap(False)
+    assert lib.consume_status() == 0
+    assert_close(outs[0].cpu().numpy(), want, f"{rows}x{tiles} S={cluster_k} N={N}")
+    assert all(torch.equal(C, outs[0]) for C in outs[1:])
+
+
 @pytest.mark.parametrize("N", [16, 64, 256])
 def test_sum_by_last_cta_is_deterministic_and_leaves_its_counters_clean(lib, oracle, N):
     """The order in which the CTAs of an output tile finish changes from launch to launch; the sum must not.  Repeated
