@@ -9,6 +9,7 @@
 #include <cstdlib>
 #include <mutex>
 #include <new>
+#include <type_traits>
 
 #include "../../include/SpMM_API.cuh"
 #include "launch.h"
@@ -190,12 +191,17 @@ template<int N_TILE>
 static cudaError_t raise_smem_limit(int optin)
 {
     cudaError_t e = raise_smem_limit_of(spmm_tcgen05_kernel<N_TILE>, optin);
-    if (e == cudaSuccess)
-        e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapWide, 8, 1>, optin);
-    if (e == cudaSuccess)
-        e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks>, optin);
-    if (e == cudaSuccess)
-        e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapPair, 4, 2, 2>, optin);
+    auto direct   = [&](auto push) {
+        if (e == cudaSuccess)
+            e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapWide, 8, 1, 1, push>, optin);
+        if (e == cudaSuccess)
+            e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks, 1, push>, optin);
+        if (e == cudaSuccess)
+            e = raise_smem_limit_of(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapPair, 4, 2, 2, push>, optin);
+    };
+    direct(std::false_type{});
+    if constexpr (N_TILE <= kPushMaxN)
+        direct(std::true_type{});
     if constexpr (N_TILE <= kScratchMaxN)
         if (e == cudaSuccess)
             e = raise_smem_limit_of(spmm_tcgen05_stream_kernel<N_TILE, kStreamCap>, optin);
@@ -382,23 +388,30 @@ static const FormCosts& form_costs(bool overlap, int n_tile)
     return kFormCosts[overlap ? 1 : 0][n_tile == 16 ? 0 : n_tile == 32 ? 1 : 2];
 }
 
+// Who has an SM to itself.  The last few clusters of three and more do not find their SMs empty (25 of five, of which 148
+// SMs hold 26, took 17.7 us where 24 take 12.5), and with overlap the next launch's CTAs are there early and pair up, unless
+// there are few of them or one for every SM (96 rows by 113 tiles, N = 16: 49 us; 148 rows: 35).
+static bool sm_to_itself(const DeviceState* st, long long clusters, int s, bool overlap)
+{
+    const long long apart  = clusters_resident(st, kClustersResident1, s);
+    const bool      sparse = s <= 2 ? clusters <= apart : 100 * clusters <= 93 * apart;
+    if (!overlap)
+        return sparse;
+    return sparse && (s == 1 ? clusters <= 32 || 100 * clusters > 95 * apart : clusters * s <= 64);
+}
+
 // One CTA or cluster of S CTAs per tile row (and workspace part).
 static double row_form_us(const DeviceState* st, int ctas_flat, int k_tiles, int s, int g, int n_tile, bool overlap)
 {
     const FormCosts& f        = form_costs(overlap, n_tile);
     const long long  clusters = static_cast<long long>(ctas_flat) * g;
-    const long long  held = clusters_resident(st, kClustersResident2, s), apart = clusters_resident(st, kClustersResident1, s);
+    const long long  held     = clusters_resident(st, kClustersResident2, s);
     const double     fixed  = s == 1 ? f.whole : f.cluster + f.per_rank / s;
     const double     tiles  = static_cast<double>((k_tiles + s * g - 1) / (s * g));
     const double     alone  = fixed + f.tile_alone * tiles;
     const double     shared = fixed + (s > 1 ? f.crowded + (10 * clusters > 9 * held ? f.full : 0.0) : 0.0) + f.tile_shared * tiles;
-    // Who has an SM to itself.  The last few clusters of three and more do not find their SMs empty (25 of five, of which 148
-    // SMs hold 26, took 17.7 us where 24 take 12.5), and with overlap the next launch's CTAs are there early and pair up, unless
-    // there are few of them or one for every SM (96 rows by 113 tiles, N = 16: 49 us; 148 rows: 35).
-    bool to_itself = s <= 2 ? clusters <= apart : 100 * clusters <= 93 * apart;
-    if (overlap)
-        to_itself = to_itself && (s == 1 ? clusters <= 32 || 100 * clusters > 95 * apart : clusters * s <= 64);
-    return (to_itself ? alone : (clusters + held - 1) / held * shared) + (g > 1 ? f.second_kernel + 0.1 * g : 0.0);
+    return (sm_to_itself(st, clusters, s, overlap) ? alone : (clusters + held - 1) / held * shared)
+           + (g > 1 ? f.second_kernel + 0.1 * g : 0.0);
 }
 
 // The row form was fitted to matrices that L2 holds a part of; 288 rows by 144 take 75.9 us from DRAM, not 69.5.
@@ -626,7 +639,13 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // columns with such room leave 28 KB, and 9216x36864 70 % in clusters of two took 102.5 us instead of 97.8.  They have it
     // for short K ranges only; time without it / with it by tiles per CTA (72 x 4 and 148 x 2 CTAs, 65 to 80 %): overlap off
     // 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %: 1.00 .. 1.07).
-    if (direct && pl.cluster_k > 1 && pl.n_tile <= kPushMaxN) {
+    // 64 columns are sent where CTAs have an SM to themselves (kPushMaxN), also from the next launch's: with overlap that is a
+    // few small clusters (sent / parked, 16 tiles a row: 8 clusters of four 6.8 / 7.6 us, 16 of four 9.1 / 8.2, 8 of six 8.7 / 7.4).
+    pl.push = direct && pl.cluster_k > 1 && pl.n_tile <= kPushMaxN
+              && (pl.n_tile <= 32 || !two_resident
+                  || (sm_to_itself(st, static_cast<long long>(ctas_flat) * extra, pl.cluster_k, overlap)
+                      && (!overlap || (pl.cluster_k <= 4 && ctas_flat * extra * pl.cluster_k <= 32))));
+    if (pl.push) {
         pl.sum_bytes       = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
         const bool short_k = (k_tiles + parts - 1) / parts <= (overlap ? 16 : 4);
         const int  room    = two_resident ? (short_k ? kSmemPerSm : kSmemForL1) / 2 - 1024 : st->smem_optin;
@@ -652,8 +671,9 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
                     && pl.smem_bytes <= st->smem_optin
                     // the fp32 partial tiles of the cluster reduction are parked over the pipeline buffers
                     && pl.smem_bytes - 1024 - 4 * pl.offsets_staged >= pl.n_tile * kTileM * 4
-                    && (!direct || pl.cluster_k == 1 || pl.sum_bytes > 0
-                        || pl.n_tile > kPushMaxN || pl.a_stages * kDenseTileBytes + pl.b_stages * pl.b_batch * slab >= cluster_sum_bytes(pl.n_tile, pl.cluster_k));
+                    && (!pl.push || pl.sum_bytes > 0
+                        || pl.a_stages * kDenseTileBytes + pl.b_stages * pl.b_batch * slab
+                               >= cluster_sum_bytes(pl.n_tile, pl.cluster_k));
     if (!ok)
         return cudaErrorInvalidConfiguration;
     *out = pl;
@@ -732,12 +752,18 @@ static cudaError_t launch_spmm(cudaStream_t stream, const CUtensorMap& tmap, con
         return cudaErrorInvalidConfiguration;
     }
     if (pl.path == kPathDirect) {
-        const int warps = 1 + kDirectIssuers + pl.scatter_warps * pl.producers;
-        if (pl.scatter_warps == 8)
-            return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapWide, 8, 1>, warps);
-        if (pl.producers == 2)
-            return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapPair, 4, 2, 2>, warps);
-        return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks>, warps);
+        const int warps  = 1 + kDirectIssuers + pl.scatter_warps * pl.producers;
+        auto      direct = [&](auto push) {
+            if (pl.scatter_warps == 8)
+                return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapWide, 8, 1, 1, push>, warps);
+            if (pl.producers == 2)
+                return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapPair, 4, 2, 2, push>, warps);
+            return launch(spmm_tcgen05_direct_kernel<N_TILE, kDirectCapNarrow, 4, kDirectBlocks, 1, push>, warps);
+        };
+        if constexpr (N_TILE <= kPushMaxN)
+            if (pl.push || pl.cluster_k == 1)
+                return direct(std::true_type{});
+        return direct(std::false_type{});
     }
     return launch(spmm_tcgen05_kernel<N_TILE>, pl.producers + 2 + pl.scatter_warps);
 }

@@ -214,7 +214,10 @@ __host__ __device__ constexpr int direct_accumulators(int n_tile)
 // (eight) 9.9 -> 8.7, 9216x1152 N = 16 (three) 9.1 -> 8.1, 4736x7232 N = 32 (seven) 19.0 -> 18.6.
 //
 // 128 columns are parked at home and fetched as before: a row per lane makes for stores of 16 bytes to as many places, and
-// 2688x8960 N = 128 in clusters of six takes 16.6 us that way instead of 15.4.
+// 2688x8960 N = 128 in clusters of six takes 16.6 us that way instead of 15.4.  64 columns, for which there is no area but the
+// operands' buffers, too where CTAs share SMs (plan.push): us per call parked / sent, 4096x4096 in clusters of eight 12.3 / 13.0,
+// of six 13.8 / 14.8; 5120x1024 in sixes 9.1 / 10.5; but with an SM to every CTA 1024x4096 in clusters of two 17.9 / 17.0, of
+// four 11.8 / 11.2, of eight 9.2 / 8.4.
 constexpr int kPushMaxN = 64;
 
 __host__ __device__ constexpr int cluster_sum_rows(int S)
@@ -244,6 +247,7 @@ __device__ __forceinline__ void accumulators_to_peers(uint32_t tmem_acc, int acc
                         + static_cast<uint32_t>((rank * cluster_sum_rows(S) + row - kTileM * q / S) * (N_TILE + 4)) * 4u;
     const uint32_t acc = tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16);
     constexpr int  A   = direct_accumulators(N_TILE);
+    const float    none = ok ? 0.0f : __int_as_float(0x7FFFFFFF);
     for (int c0 = col_begin; c0 < col_end; c0 += 8) {
         float    v[8];
         uint32_t t[A][8];
@@ -254,16 +258,13 @@ __device__ __forceinline__ void accumulators_to_peers(uint32_t tmem_acc, int acc
         ptx::tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            v[i] = accumulators > 0 ? __uint_as_float(t[0][i]) : 0.0f;
+            v[i] = ok && accumulators > 0 ? __uint_as_float(t[0][i]) : none;
 #pragma unroll
         for (int a = 1; a < A; ++a)
             if (a < accumulators)
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     v[i] += __uint_as_float(t[a][i]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            v[i] = ok ? v[i] : __int_as_float(0x7FFFFFFF);
         ptx::st_async_v4_f32(to + c0 * 4, v, bar);
         ptx::st_async_v4_f32(to + c0 * 4 + 16, v + 4, bar);
     }
@@ -335,17 +336,19 @@ __device__ __forceinline__ void finish_cluster_rows(const SpmmParams& p, uint32_
 // CAP: vectors per lane kept in registers.  WARPS: stages = tiles in flight per CTA.  WPT: warps that share one tile
 // (row q of warp h is the tile's row q * WPT + h), so a tile of up to 32 * CAP * WPT vectors is handled without the
 // overflow loop and a warp's instruction stream per tile is 1 / WPT as long.  MIN_BLOCKS: CTAs per SM the register
-// budget is sized for.
+// budget is sized for.  PUSH: the CTAs of a cluster send one another their sums (a kernel of its own, since both ways in one
+// cost every call 0.2 us).
 //
 // One thread cannot issue tcgen05.mma as fast as the tensor core retires them (measured: 4 MMAs and the commit that
 // hands a stage back cost an issuing thread ~400 cycles, the tensor core ~180), so tiles alternate between
 // kDirectIssuers issuing threads, each with accumulators of its own in tensor memory; the epilogue adds them.
-template<int N_TILE, int CAP, int WARPS, int MIN_BLOCKS, int WPT = 1>
+template<int N_TILE, int CAP, int WARPS, int MIN_BLOCKS, int WPT, bool PUSH>
 __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_BLOCKS)
     spmm_tcgen05_direct_kernel(const __grid_constant__ CUtensorMap tmap_b, const SpmmParams p)
 {
     static_assert(N_TILE == 16 || N_TILE == 32 || N_TILE == 64 || N_TILE == 128, "unsupported MMA N");
     static_assert(WARPS >= 4 && WARPS <= 12, "four warps cover the TMEM lane quarters in the epilogue");
+    static_assert(!PUSH || N_TILE <= kPushMaxN, "wider outputs are parked");
     static_assert(WPT == 1 || WPT == 2, "a tile is decompressed by one warp or by a pair");
     static_assert(CAP % 2 == 0 && 32 % WPT == 0, "batches are issued in two halves; the clear is split evenly");
     constexpr uint32_t kBSlab    = N_TILE * kTileK * 2;  // one K tile of B in shared memory
@@ -490,8 +493,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     }
     const uint32_t tmem_acc = *tmem_slot;
     const int      n_valid  = (p.N - n_idx * N_TILE) < N_TILE ? (p.N - n_idx * N_TILE) : N_TILE;
-    constexpr bool kPush = N_TILE <= kPushMaxN;
-    if (kPush && S > 1) {
+    if (PUSH && S > 1) {
         if (threadIdx.x == 0)  // everything the peers (and this CTA) will store here
             ptx::mbar_arrive_expect_tx(sum_full,
                                        static_cast<uint32_t>(S * (kTileM * (rank + 1) / S - kTileM * rank / S) * n_valid) * 4u);
@@ -682,13 +684,13 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
         if (sw == 0 && lane == 0)
             FL_CTA_TIME(2);
 
-        if (!kPush || S == 1)
+        if (!PUSH || S == 1)
             accumulators_to_output<N_TILE>(p, tmem_acc, L < accs ? L : accs, N_TILE, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, G, g, n_idx,
                                            tile_row, acc_ok, reinterpret_cast<float*>(smem));
     }
 
     // ================================================================ cluster reduction and tear-down
-    if (!kPush && S > 1) {
+    if (!PUSH && S > 1) {
         __syncwarp();
         ptx::cluster_sync_all();  // every CTA's partial tile is parked in its shared memory
         if (warp >= first_sw)
@@ -715,7 +717,7 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
     ptx::tc_fence_before_sync();
     __syncthreads();
     // A CTA that gave up leaves only when its peers have left or given up too: until then they may store into its shared memory.
-    if (kPush && S > 1 && *abort_flag != 0u) {
+    if (PUSH && S > 1 && *abort_flag != 0u) {
         __syncwarp();
         ptx::cluster_sync_all();
     }

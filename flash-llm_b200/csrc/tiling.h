@@ -69,7 +69,8 @@ struct SpmmPlan {
     int reduce;          // kReduceSecondKernel or kReduceLastCta (meaningful when workspace_k > 1)
     int offsets_staged;  // TileOffsets entries a CTA may stage in shared memory (0 = read them from global memory)
     int accumulators;    // kPathDirect: accumulators the tiles of a CTA take turns with, 2 or 4
-    int sum_bytes;       // kPathDirect with cluster_k > 1: shared memory set aside for the peers' partial sums, or 0
+    int push;            // kPathDirect with cluster_k > 1: the CTAs send one another their sums (or park them at home: 0)
+    int sum_bytes;       // kPathDirect with push: shared memory set aside for the peers' partial sums, or 0
     int smem_bytes;      // dynamic shared memory of the launch
 };
 
