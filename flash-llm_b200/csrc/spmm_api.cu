@@ -641,7 +641,8 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %: 1.00 .. 1.07).
     // 64 columns are sent where CTAs have an SM to themselves (kPushMaxN), also from the next launch's: with overlap that is a
     // few small clusters (sent / parked, 16 tiles a row: 8 clusters of four 6.8 / 7.6 us, 16 of four 9.1 / 8.2, 8 of six 8.7 / 7.4).
-    pl.push = direct && pl.cluster_k > 1 && pl.n_tile <= kPushMaxN
+    // The fused all-reduce parks: its CTAs then store whole columns of 512 bytes to the other GPUs, not runs of 64.
+    pl.push = direct && pl.cluster_k > 1 && pl.n_tile <= kPushMaxN && !sends
               && (pl.n_tile <= 32 || !two_resident
                   || (sm_to_itself(st, static_cast<long long>(ctas_flat) * extra, pl.cluster_k, overlap)
                       && (!overlap || (pl.cluster_k <= 4 && ctas_flat * extra * pl.cluster_k <= 32))));

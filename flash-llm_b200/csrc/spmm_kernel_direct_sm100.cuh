@@ -282,7 +282,7 @@ __device__ __forceinline__ void finish_cluster_rows(const SpmmParams& p, uint32_
     const uint32_t step  = static_cast<uint32_t>(cluster_sum_rows(S) * (N_TILE + 4)) * 4u;
     const int      shift = 32 - __clz(rows - 1);  // rows, rounded up to a power of two, are 16 to 64
     const int      r_1   = tid & ((1 << shift) - 1), c_1 = (tid >> shift) * 4;
-    const bool     direct = G == 1 && p.push_world == 0, first = direct && r_1 < rows && c_1 < n_valid;
+    const bool     first = G == 1 && r_1 < rows && c_1 < n_valid;
     float          bias_1 = -0.0f;
     half           res_1[4];
     if (first)
@@ -317,12 +317,6 @@ __device__ __forceinline__ void finish_cluster_rows(const SpmmParams& p, uint32_
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 part[static_cast<size_t>(i) * p.M] = v[i];
-        }
-        else if (p.push_world > 0) {
-            for (int w = 0; w < p.push_world; ++w)
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    p.push_slot[w][tile_off + at + static_cast<size_t>(i) * p.M] = v[i];
         }
         else if (e == tid)
             finish_columns<4>(p, v, tile_off + at, 4, bias_1, res_1);
