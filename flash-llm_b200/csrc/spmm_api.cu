@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -319,17 +320,6 @@ static int stream_smem_bytes(const SpmmPlan& pl)
            + 8 * (2 * kStreamStages + 4 + 2 * pl.b_stages) + 16 + kStreamSumBytes + 4 * pl.offsets_staged;
 }
 
-// K tiles that the tensor core may add up in one accumulator.  It truncates each of its additions, so the error of a sum grows
-// with their number (measured: 7e-8 of the sum per tile of four).  No more than when K is cut into `parts`, or into as many parts
-// as fill the GPU (in clusters and in the caller's workspace) if that is more, and every part alternates between two.
-static int tiles_per_accumulator(const DeviceState* st, int tile_rows, int k_tiles, int max_extra, int parts)
-{
-    const int most = kMaxClusterK * max_extra, fill = kStreamCtasPerSm * st->sm_count / tile_rows;
-    const int cut  = fill < most ? fill : most;
-    parts          = parts < cut ? cut : parts;
-    return ((k_tiles + parts - 1) / parts + 1) / 2;
-}
-
 // The streaming form: as many CTAs as the GPU holds, fewer only when there are fewer tiles.
 static cudaError_t make_stream_plan(const DeviceState* st, SpmmPlan pl, int tile_rows, int k_tiles, int chunk_tiles, SpmmPlan* out)
 {
@@ -496,8 +486,9 @@ static cudaError_t make_wide_plan(const DeviceState* st, SpmmPlan pl, const Plan
 // `sends`: the call is the sending half of a fused all-reduce, where workspace parts are always summed by the last
 // CTA of a tile, which then also stores the sum to every GPU.
 // `may_stream`: the call may use the streaming form (the stream's scratch is at hand).
+// `parts_fit`: workspace and C are aligned for workspace parts; a plan's are dropped otherwise.
 static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max_parts, SpmmPlan* out, bool sends = false,
-                             bool may_stream = true)
+                             bool may_stream = true, bool parts_fit = true)
 {
     PlanOverride ov;
     {
@@ -571,52 +562,74 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
         pl.reduce = kReduceSecondKernel;
     // (Without launch overlap a second kernel used to cost a whole launch, and small problems did better with clusters alone.
     // This rule and the costs in tiles below were fitted before every kernel was launched with programmatic serialisation.)
-    const bool no_second = pl.reduce == kReduceSecondKernel && static_cast<long long>(tile_rows) * k_tiles <= 4096
-                           && g_launch_overlap.load(std::memory_order_relaxed) == 0;
-    const bool overlap = g_launch_overlap.load(std::memory_order_relaxed) != 0;
-    // Priced in us where the row form with two CTAs per SM and the streaming form are the choice.
-    const bool priced = direct && two_resident && pl.n_tile <= kScratchMaxN && !sends;
-    int    best_s = 1, best_g = 1;
-    double best_cost = 0.0;
-    for (int s_ = 1; s_ <= kMaxClusterK && s_ <= k_tiles; ++s_) {
-        for (int g = 1; g <= max_extra && g <= 32 && s_ * g <= k_tiles; ++g) {
-            if (g > 1 && no_second)
-                break;
-            if (priced) {
-                const double cost = row_form_us(st, ctas_flat, k_tiles, s_, g, pl.n_tile, overlap);
-                if ((s_ == 1 && g == 1) || cost < best_cost) {
+    const bool overlap   = g_launch_overlap.load(std::memory_order_relaxed) != 0;
+    const bool few_tiles = static_cast<long long>(tile_rows) * k_tiles <= 4096 && !overlap;
+    // The cut by tiles.
+    struct Cut {
+        int s, g;
+    };
+    auto cut_by_tiles = [&](int reduce) {
+        Cut    best{1, 1};
+        double best_cost = 0.0;
+        for (int s_ = 1; s_ <= kMaxClusterK && s_ <= k_tiles; ++s_) {
+            for (int g = 1; g <= max_extra && g <= 32 && s_ * g <= k_tiles; ++g) {
+                if (g > 1 && reduce == kReduceSecondKernel && few_tiles)
+                    break;
+                const long long clusters = static_cast<long long>(ctas_flat) * g, capacity = clusters_resident(st, resident, s_);
+                const double    waves    = static_cast<double>((clusters + capacity - 1) / capacity);
+                const double    per_cta  = static_cast<double>((k_tiles + s_ * g - 1) / (s_ * g)) + 16.0 + (s_ > 1 ? 3.0 : 0.0)
+                                        + (g > 1 && reduce == kReduceLastCta ? (sends ? 8.0 : 2.0) + 0.1 * g : 0.0);
+                const double cost = waves * per_cta + (g > 1 && reduce == kReduceSecondKernel ? 0.5 * g : 0.0);
+                if ((s_ == 1 && g == 1) || cost < best_cost - 1e-9 || (cost < best_cost + 1e-9 && s_ * g < best.s * best.g)) {
                     best_cost = cost;
-                    best_s    = s_;
-                    best_g    = g;
+                    best      = {s_, g};
                 }
-                continue;
             }
-            const long long clusters = static_cast<long long>(ctas_flat) * g, capacity = clusters_resident(st, resident, s_);
-            const double    waves    = static_cast<double>((clusters + capacity - 1) / capacity);
-            const double    per_cta  = static_cast<double>((k_tiles + s_ * g - 1) / (s_ * g)) + 16.0 + (s_ > 1 ? 3.0 : 0.0)
-                                    + (g > 1 && pl.reduce == kReduceLastCta ? (sends ? 8.0 : 2.0) + 0.1 * g : 0.0);
-            const double cost = waves * per_cta + (g > 1 && pl.reduce == kReduceSecondKernel ? 0.5 * g : 0.0);
-            if ((s_ == 1 && g == 1) || cost < best_cost - 1e-9
-                || (cost < best_cost + 1e-9 && s_ * g < best_s * best_g)) {
+        }
+        return best;
+    };
+    // It also bounds the sums of every other cut: the tensor core truncates each of its additions, so the error of a sum grows
+    // with the tiles added up in one accumulator (measured: 0.7e-7 to 1.4e-7 of the sum per tile of four).  No cut that is
+    // cheaper may add up more of them, in four accumulators, than this one in two; and where two of them would hold more than if
+    // K were cut into as many parts as fill the GPU, it takes the four.
+    auto      in_one_of_two = [&](int parts) { return ((k_tiles + parts - 1) / parts + 1) / 2; };
+    const Cut by_tiles      = cut_by_tiles(kReduceSecondKernel);
+    const int bound         = in_one_of_two(by_tiles.s * (parts_fit ? by_tiles.g : 1));
+    const int fill          = std::min(kStreamCtasPerSm * st->sm_count / tile_rows, kMaxClusterK * max_extra);
+    const int full_parts    = std::max(by_tiles.s * by_tiles.g, fill);
+    Cut       best          = pl.reduce == kReduceSecondKernel ? by_tiles : cut_by_tiles(pl.reduce);
+    // The cut by us, where the row form with two CTAs per SM and the streaming form are the choice.
+    const bool priced    = direct && two_resident && pl.n_tile <= kScratchMaxN && !sends;
+    double     best_cost = -1.0;
+    for (int s_ = 1; priced && s_ <= kMaxClusterK && s_ <= k_tiles; ++s_) {
+        for (int g = 1; g <= (parts_fit ? max_extra : 1) && g <= 32 && s_ * g <= k_tiles; ++g) {
+            if (g > 1 && pl.reduce == kReduceSecondKernel && few_tiles)
+                break;
+            const int accumulators = direct_accumulators(pl.n_tile), longest = (k_tiles + s_ * g - 1) / (s_ * g);
+            if ((longest + accumulators - 1) / accumulators > bound)
+                continue;
+            const double cost = row_form_us(st, ctas_flat, k_tiles, s_, g, pl.n_tile, overlap);
+            if (best_cost < 0.0 || cost < best_cost) {
                 best_cost = cost;
-                best_s    = s_;
-                best_g    = g;
+                best      = {s_, g};
             }
         }
     }
     if (may_stream && !pinned && priced) {
         SpmmPlan sp = pl;
         sp.path     = kPathStream;
-        if (make_stream_plan(st, sp, tile_rows, k_tiles, tiles_per_accumulator(st, tile_rows, k_tiles, max_extra, best_s * best_g), &sp) == cudaSuccess
+        // a chunk holds what any of these cuts would put into one of two accumulators
+        const int chunk_tiles = in_one_of_two(std::max(full_parts, best.s * best.g));
+        if (make_stream_plan(st, sp, tile_rows, k_tiles, chunk_tiles, &sp) == cudaSuccess
             && stream_form_us(sp, tile_rows, k_tiles, overlap) < row_form_margin(tile_rows, k_tiles) * best_cost) {
             *out = sp;
             return cudaSuccess;
         }
     }
-    pl.cluster_k = ov.v[kPlanClusterK] ? ov.v[kPlanClusterK] : best_s;
+    pl.cluster_k = ov.v[kPlanClusterK] ? ov.v[kPlanClusterK] : best.s;
     if (pl.cluster_k > k_tiles)
         pl.cluster_k = k_tiles;
-    int extra = ov.v[kPlanWorkspaceK] ? ov.v[kPlanWorkspaceK] : best_g;
+    int extra = ov.v[kPlanWorkspaceK] ? ov.v[kPlanWorkspaceK] : best.g;
     if (extra > max_extra)
         extra = max_extra;  // the workspace is promised to hold Split_K fp16 matrices = Split_K/2 fp32 partials
     if (extra * pl.cluster_k > k_tiles)
@@ -624,11 +637,9 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     if (extra < 1)
         extra = 1;
     pl.workspace_k = extra;
-    // A K range that is longer than if K were cut into as many parts as fill the GPU takes turns with four accumulators, so that
-    // no sum in the tensor core gets longer for it.
+    const int parts = pl.cluster_k * (parts_fit ? extra : 1);
     pl.accumulators = kDirectIssuers;
-    const int parts = pl.cluster_k * extra;
-    if (direct && (k_tiles + parts - 1) / parts > 2 * tiles_per_accumulator(st, tile_rows, k_tiles, max_extra, parts))
+    if (direct && (k_tiles + parts - 1) / parts > kDirectIssuers * in_one_of_two(full_parts))
         pl.accumulators = direct_accumulators(pl.n_tile);
     // room for this CTA's slice of TileOffsets (K tiles of the longest part, plus one), up to 8 KB
     const int longest = (k_tiles + pl.cluster_k * pl.workspace_k - 1) / (pl.cluster_k * pl.workspace_k) + 1;
@@ -702,12 +713,13 @@ static cudaError_t encode_b_map(const half* B, int N, int K, int ldb, const Spmm
 struct CallKey {
     const DeviceState* device;
     int                M, N, K, ldb, max_parts;
-    bool               sends, may_stream, overlap;
+    bool               sends, may_stream, overlap, parts_fit;
     unsigned           override_version;
     bool operator==(const CallKey& o) const
     {
         return device == o.device && M == o.M && N == o.N && K == o.K && ldb == o.ldb && max_parts == o.max_parts && sends == o.sends
-               && may_stream == o.may_stream && overlap == o.overlap && override_version == o.override_version;
+               && may_stream == o.may_stream && overlap == o.overlap && parts_fit == o.parts_fit
+               && override_version == o.override_version;
     }
 };
 struct CallMemo {
@@ -726,7 +738,8 @@ static cudaError_t plan_call(const CallKey& key, CallMemo** out)
     CallMemo& m = memo[(hash ^ (hash >> 16)) % kEntries];
     if (!(m.key == key)) {
         SpmmPlan          plan{};
-        const cudaError_t err = make_plan(key.device, key.M, key.N, key.K, key.max_parts, &plan, key.sends, key.may_stream);
+        const cudaError_t err = make_plan(key.device, key.M, key.N, key.K, key.max_parts, &plan, key.sends, key.may_stream,
+                                                key.parts_fit);
         if (err != cudaSuccess)
             return err;
         m.key     = key;
@@ -885,8 +898,11 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
 
     SpmmParams params{};
     SpmmPlan&  pl = params.plan;
+    // The sum over workspace parts reads 16-byte groups of the workspace and writes 8-byte groups of C.
+    const bool parts_fit = comm != nullptr || Split_K < 4 || ((reinterpret_cast<uintptr_t>(Reduction_Workspace) & 15u) == 0
+                                                              && (reinterpret_cast<uintptr_t>(C) & 7u) == 0);
     CallKey    key{st,           M_Global,     N_Global, K_Global, ldb ? ldb : K_Global, comm ? kCommLocalParts : Split_K / 2,
-                comm != nullptr, may_allocate, g_launch_overlap.load(std::memory_order_relaxed) != 0,
+                comm != nullptr, may_allocate, g_launch_overlap.load(std::memory_order_relaxed) != 0, parts_fit,
                 g_override_version.load(std::memory_order_relaxed)};
     CallMemo*  memo = nullptr;
     if ((err = plan_call(key, &memo)) != cudaSuccess)
@@ -904,9 +920,7 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
         }
     }
     pl = memo->plan;
-    // The sum over workspace parts reads 16-byte groups of the workspace and writes 8-byte groups of C.
-    if (!comm && pl.workspace_k > 1
-        && ((reinterpret_cast<uintptr_t>(Reduction_Workspace) & 15u) != 0 || (reinterpret_cast<uintptr_t>(C) & 7u) != 0))
+    if (!parts_fit)
         pl.workspace_k = 1;
 
     params.compressed   = Compressed_A;

@@ -29,7 +29,7 @@ __host__ __device__ constexpr int wide_slabs(int n_tile) { return n_tile / wide_
 __host__ __device__ constexpr int wide_a_stages(int n_tile) { return n_tile <= 384 ? 8 : 6; }
 __host__ __device__ constexpr int wide_b_stages(int n_tile) { return n_tile == 256 ? 3 : 4; }
 // Accumulators that the tiles take turns in.  Two halve the truncated additions of a sum; 384 and 512 columns leave no room
-// for a second one (see tiles_per_accumulator): 36864x9216 N = 512 at 80 % is 2.0755e-4 off its exact values in the 2-norm,
+// for a second one (a sum loses 7e-8 of itself per tile in one accumulator): 36864x9216 N = 512 at 80 % is 2.0755e-4 off its exact values in the 2-norm,
 // with 256 columns and two accumulators 2.0736e-4 and 29 % slower, where rounding to fp16 alone is 2.0730e-4.
 __host__ __device__ constexpr int wide_accumulators(int n_tile) { return n_tile <= 256 ? 2 : 1; }
 constexpr int kWideFirstScatter = 2;

@@ -201,3 +201,30 @@ def test_malformed_offsets_are_reported_not_followed(lib, oracle, streaming):
     assert np.isnan(got[:, :128]).all(), "the row whose tiles 4 and 5 were given up is not stored"
     assert_close(got[:, 128:], want[:, 128:], "the other rows")
     assert_close(DeviceProblem(lib, comp, offs, B, M, N, K, 1).run(), want, "call after a malformed one")
+
+
+@pytest.mark.parametrize("M,K,split_k,cluster_k,workspace_k", [(25472, 11264, 2, 4, 1), (27648, 12288, 4, 2, 2),
+                                                               (27648, 20480, 1, 5, 1)])
+def test_sums_are_as_exact_as_in_the_cut_that_bounds_them(lib, M, K, split_k, cluster_k, workspace_k):
+    """149 to 296 tile rows fill the GPU uncut, and a cut by cost alone would add up 88 to 160 tiles in each of a K range's two
+    accumulators.  Streamed or not, no sum in the tensor core may be longer than in the cut by tiles (22, 24, 32 of them), so
+    that the mean share a sum of positive products loses is no larger; 1e-6 for rounding and sums in fp32, as above."""
+    from flash_llm_b200 import torch_op  # noqa: F401  (registers torch.ops.flashllm)
+    N = 64
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M + K)
+    A = torch.rand((M, K), generator=gen, device="cuda").half()
+    A *= torch.rand((M, K), generator=gen, device="cuda") >= 0.8
+    B = torch.rand((N, K), generator=gen, device="cuda").half()
+    want = torch.cat([B.double() @ A[r:r + 1024].double().T for r in range(0, M, 1024)], dim=1)
+    words, offs = torch.ops.flashllm.encode(A)
+    share = {}
+    assert lib.get_plan(M, N, K, split_k)["path"] == lib.api.PATH_STREAM
+    try:
+        for name, plan in (("streamed", {}), ("rows", dict(path=2)), ("by tiles", dict(path=2, cluster_k=cluster_k, workspace_k=workspace_k))):
+            lib.set_plan(**plan)
+            share[name] = abs(float(((want - torch.ops.flashllm.spmm(words, offs, B, M, split_k).double()) / want).mean()))
+    finally:
+        lib.set_plan()
+    assert lib.consume_status() == 0
+    assert max(share["streamed"], share["rows"]) <= share["by tiles"] + 1e-6, share
