@@ -390,6 +390,12 @@ static bool sm_to_itself(const DeviceState* st, long long clusters, int s, bool 
     return sparse && (s == 1 ? clusters <= 32 || 100 * clusters > 95 * apart : clusters * s <= 64);
 }
 
+// Hardly a place is left for the clusters of the next launch.
+static bool grid_is_full(const DeviceState* st, long long clusters, int s)
+{
+    return 10 * clusters > 9 * clusters_resident(st, kClustersResident2, s);
+}
+
 // One CTA or cluster of S CTAs per tile row (and workspace part).
 static double row_form_us(const DeviceState* st, int ctas_flat, int k_tiles, int s, int g, int n_tile, bool overlap)
 {
@@ -399,7 +405,7 @@ static double row_form_us(const DeviceState* st, int ctas_flat, int k_tiles, int
     const double     fixed  = s == 1 ? f.whole : f.cluster + f.per_rank / s;
     const double     tiles  = static_cast<double>((k_tiles + s * g - 1) / (s * g));
     const double     alone  = fixed + f.tile_alone * tiles;
-    const double     shared = fixed + (s > 1 ? f.crowded + (10 * clusters > 9 * held ? f.full : 0.0) : 0.0) + f.tile_shared * tiles;
+    const double     shared = fixed + (s > 1 ? f.crowded + (grid_is_full(st, clusters, s) ? f.full : 0.0) : 0.0) + f.tile_shared * tiles;
     return (sm_to_itself(st, clusters, s, overlap) ? alone : (clusters + held - 1) / held * shared)
            + (g > 1 ? f.second_kernel + 0.1 * g : 0.0);
 }
@@ -650,6 +656,8 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // columns with such room leave 28 KB, and 9216x36864 70 % in clusters of two took 102.5 us instead of 97.8.  They have it
     // for short K ranges only; time without it / with it by tiles per CTA (72 x 4 and 148 x 2 CTAs, 65 to 80 %): overlap off
     // 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %: 1.00 .. 1.07).
+    // Where large clusters leave no place for the next launch's, a CTA's end counts for more: off, 56 clusters of five 1.04 at 8,
+    // 1.07 at 13, 1.02 at 29, 45 of six 1.00, 0.99, 0.96 at 7, 11, 24, 33 of eight 1.02, 1.03, 1.00 at 5, 8, 18.
     // 64 columns are sent where CTAs have an SM to themselves (kPushMaxN), also from the next launch's: with overlap that is a
     // few small clusters (sent / parked, 16 tiles a row: 8 clusters of four 6.8 / 7.6 us, 16 of four 9.1 / 8.2, 8 of six 8.7 / 7.4).
     // The fused all-reduce parks: its CTAs then store whole columns of 512 bytes to the other GPUs, not runs of 64.
@@ -659,7 +667,8 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
                       && (!overlap || (pl.cluster_k <= 4 && ctas_flat * extra * pl.cluster_k <= 32))));
     if (pl.push) {
         pl.sum_bytes       = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
-        const bool short_k = (k_tiles + parts - 1) / parts <= (overlap ? 16 : 4);
+        const bool full    = pl.cluster_k >= 5 && grid_is_full(st, static_cast<long long>(ctas_flat) * extra, pl.cluster_k);
+        const bool short_k = (k_tiles + parts - 1) / parts <= (overlap || full ? 16 : 4);
         const int  room    = two_resident ? (short_k ? kSmemPerSm : kSmemForL1) / 2 - 1024 : st->smem_optin;
         if (plan_smem_bytes(pl) > room)
             pl.sum_bytes = 0;
