@@ -404,9 +404,6 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
     }
     else {
         // ================================================================ epilogue warps
-        // Bias, residual, parked parts and counters may belong to the stream's earlier work; with launch overlap on nothing has
-        // waited for that here.
-        ptx::grid_dependency_wait();
         const int tid     = threadIdx.x - kStreamFirstEpi * 32;
         const int quarter = warp & 3;  // the tensor-memory lanes this warp may read
         const int r       = quarter * 32 + lane;
@@ -450,11 +447,11 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
             const int  c_last    = whole ? cta : stream_owner(p, ctas, row_begin + p.k_tiles - 1);
             const bool ask       = c_last == cta + 1 && t_begin <= row_begin;
             bool       asked = false, complete = false;
-            const float bias = bias_of(p, row * kTileM + r);
             auto       other_has_parked = [&](bool look) {  // every epilogue warp asks once
                 asked             = true;
                 unsigned int seen = 0u;
                 if (look && tid == 0) {
+                    ptx::grid_dependency_wait();  // counters may be in use by the stream's previous launch until it is over
                     seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
                     for (int n = 1; seen == 0u && n < kStreamLooks && !ptx::mbar_test_wait(acc_full + 8u * (q & 1), (q >> 1) & 1u); ++n)
                         seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
@@ -491,6 +488,9 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                 }
                 ptx::tmem_wait_st();
             }
+            // Bias and residual may be the stream's earlier work.  With launch overlap on these warps have not waited for that, but
+            // a full accumulator has: it took a B that was loaded after the wait.  (A wait of their own costs 0.6 % of a call.)
+            const float bias = ok ? bias_of(p, row * kTileM + r) : 0.0f;
             if (ask && !asked)  // gave up on the way
                 complete = other_has_parked(false);
             float* const park = whole || complete ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (j == 0 ? 0 : 1)) + r;
@@ -528,6 +528,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                     // arrivals in the low half of the counter; a CTA that gave up also marks the high half, so that the
                     // last one knows the row's sum is not to be trusted
                     const unsigned int mine = gave_up ? 0x10001u : 1u;
+                    ptx::grid_dependency_wait();  // (as above)
                     const int          c_first = stream_owner(p, ctas, row_begin);
                     const unsigned int before  = ptx::atom_add_acq_rel_gpu(p.tile_counters + row, mine);
                     if ((before & 0xFFFFu) + 1u == static_cast<unsigned int>(c_last - c_first + 1)) {

@@ -38,11 +38,14 @@ def test_every_kernel_waits_for_its_predecessors():
     assert kernels >= 12
 
 
-def test_the_streaming_epilogue_waits_before_it_reads_anything():
-    """The epilogue warps read bias, residual, parked parts and counters, all of which earlier work in the stream may be
-    writing; with launch overlap on they have not waited for it at the kernel's top."""
+def test_the_streaming_epilogue_reads_bias_and_residual_behind_an_accumulator():
+    """Earlier work in the stream may be writing them, and with launch overlap on the epilogue warps have not waited for it at
+    the kernel's top.  A full accumulator holds products of a B that was loaded after the wait."""
     code = _code(os.path.join(ROOT, "flash-llm_b200", "csrc", "spmm_kernel_stream_sm100.cuh"))
     body = code[code.index("spmm_tcgen05_stream_kernel("):]
     epilogue = body[re.search(r"else if \(warp < kStreamFirstEpi\).*?else \{", body, re.S).end():]
-    before = epilogue[:epilogue.index("grid_dependency_wait()")]
-    assert not re.search(r"\bp\.|bias_of|load_residual|for\s*\(|if\s*\(", before), before
+    assert re.search(r"bias_of|p\.residual|load_residual|finish_columns", epilogue)
+    segment = epilogue[epilogue.index("for (int row = row0"):]
+    before = epilogue[:epilogue.index("for (int row = row0")] + segment[:segment.index("wait_bounded_converged(acc_full")]
+    assert not re.search(r"bias_of|p\.bias|p\.residual|load_residual|finish_columns", before)
+    assert re.search(r"=\s*ok \? bias_of", segment)
