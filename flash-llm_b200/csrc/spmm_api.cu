@@ -356,9 +356,11 @@ static long long clusters_resident(const DeviceState* st, const int* table, int 
     return c < 1 ? 1ll : c;
 }
 
-// What a launch with N <= 64 costs, in us, back to back on one stream: fitted to 4..200 tile rows by 16..512 K tiles at 80 %
-// sparsity on a B200, launch overlap off and on, with every cluster size and the streaming form timed at each; against the
-// fastest of them the choice then loses 0.8 % on average, where one cost for all K cuts lost 6.1.
+// What a launch with N <= 64 costs, in us, back to back on one stream, at 80 % sparsity on a B200.  Fitted to 8..288 tile rows (with
+// overlap 2..288) by 16..288 K tiles, every cluster size, one to four workspace parts and the streaming form timed at each; what
+// the choice then loses to the fastest of them, on average and at most, overlap off: N = 16 0.8 % (12 %; these prices are older
+// and the rule about SMs is not), 32 0.3 % (5 %), 64 0.3 % (9 %); on, where CTAs pair up by luck: 0.4 % (9 %), 0.8 % (12 %),
+// 1.1 % (15 %).  Over 45 further sizes at 60 to 95 % the calls took 0.892 of the time of one cost for all K cuts.
 struct FormCosts {
     double whole, cluster, per_rank;  // fixed part: uncut, in clusters, and what their sum adds for the rows a CTA sums
     double crowded, full;             // more with two CTAs per SM, and when a grid leaves no place for the next one's clusters
@@ -367,27 +369,27 @@ struct FormCosts {
     double stream, stream_tile, stream_part;
 };
 static const FormCosts kFormCosts[2][3] = {{{3.3, 4.0, 1.3, 0.35, 0.5, 0.280, 0.46, 2.5, 6.2, 0.450, 0.07},
-                                            {3.85, 4.2, 3.3, 0.8, 0.9, 0.295, 0.50, 2.5, 6.9, 0.475, 0.17},
-                                            {4.75, 5.4, 3.7, 2.0, 2.0, 0.315, 0.53, 2.5, 8.7, 0.525, 0.41}},
-                                           {{3.0, 3.7, 0.0, 0.0, 1.0, 0.280, 0.45, 1.6, 5.0, 0.440, 0.07},
-                                            {3.6, 4.8, 0.0, 0.0, 1.3, 0.295, 0.48, 1.6, 6.0, 0.465, 0.17},
-                                            {4.3, 7.2, 0.0, 0.0, 2.2, 0.315, 0.51, 1.6, 7.6, 0.500, 0.41}}};
+                                            {3.75, 4.2, 1.7, 1.4, 0.9, 0.305, 0.46, 2.5, 6.9, 0.475, 0.17},
+                                            {4.75, 5.6, 2.9, 2.4, 0.8, 0.335, 0.51, 2.5, 8.7, 0.525, 0.47}},
+                                           {{2.1, 3.6, 0.0, 0.0, 0.4, 0.330, 0.39, 2.0, 5.2, 0.375, 0.10},
+                                            {3.9, 4.9, 0.0, 0.0, 0.9, 0.375, 0.46, 2.4, 6.2, 0.465, 0.17},
+                                            {4.0, 7.2, 0.0, 0.0, 0.9, 0.365, 0.48, 2.0, 7.5, 0.495, 0.41}}};
 
 static const FormCosts& form_costs(bool overlap, int n_tile)
 {
     return kFormCosts[overlap ? 1 : 0][n_tile == 16 ? 0 : n_tile == 32 ? 1 : 2];
 }
 
-// Who has an SM to itself.  The last few clusters of three and more do not find their SMs empty (25 of five, of which 148
-// SMs hold 26, took 17.7 us where 24 take 12.5), and with overlap the next launch's CTAs are there early and pair up, unless
-// there are few of them or one for every SM (96 rows by 113 tiles, N = 16: 49 us; 148 rows: 35).
-static bool sm_to_itself(const DeviceState* st, long long clusters, int s, bool overlap)
+// Who has an SM to itself, and with it a tile in 0.3 us instead of 0.45 to 0.5.  The last few clusters of three and more do not
+// find their SMs empty (25 of five, of which 148 SMs hold 26, took 17.7 us where 24 take 12.5), but for those of four (33 of 33
+// do).  With overlap the next launch's CTAs are there early and pair up: hardly ever up to 32 CTAs, or 48 with a second kernel in
+// between, and from 64 on more often than not (8 clusters of eight 0.35 us per tile, 7 of them 0.46: the luck of the launch),
+// unless there is one for every SM (148 rows by 144 tiles, N = 16 and 32: 0.31 us per tile, 136 rows 0.48).
+static bool sm_to_itself(const DeviceState* st, int ctas_flat, int s, int g, bool overlap)
 {
-    const long long apart  = clusters_resident(st, kClustersResident1, s);
-    const bool      sparse = s <= 2 ? clusters <= apart : 100 * clusters <= 93 * apart;
-    if (!overlap)
-        return sparse;
-    return sparse && (s == 1 ? clusters <= 32 || 100 * clusters > 95 * apart : clusters * s <= 64);
+    const long long clusters = static_cast<long long>(ctas_flat) * g, apart = clusters_resident(st, kClustersResident1, s);
+    const bool      sparse   = s <= 2 || s == 4 ? clusters <= apart : 100 * clusters <= 93 * apart;
+    return sparse && (!overlap || clusters * s <= (g > 1 ? 48 : 32) || (s == 1 && 100 * clusters > 98 * apart));
 }
 
 // Hardly a place is left for the clusters of the next launch.
@@ -402,15 +404,17 @@ static double row_form_us(const DeviceState* st, int ctas_flat, int k_tiles, int
     const FormCosts& f        = form_costs(overlap, n_tile);
     const long long  clusters = static_cast<long long>(ctas_flat) * g;
     const long long  held     = clusters_resident(st, kClustersResident2, s);
-    const double     fixed  = s == 1 ? f.whole : f.cluster + f.per_rank / s;
-    const double     tiles  = static_cast<double>((k_tiles + s * g - 1) / (s * g));
-    const double     alone  = fixed + f.tile_alone * tiles;
-    const double     shared = fixed + (s > 1 ? f.crowded + (grid_is_full(st, clusters, s) ? f.full : 0.0) : 0.0) + f.tile_shared * tiles;
-    return (sm_to_itself(st, clusters, s, overlap) ? alone : (clusters + held - 1) / held * shared)
+    const double     fixed    = s == 1 ? f.whole : f.cluster + f.per_rank / s;
+    const double     crowded  = s == 1 ? 0.0 : f.crowded + (grid_is_full(st, clusters, s) ? f.full : 0.0);
+    const double     tiles    = static_cast<double>((k_tiles + s * g - 1) / (s * g));
+    const double     alone    = fixed + f.tile_alone * tiles;
+    const double     shared   = fixed + crowded + f.tile_shared * tiles;
+    return (sm_to_itself(st, ctas_flat, s, g, overlap) ? alone : (clusters + held - 1) / held * shared)
            + (g > 1 ? f.second_kernel + 0.1 * g : 0.0);
 }
 
-// The row form was fitted to matrices that L2 holds a part of; 288 rows by 144 take 75.9 us from DRAM, not 69.5.
+// Most of the matrices that the row form was fitted to stay in L2 from call to call, large ones do not.  One size says how much
+// that is, 288 rows by 144 tiles: 75.9 us from DRAM where the prices say 69.5.  Up to 4000 tiles (26 MB) nothing is added.
 static double row_form_margin(int tile_rows, int k_tiles)
 {
     return static_cast<long long>(tile_rows) * k_tiles < 4000 ? 1.0 : 1.05;
@@ -658,13 +662,12 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %: 1.00 .. 1.07).
     // Where large clusters leave no place for the next launch's, a CTA's end counts for more: off, 56 clusters of five 1.04 at 8,
     // 1.07 at 13, 1.02 at 29, 45 of six 1.00, 0.99, 0.96 at 7, 11, 24, 33 of eight 1.02, 1.03, 1.00 at 5, 8, 18.
-    // 64 columns are sent where CTAs have an SM to themselves (kPushMaxN), also from the next launch's: with overlap that is a
-    // few small clusters (sent / parked, 16 tiles a row: 8 clusters of four 6.8 / 7.6 us, 16 of four 9.1 / 8.2, 8 of six 8.7 / 7.4).
+    // 64 columns are sent where CTAs have an SM to themselves (kPushMaxN), also from the next launch's (overlap on, sent / parked: 4
+    // clusters of eight by 46 tiles 7.2 / 8.4 us, 8 of four by 16 6.8 / 7.6, but 16 of four 9.1 / 8.2, 8 of six 8.7 / 7.4).
     // The fused all-reduce parks: its CTAs then store whole columns of 512 bytes to the other GPUs, not runs of 64.
     pl.push = direct && pl.cluster_k > 1 && pl.n_tile <= kPushMaxN && !sends
               && (pl.n_tile <= 32 || !two_resident
-                  || (sm_to_itself(st, static_cast<long long>(ctas_flat) * extra, pl.cluster_k, overlap)
-                      && (!overlap || (pl.cluster_k <= 4 && ctas_flat * extra * pl.cluster_k <= 32))));
+                  || sm_to_itself(st, ctas_flat, pl.cluster_k, extra, overlap));
     if (pl.push) {
         pl.sum_bytes       = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
         const bool full    = pl.cluster_k >= 5 && grid_is_full(st, static_cast<long long>(ctas_flat) * extra, pl.cluster_k);
