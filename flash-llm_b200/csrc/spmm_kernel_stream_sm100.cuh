@@ -20,7 +20,7 @@
 // What a call takes after its last MMA is no other CTA's work any more, so it is kept short.  The first of two CTAs that share
 // a row usually finds the other's part parked, takes it into tensor memory while its own is being multiplied and finishes the
 // row without parking.  Other rows are added up when the CTA's roles are done, by all of its threads instead of the four
-// epilogue warps: a part is an L2 round trip away.  Both together, us per call: 2048x32768 N=16 70 % (19 parts a row) 26.5 ->
+// epilogue warps: a part is an L2 round trip away.  Both together, us per call with two matrices in turn: 2048x32768 N=16 70 % (19 parts a row) 26.5 ->
 // 24.5, 9216x36864 N=32 70 % (5 parts) 97.1 -> 93.4, 49152x12288 N=64 143.8 -> 141.1, 36864x9216 N=16 71.4 -> 70.6.
 //
 // The MMA-issuing warp runs converged and elects one lane inside the instruction block: operands then stay in uniform
@@ -29,8 +29,9 @@
 //
 // Measured (B200, back to back on one stream, two matrices in turn, against one CTA or cluster per tile row): 27648x9216 N=8
 // 90 % 62.2 -> 45.4 us, 2048x32768 N=16 70 % 27.0 -> 24.5, 9216x36864 N=32 70 % 100 -> 93, 49152x12288 N=64 80 % 170 -> 141,
-// 36864x9216 N=16 80 % (288 rows: hardly any quantisation to begin with) 75.9 -> 70.6.  The chunks cost 0 to 0.7 % of that, at
-// N = 64 1.3 %.
+// 36864x9216 N=16 80 % (288 rows: hardly any quantisation to begin with) 75.9 -> 70.6.  (With another matrix on every call, none
+// of which L2 holds, the large ones take 2 to 15 % longer.)  The chunks cost 0 to 0.7 % of that, at N = 64 1.3 %; as short as 24
+// tiles there, which the cut by tiles asks of 27648x12288 with a workspace, 4.8 % (85.2 -> 89.3).
 // A CTA's share is bound by the shared-memory work of its tiles: of ~3300 cycles from one tile of a stage to the next at
 // 80 % (8 stages per SM: 412 per tile), 570 go to clearing the stage, 1140 to the 16-bit scatter stores (they wait for the
 // tensor core's operand reads), 1070 to getting the next tile's loads issued behind the other warps' stores, 430 to the
@@ -447,13 +448,15 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
             const int  c_last    = whole ? cta : stream_owner(p, ctas, row_begin + p.k_tiles - 1);
             const bool ask       = c_last == cta + 1 && t_begin <= row_begin;
             bool       asked = false, complete = false;
+            float      bias  = 0.0f;
             auto       other_has_parked = [&](bool look) {  // every epilogue warp asks once
                 asked             = true;
                 unsigned int seen = 0u;
                 if (look && tid == 0) {
                     ptx::grid_dependency_wait();  // counters may be in use by the stream's previous launch until it is over
                     seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
-                    for (int n = 1; seen == 0u && n < kStreamLooks && !ptx::mbar_test_wait(acc_full + 8u * (q & 1), (q >> 1) & 1u); ++n)
+                    for (int n = 1; seen == 0u && n < kStreamLooks && !ptx::mbar_test_wait(acc_full + 8u * (q & 1), (q >> 1) & 1u);
+                         ++n)
                         seen = ptx::ld_relaxed_gpu_u32(p.tile_counters + row);
                     ptx::fence_acq_rel_gpu();
                 }
@@ -478,6 +481,10 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                 }
                 ok = __all_sync(0xFFFFFFFFu, wait_bounded_converged(acc_full + 8u * (q & 1), (q >> 1) & 1u, abort_flag, p.status));
                 ptx::tc_fence_after_sync();
+                // Bias and residual may be the stream's earlier work.  With launch overlap on these warps have not waited for that,
+                // but a full accumulator has: it took a B that was loaded after the wait.  (A wait of their own costs 0.6 %.)
+                if (i == 0)
+                    bias = ok ? bias_of(p, row * kTileM + r) : 0.0f;
                 if (!ok || last_chunk)
                     break;
 #pragma unroll 1
@@ -488,12 +495,10 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCtasPerSm)
                 }
                 ptx::tmem_wait_st();
             }
-            // Bias and residual may be the stream's earlier work.  With launch overlap on these warps have not waited for that, but
-            // a full accumulator has: it took a B that was loaded after the wait.  (A wait of their own costs 0.6 % of a call.)
-            const float bias = ok ? bias_of(p, row * kTileM + r) : 0.0f;
             if (ask && !asked)  // gave up on the way
                 complete = other_has_parked(false);
-            float* const park = whole || complete ? nullptr : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (j == 0 ? 0 : 1)) + r;
+            float* const park = whole || complete ? nullptr
+                                                  : p.partial + static_cast<size_t>(N_TILE) * kTileM * (2 * cta + (j == 0 ? 0 : 1)) + r;
             if (ok) {  // the segment's last chunk
 #pragma unroll 1
                 for (int c0 = 0; c0 < N_TILE; c0 += 8) {
