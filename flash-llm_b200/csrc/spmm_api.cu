@@ -520,7 +520,8 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     for (int v : ov.v)
         pinned |= v != 0;
     if (pl.path == kPathStream)  // pinned: other fields do not apply to it
-        return may_stream && !sends ? make_stream_plan(st, pl, tile_rows, k_tiles, (k_tiles + 1) / 2, out) : cudaErrorInvalidConfiguration;
+        return may_stream && !sends ? make_stream_plan(st, pl, tile_rows, k_tiles, (k_tiles + 1) / 2, out)
+                                    : cudaErrorInvalidConfiguration;
     if (pl.path == kPathWide || (N >= 256 && !pinned && !sends)) {
         if (N < 256 || N % 128 != 0 || sends)
             return cudaErrorInvalidConfiguration;
@@ -556,11 +557,11 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // kernel).  A launch of rows*G clusters of S CTAs runs in ceil(rows*G / capacity(S)) waves, where capacity(S) is
     // the number of clusters of S CTAs the GPU holds at a time -- measured, and well below slots/S for S >= 3 (71
     // clusters of 4, 33 of 8 on 296 slots): one cluster more than that and the launch takes twice as long.  Up to 64
-    // columns row_form_us prices a cut.  Elsewhere every
-    // CTA processes k_tiles/(S*G) tiles after a fixed cost worth about 16 tiles; a cluster sum costs about 3 more,
-    // the sum by the last CTA 2 + 0.1 per part (8 + 0.1 per part in a fused all-reduce, where the peers wait for that
-    // CTA: measured on 2 GPUs, 9216x1152 ... 9216x18432), a second kernel half a tile per part.  The cheapest (S, G) wins,
-    // fewer parts on a tie.  Replaces the reference's hand-tuned Split_K tables (kernel_benchmark/benchmark.sh:13-15).
+    // columns row_form_us prices a cut.  Elsewhere it is cut by tiles: every CTA processes k_tiles/(S*G) tiles after a
+    // fixed cost worth about 16 tiles; a cluster sum costs about 3 more, the sum by the last CTA 2 + 0.1 per part (8 + 0.1
+    // per part in a fused all-reduce, where the peers wait for that CTA: measured on 2 GPUs, 9216x1152 ... 9216x18432), a
+    // second kernel half a tile per part.  The cheapest (S, G) wins, fewer parts on a tie.  Replaces the reference's
+    // hand-tuned Split_K tables (kernel_benchmark/benchmark.sh:13-15).
     const bool two_resident = two_per_sm && ((direct && pl.producers == 1) ? kDirectBlocks : 2) == 2;
     const int* resident     = two_resident ? kClustersResident2 : kClustersResident1;
     const int max_extra = max_parts > 1 ? max_parts : 1;
@@ -704,8 +705,9 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     return cudaSuccess;
 }
 
-// B as a 3-D tensor {64 K-elements (inner), N, K/64}: one box = b_batch K tiles of [n_tile x 64] (wide form: of one MMA's columns), each stored as a
-// 128-byte-swizzled slab; rows past N and K tiles past K/64 read as 0.  ldb: halves from one row of B to the next.
+// B as a 3-D tensor {64 K-elements (inner), N, K/64}: one box = b_batch K tiles of [n_tile x 64] (wide form: of one MMA's
+// columns), each stored as a 128-byte-swizzled slab; rows past N and K tiles past K/64 read as 0.  ldb: halves from one row of
+// B to the next.
 static cudaError_t encode_b_map(const half* B, int N, int K, int ldb, const SpmmPlan& pl, CUtensorMap* map)
 {
     const cuuint64_t dims[3]    = {static_cast<cuuint64_t>(kTileK), static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(K / kTileK)};
@@ -898,7 +900,8 @@ static cudaError_t spmm_launch_all(cudaStream_t stream,
     if (M_Global <= 0 || K_Global <= 0 || M_Global % kTileM != 0 || K_Global % kTileK != 0 || Split_K < 1
         || Compressed_A == nullptr || TileOffsets == nullptr || B == nullptr || C == nullptr
         || (reinterpret_cast<uintptr_t>(Compressed_A) & 15u) != 0 || (reinterpret_cast<uintptr_t>(B) & 15u) != 0
-        || (ldb != 0 && (ldb < K_Global || ldb % 8 != 0)) || (reinterpret_cast<uintptr_t>(C) & 1u) != 0 || (Split_K > 1 && Reduction_Workspace == nullptr))
+        || (ldb != 0 && (ldb < K_Global || ldb % 8 != 0)) || (reinterpret_cast<uintptr_t>(C) & 1u) != 0
+        || (Split_K > 1 && Reduction_Workspace == nullptr))
         return cudaErrorInvalidValue;
 
     cudaError_t  err = cudaSuccess;

@@ -558,7 +558,8 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
                     if (false)
 #endif
                     ready = ptx::umma_tile_commit_probe(
-                        tmem_acc + static_cast<uint32_t>((j & (accs - 1)) * N_TILE), a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
+                        tmem_acc + static_cast<uint32_t>((j & (accs - 1)) * N_TILE),
+                        a_desc0 + static_cast<uint32_t>(s * (kDenseTileBytes >> 4)),
                         b_desc0 + static_cast<uint32_t>((bs * KB + kb) * (kBSlab >> 4)), idesc, j >= accs ? 1u : 0u, a_empty + 8u * s,
                         b_empty + 8u * bs, (batch_done || !has_next) ? 1u : 0u, a_full + 8u * s_n, a_par_n, b_full + 8u * bs_n,
                         b_par_n, has_next ? 1u : 0u, (has_next && batch_done) ? 1u : 0u);
@@ -679,8 +680,8 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
             FL_CTA_TIME(2);
 
         if (!PUSH || S == 1)
-            accumulators_to_output<N_TILE>(p, tmem_acc, L < accs ? L : accs, N_TILE, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, G, g, n_idx,
-                                           tile_row, acc_ok, reinterpret_cast<float*>(smem));
+            accumulators_to_output<N_TILE>(p, tmem_acc, L < accs ? L : accs, N_TILE, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, G, g,
+                                           n_idx, tile_row, acc_ok, reinterpret_cast<float*>(smem));
     }
 
     // ================================================================ cluster reduction and tear-down
@@ -701,8 +702,8 @@ __global__ void __launch_bounds__((1 + kDirectIssuers + WARPS * WPT) * 32, MIN_B
             ptx::cluster_sync_all();  // nobody multiplies any more, the stages are free
         if (warp >= first_sw) {
             ptx::tc_fence_after_sync();
-            accumulators_to_peers<N_TILE>(tmem_acc, L < accs ? L : accs, n_valid, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, rank, sum_base,
-                                          sum_full, acc_ok);
+            accumulators_to_peers<N_TILE>(tmem_acc, L < accs ? L : accs, n_valid, warp & 3, lane, sw, NSW >= 8 ? 2 : 1, S, rank,
+                                          sum_base, sum_full, acc_ok);
             finish_cluster_rows<N_TILE>(p, sum_base, rank, S, G, g, n_idx, tile_row, n_valid, threadIdx.x - first_sw * 32, NTS, [&]() {
                 return __all_sync(0xFFFFFFFFu, wait_bounded_cluster(sum_full, 0u, abort_flag, p.status)) && *abort_flag == 0u;
             });

@@ -45,9 +45,6 @@ struct SpmmParams {
     int           M, N, K;
     int           k_tiles;  // K / 64
     SpmmPlan      plan;
-    // Fused all-reduce of a row-parallel SpMM (push_world > 0): every finished fp32 value of this GPU's partial product
-    // is stored into the receive slot this rank owns on every GPU of the group (its own included) instead of C, and
-    // each CTA then raises one flag per GPU; allreduce_sum_kernel on each GPU adds the slots up.
     // Split-K sum without a second kernel (workspace_k > 1 and tile_counters != nullptr): every CTA stores its fp32
     // partial tile, then counts itself in on the tile's counter; the CTA that finds all the others already counted adds
     // the parts up in part order and finishes the output.  Nobody waits.  Counters are zero between launches.
@@ -55,6 +52,9 @@ struct SpmmParams {
     // Streaming form: the CTAs' shares of the tile sequence (stream_begin).
     unsigned long long stream_share;
     float              ctas_per_tile;
+    // Fused all-reduce of a row-parallel SpMM (push_world > 0): every finished fp32 value of this GPU's partial product
+    // is stored into the receive slot this rank owns on every GPU of the group (its own included) instead of C, and
+    // each CTA then raises one flag per GPU; allreduce_sum_kernel on each GPU adds the slots up.
     int           push_world;
     unsigned int  push_epoch;                  // value the flags are raised to by this call
     float*        push_slot[kMaxPushWorld];    // [N][M] fp32 slot of this rank in GPU w's receive buffer
@@ -86,10 +86,7 @@ __device__ __forceinline__ half finish_output(float acc, const half* bias, int m
     return __float2half_rn(acc);
 }
 
-// C consecutive columns of output row m as finish_output finishes them; the first is element `at` of the output, and all
-// C or none of them lie inside it (`columns` left: N is 8 or a multiple of C wherever this is called).  Nothing is decided
-// per element: with a chain of branches on p's pointers for every element the 128 columns of one tile took 10 us of a
-// 13.0 us launch (128x64, N = 128), this way the launch takes 7.2 us.  Adding -0.0 leaves every value as it is.
+// Adding -0.0 leaves every value as it is.
 __device__ __forceinline__ float bias_of(const SpmmParams& p, int m)
 {
     return p.bias != nullptr ? __half2float(p.bias[m]) : -0.0f;
@@ -103,6 +100,10 @@ __device__ __forceinline__ void load_residual(const SpmmParams& p, half (&res)[C
         res[i] = p.residual[at + i * static_cast<size_t>(p.M)];
 }
 
+// C consecutive columns of an output row as finish_output finishes them; the first is element `at` of the output, and all C
+// or none of them lie inside it (`columns` left: N is 8 or a multiple of C wherever this is called).  Nothing is decided per
+// element: with a chain of branches on p's pointers for every element the 128 columns of one tile took 10 us of a 13.0 us
+// launch (128x64, N = 128), this way the launch takes 7.2 us.
 // `loaded`: the residual's values, where the caller has asked for them before it had the sums.
 template<int C>
 __device__ __forceinline__ void finish_columns(const SpmmParams& p, float (&v)[C], size_t at, int columns, float bias,
@@ -246,10 +247,11 @@ wait_bounded_relaxed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_fla
     }
 }
 
-// Warp-collective form: lane 0 alone probes the mbarrier and the other lanes take its answer at a warp barrier.
-// A probe executed by all 32 lanes costs several hundred cycles (measured: ~380 per already-completed wait), so a
-// warp must never wait lane by lane.  The warp barrier orders lane 0's observation of the completed phase before
-// the other lanes' later reads of the data it guards.
+// Warp-collective form of the sleeping wait: lane 0 alone probes the mbarrier and the other lanes take its answer at a warp
+// barrier, which orders lane 0's observation of the completed phase before their later reads of the data it guards.  (All 32
+// lanes of a sleeping wait, each testing and sleeping by itself, cost ~380 cycles per already completed phase.  The parked
+// wait, wait_bounded_converged, is the other way round: with a lane of its own to probe, and then a shuffle, the
+// register-streaming form's calls take 0 to 4 % longer.)
 __device__ __forceinline__ bool
 wait_bounded_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int* status)
 {
