@@ -296,3 +296,34 @@ def test_output_that_is_only_two_byte_aligned(lib, oracle, plan, offset_halves):
     assert lib.consume_status() == 0
     assert_close(C.view(N, M).cpu().numpy(), want, f"C at +{2 * offset_halves} bytes, plan {plan}")
     assert torch.isnan(backing[:offset_halves]).all() and torch.isnan(backing[offset_halves + N * M:]).all()
+
+
+@pytest.mark.parametrize("M,K,N,split_k,cluster_k", [(2048, 32768, 16, 4, 8), (9216, 18432, 32, 6, 2)])
+def test_workspace_parts_that_do_not_fit(lib, M, K, N, split_k, cluster_k):
+    """A call whose C is not aligned for workspace parts is planned without them: right, and its sums no longer in the tensor
+    core than in the cluster parts of the plan with them (`cluster_k`, 7e-8 to 1.4e-7 of a sum per tile).  The mean over the
+    outputs, rounding to fp16 included, is uncertain by 2^-11 / sqrt(12 * 32768) = 8e-7 at most; 2e-6 is allowed."""
+    from flash_llm_b200 import torch_op  # noqa: F401  (registers torch.ops.flashllm)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M + K)
+    A = torch.rand((M, K), generator=gen, device="cuda").half()
+    A *= torch.rand((M, K), generator=gen, device="cuda") >= 0.8
+    B = torch.rand((N, K), generator=gen, device="cuda").half()
+    want = torch.cat([B.double() @ A[r:r + 1024].double().T for r in range(0, M, 1024)], dim=1)
+    words, offs = torch.ops.flashllm.encode(A)
+    ws = torch.empty((split_k, N, M), dtype=torch.float16, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    share = {}
+    try:
+        for name, shift, plan in (("moved", 1, {}), ("cut", 0, dict(cluster_k=cluster_k, workspace_k=1))):
+            C = torch.full((N * M + 8,), float("nan"), dtype=torch.float16, device="cuda")[shift:shift + N * M]
+            lib.set_plan(path=lib.api.PATH_DIRECT, **plan)
+            lib.SpMM_SplitK_API(stream, None, words.data_ptr(), offs.data_ptr(), B.data_ptr(), C.data_ptr(), M, N, K, ws.data_ptr(),
+                                split_k)
+            torch.cuda.synchronize()
+            assert lib.consume_status() == 0
+            assert_close(C.view(N, M).cpu().numpy(), want.float().cpu().numpy(), name)
+            share[name] = abs(float(((want - C.view(N, M).double()) / want).mean()))
+    finally:
+        lib.set_plan()
+    assert share["moved"] <= share["cut"] + 2e-6, share
