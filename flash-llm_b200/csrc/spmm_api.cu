@@ -663,6 +663,7 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %: 1.00 .. 1.07).
     // Where large clusters leave no place for the next launch's, a CTA's end counts for more: off, 56 clusters of five 1.04 at 8,
     // 1.07 at 13, 1.02 at 29, 45 of six 1.00, 0.99, 0.96 at 7, 11, 24, 33 of eight 1.02, 1.03, 1.00 at 5, 8, 18.
+    // Up to 64 CTAs do not meet the next launch's on an SM, and have the area at any length: 1.00 at 65 and 80 %, 1.02 at 92 %.
     // 64 columns are sent where CTAs have an SM to themselves (kPushMaxN), also from the next launch's (overlap on, sent / parked: 4
     // clusters of eight by 46 tiles 7.2 / 8.4 us, 8 of four by 16 6.8 / 7.6, but 16 of four 9.1 / 8.2, 8 of six 8.7 / 7.4).
     // The fused all-reduce parks: its CTAs then store whole columns of 512 bytes to the other GPUs, not runs of 64.
@@ -672,7 +673,7 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     if (pl.push) {
         pl.sum_bytes       = cluster_sum_bytes(pl.n_tile, pl.cluster_k);
         const bool full    = pl.cluster_k >= 5 && grid_is_full(st, static_cast<long long>(ctas_flat) * extra, pl.cluster_k);
-        const bool short_k = (k_tiles + parts - 1) / parts <= (overlap || full ? 16 : 4);
+        const bool short_k = (k_tiles + parts - 1) / parts <= (overlap || full ? 16 : 4) || ctas_flat * extra * pl.cluster_k <= 64;
         const int  room    = two_resident ? (short_k ? kSmemPerSm : kSmemForL1) / 2 - 1024 : st->smem_optin;
         if (plan_smem_bytes(pl) > room)
             pl.sum_bytes = 0;

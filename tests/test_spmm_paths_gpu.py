@@ -110,10 +110,11 @@ def test_cluster_sums_of_every_width(lib, oracle, form, cluster_k, N):
 
 @pytest.mark.parametrize("overlap", [False, True])
 @pytest.mark.parametrize("rows,tiles,cluster_k,N", [
-    (3, 8, 2, 32), (3, 9, 2, 32), (3, 10, 2, 32),     # 4 tiles a CTA and more: the receiving area goes, launch overlap off
-    (3, 32, 2, 32), (3, 33, 2, 32), (3, 115, 7, 32),  # 16 and more: it goes with launch overlap on
+    (33, 8, 2, 32), (33, 9, 2, 32), (3, 10, 2, 32),     # 4 tiles a CTA and more: the receiving area goes, launch overlap off
+    (33, 32, 2, 32), (33, 33, 2, 32), (10, 115, 7, 32),  # 16 and more: it goes with launch overlap on
     (100, 38, 2, 32), (100, 38, 2, 64), (40, 33, 7, 64), (12, 16, 4, 64), (13, 16, 4, 64), (8, 24, 6, 64), (72, 9, 2, 64),
-    (75, 9, 2, 64), (16, 16, 8, 64),                  # 64 columns: CTAs with an SM to themselves, and pairs on every SM
+    (8, 130, 8, 32), (9, 130, 8, 32),                    # 64 CTAs and more: off, only few of them have it at this length
+    (75, 9, 2, 64), (16, 16, 8, 64),                     # 64 columns: CTAs with an SM to themselves, and pairs on every SM
 ])
 def test_cluster_sums_by_length_and_crowding(lib, rows, tiles, cluster_k, N, overlap):
     """What a cluster's sum goes through (an area of its own, the operands' buffers, the parked tiles) depends on the K tiles of
