@@ -659,8 +659,9 @@ static cudaError_t make_plan(const DeviceState* st, int M, int N, int K, int max
     // multiplies.  (Wide outputs take the operands' buffers, once everybody's MMAs are over.)  That saves a call 0.1 to 0.6 us,
     // but an L1 too small for the loads in flight (8 warps x 13 rows of 512 bytes at 80 %) costs every tile: two CTAs of 32
     // columns leave 28 KB with such room and 92 without, and 9216x36864 70 % in clusters of two took 102.5 us instead of 97.8.
-    // They have it for short K ranges only; time without it / with it by tiles per CTA (72 x 4 and 148 x 2 CTAs, 65 to 80 %): overlap off
-    // 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %: 1.00 .. 1.07).
+    // They have it for short K ranges only; time without it / with it by tiles per CTA (72 x 4 and 148 x 2 CTAs, 65 to 80 %):
+    // overlap off 0.98 .. 0.99 at 4, 0.97 at 8, 0.95 at 24; on 1.00 .. 1.04 at 8, 0.96 .. 1.01 at 16, 0.96 .. 0.98 at 24 (92 %:
+    // 1.00 .. 1.07).
     // Where large clusters leave no place for the next launch's, a CTA's end counts for more: off, 56 clusters of five 1.04 at 8,
     // 1.07 at 13, 1.02 at 29, 45 of six 1.00, 0.99, 0.96 at 7, 11, 24, 33 of eight 1.02, 1.03, 1.00 at 5, 8, 18.
     // Up to 64 CTAs do not meet the next launch's on an SM, and have the area at any length: 1.00 at 65 and 80 %, 1.02 at 92 %.
@@ -754,7 +755,7 @@ static cudaError_t plan_call(const CallKey& key, CallMemo** out)
     if (!(m.key == key)) {
         SpmmPlan          plan{};
         const cudaError_t err = make_plan(key.device, key.M, key.N, key.K, key.max_parts, &plan, key.sends, key.may_stream,
-                                                key.parts_fit);
+                                          key.parts_fit);
         if (err != cudaSuccess)
             return err;
         m.key     = key;

@@ -20,8 +20,9 @@
 // What a call takes after its last MMA is no other CTA's work any more, so it is kept short.  The first of two CTAs that share
 // a row usually finds the other's part parked, takes it into tensor memory while its own is being multiplied and finishes the
 // row without parking.  Other rows are added up when the CTA's roles are done, by all of its threads instead of the four
-// epilogue warps: a part is an L2 round trip away.  Both together, us per call with two matrices in turn: 2048x32768 N=16 70 % (19 parts a row) 26.5 ->
-// 24.5, 9216x36864 N=32 70 % (5 parts) 97.1 -> 93.4, 49152x12288 N=64 143.8 -> 141.1, 36864x9216 N=16 71.4 -> 70.6.
+// epilogue warps: a part is an L2 round trip away.  Both together, us per call with two matrices in turn: 2048x32768 N=16 70 %
+// (19 parts a row) 26.5 -> 24.5, 9216x36864 N=32 70 % (5 parts) 97.1 -> 93.4, 49152x12288 N=64 143.8 -> 141.1, 36864x9216 N=16
+// 71.4 -> 70.6.
 //
 // The MMA-issuing warp runs converged and elects one lane inside the instruction block: operands then stay in uniform
 // registers.  Issued from a branch taken by one lane, the four MMAs and the commit of a tile cost 271 cycles instead of
